@@ -1,6 +1,5 @@
 // C ABI of libdpb200: model upload, workspace sizing and evaluation dispatch.
-#include "internal.cuh"
-#include "tc.cuh"
+#include "rows.cuh"
 #include <cuda_bf16.h>
 #include <cmath>
 #include <cstring>
@@ -57,13 +56,22 @@ static void prof_collect() {
   g_prof_next = 0;
 }
 
-// fp32 path (eval_fp32.cu)
-template <int E0, int E1, int E2>
-int launch_embed_fwd(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
-                     const int32_t *, float *, float *, cudaStream_t);
-template <int E0, int E1, int E2>
-int launch_embed_bwd(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
-                     const int32_t *, const float *, const float *, float4 *, double *, cudaStream_t);
+// fp32 path: tuned nets on the tensor cores (embed_split.cu), compressed
+// tables and the fitting chain (eval_fp32.cu)
+void split_net_image(int E2, const float *w0, const float *b0, const float *w1, const float *b1, const float *w2,
+                     const float *b2, double s_lo, double s_hi, std::vector<char> &img, std::vector<float> &small);
+int split_block_atoms(const SysDesc &D);
+int split_embed_fwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
+                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, cudaStream_t st);
+int split_embed_bwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
+                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, const float *dG, float4 *F4,
+                    double *virial, cudaStream_t st);
+template <int E2>
+int launch_embed_fwd_cmp(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
+                         const int32_t *, float *, float *, cudaStream_t);
+template <int E2>
+int launch_embed_bwd_cmp(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
+                         const int32_t *, const float *, const float *, float4 *, double *, cudaStream_t);
 int launch_sgemm(int, int, int, const float *, int, RowMap, const float *, const Epi &, cudaStream_t);
 // any embedding shape (eval_general.cu)
 int launch_embed_fwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
@@ -125,15 +133,6 @@ static int upload_fit_tiles(dpb_model *m, const std::vector<float> &a, int rows,
   std::vector<__half> b(t.size());
   for (size_t i = 0; i < t.size(); ++i) b[i] = __float2half_rn(t[i] * scale);
   return upload(m, b.data(), b.size(), dev);
-}
-
-// 2^k with x 2^k in (2^13, 2^14] (x > 0; 1 for x = 0 or non-finite), k
-// clamped to [-40, 40].
-static float pow2_scale_to_2p14(double x) {
-  if (!(x > 0.0) || !std::isfinite(x)) return 1.f;
-  int k = 14 - (int)std::ceil(std::log2(x));
-  k = std::max(-40, std::min(40, k));
-  return std::ldexp(1.f, k);
 }
 
 // The tuned three-layer embedding instantiations (FP32 and tensor-core kernels).
@@ -262,6 +261,14 @@ extern "C" int dpb_model_create(const dpb_model_desc *d, dpb_model **out) {
         sm[M.E0 + e] = b0[e];
       }
       if (rc == DPB_OK) rc = upload(m, sm.data(), sm.size(), &M.net_small[k]);
+      std::vector<char> simg;
+      std::vector<float> ssm;
+      // s~ of centre type k / ntypes from the cutoff down to 0.15 rcut
+      const double t = 0.15, smax = (1.0 - 3.0 * t * t + 2.0 * t * t * t) / (t * d->rcut);
+      const double mu = d->sr_mean[k / nt], sd = d->sr_std[k / nt];
+      dpb::split_net_image(M.E2, w0, b0, W1, b1, W2, b2, -mu / sd, (smax - mu) / sd, simg, ssm);
+      if (rc == DPB_OK) rc = upload(m, (const char *)simg.data(), simg.size(), &M.spl_img[k]);
+      if (rc == DPB_OK) rc = upload(m, (const float *)ssm.data(), ssm.size(), &M.spl_small[k]);
     }
   }
   if (rc == DPB_OK) rc = upload(m, d->tbias, (size_t)M.E2, &M.tbias);
@@ -494,32 +501,77 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
   return DPB_OK;
 }
 
+// The workspace past the FP32 layout (sized for the larger of the two forms)
+// that holds the type-sorted positions and the row store of the tensor-core
+// embedding; where it is too small (fitting widths beyond the mixed form's) the
+// positions go to the fitting chain's scratch, idle then, and the kernels
+// compact the neighbour lists themselves.
+struct SplitWs {
+  float4 *posS, *rows;
+  int *rcnt;
+};
+static SplitWs split_ws(const DevModel &M, size_t NF, size_t nE, char *base, char *fit_scratch) {
+  const size_t a = al(NF * fp32_ws_per_atom(M)) + 16 * 256 + al(nE * 9 * 8);
+  const size_t need = al(NF * 16) + al(NF * kRowStoreCap * 16) + al(NF * M.ntypes * 4);
+  SplitWs s{reinterpret_cast<float4 *>(fit_scratch), nullptr, nullptr};
+  if (eval_ws_bytes(M, NF, nE) >= a + need) {
+    char *w = base + a;
+    s.posS = (float4 *)w; w += al(NF * 16);
+    s.rows = (float4 *)w; w += al(NF * kRowStoreCap * 16);
+    s.rcnt = (int *)w;
+  }
+  return s;
+}
+
+// T and G of every atom in FP32: the tuned nets on the tensor cores, compressed
+// tables and other shapes in the FP32 kernels.
+static int embed_fwd_fp32(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm,
+                          const float *box, const int32_t *nbrs, const SplitWs &sw, int ba, float *T, float *G,
+                          cudaStream_t st) {
+  int rc = DPB_OK;
+  if (M.ngrids == 0 && M.emb_tuned) {
+    rc = launch_pos_sorted(D, pos, perm, sw.posS, st);
+    if (!rc && sw.rows && D.S <= kRowStoreCap) rc = launch_rows(M, D, ba, sw.posS, box, nbrs, sw.rows, sw.rcnt, st);
+    if (!rc) rc = split_embed_fwd(M, D, ba, sw.posS, box, nbrs, sw.rows, sw.rcnt, T, G, st);
+    return rc;
+  }
+  for (int ti = 0; ti < M.ntypes && !rc; ++ti)
+    rc = !M.emb_tuned   ? launch_embed_fwd_gen(M, D, ti, pos, perm, box, nbrs, T, G, st)
+         : M.E2 == 100 ? launch_embed_fwd_cmp<100>(M, D, ti, pos, perm, box, nbrs, T, G, st)
+                       : launch_embed_fwd_cmp<64>(M, D, ti, pos, perm, box, nbrs, T, G, st);
+  return rc;
+}
+
 static int eval_fp32(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm,
                      const float *box, const int32_t *nbrs, double *energy, float4 *F4, float *Eatom,
-                     double *virial, char *w, cudaStream_t st) {
+                     double *virial, char *base, char *w, size_t nE, cudaStream_t st) {
   const size_t NF = (size_t)D.N * D.F;
   const int E2 = M.E2, A = M.A, K0 = A * E2;
   float *T = (float *)w; w += al(NF * 10 * E2 * 4);
   float *G = (float *)w; w += al(NF * K0 * 4);  // G, later dE/dG
+  const SplitWs sw = split_ws(M, NF, nE, base, w);
+  const int ba = split_block_atoms(D);
   int rc;
   prof_begin(PROF_EMBED_FWD, st);
-  for (int ti = 0; ti < M.ntypes; ++ti) {
-    if (!M.emb_tuned) rc = launch_embed_fwd_gen(M, D, ti, pos, perm, box, nbrs, T, G, st);
-    else if (M.E2 == 100) rc = launch_embed_fwd<25, 50, 100>(M, D, ti, pos, perm, box, nbrs, T, G, st);
-    else rc = launch_embed_fwd<32, 32, 64>(M, D, ti, pos, perm, box, nbrs, T, G, st);
-    if (rc) return rc;
-  }
+  rc = embed_fwd_fp32(M, D, pos, perm, box, nbrs, sw, ba, T, G, st);
+  if (rc) return rc;
   prof_end(PROF_EMBED_FWD, st);
   prof_begin(PROF_FIT, st);
   rc = fit_fp32_chain(M, D, G, Eatom, energy, w, st);
   if (rc) return rc;
   prof_end(PROF_FIT, st);
   prof_begin(PROF_EMBED_BWD, st);
-  for (int ti = 0; ti < M.ntypes; ++ti) {
-    if (!M.emb_tuned) rc = launch_embed_bwd_gen(M, D, ti, pos, perm, box, nbrs, T, G, F4, virial, st);
-    else if (M.E2 == 100) rc = launch_embed_bwd<25, 50, 100>(M, D, ti, pos, perm, box, nbrs, T, G, F4, virial, st);
-    else rc = launch_embed_bwd<32, 32, 64>(M, D, ti, pos, perm, box, nbrs, T, G, F4, virial, st);
+  if (M.ngrids == 0 && M.emb_tuned) {
+    if (!sw.rows) rc = launch_pos_sorted(D, pos, perm, sw.posS, st);  // the fitting chain overwrote them
+    if (!rc) rc = split_embed_bwd(M, D, ba, sw.posS, box, nbrs, sw.rows, sw.rcnt, T, G, F4, virial, st);
     if (rc) return rc;
+  } else {
+    for (int ti = 0; ti < M.ntypes; ++ti) {
+      if (!M.emb_tuned) rc = launch_embed_bwd_gen(M, D, ti, pos, perm, box, nbrs, T, G, F4, virial, st);
+      else if (M.E2 == 100) rc = launch_embed_bwd_cmp<100>(M, D, ti, pos, perm, box, nbrs, T, G, F4, virial, st);
+      else rc = launch_embed_bwd_cmp<64>(M, D, ti, pos, perm, box, nbrs, T, G, F4, virial, st);
+      if (rc) return rc;
+    }
   }
   prof_end(PROF_EMBED_BWD, st);
   return DPB_OK;
@@ -553,7 +605,7 @@ int dpb::eval_impl(const dpb_model *m, int precision, const float *pos, const in
   DPB_CUDA_TRY(cudaMemsetAsync(energy, 0, nE * 8, st));
   DPB_CUDA_TRY(cudaMemsetAsync(vir, 0, nE * 72, st));
   if (precision == DPB_PREC_FP32) {
-    rc = eval_fp32(M, D, pos, perm, box, nbrs, energy, F4, Eatom, vir, w, st);
+    rc = eval_fp32(M, D, pos, perm, box, nbrs, energy, F4, Eatom, vir, (char *)workspace, w, nE, st);
   } else {
     if (!mixed_supported(M)) return DPB_ERR_UNSUPPORTED;
     rc = mixed_eval(M, D, pos, perm, box, nbrs, energy, Eatom, F4, vir, w, st, m->dT_warps, m->fit_deep != 0);
@@ -609,18 +661,6 @@ extern "C" int dpb_profile_read(int id, double *ms, uint64_t *count) {
   return DPB_OK;
 }
 
-// fp32 descriptor stage (eval_fp32.cu kernels), T and G of every atom
-static int descriptors_fp32(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm,
-                            const float *box, const int32_t *nbrs, float *T, float *G, cudaStream_t st) {
-  for (int ti = 0; ti < M.ntypes; ++ti) {
-    int rc = !M.emb_tuned   ? launch_embed_fwd_gen(M, D, ti, pos, perm, box, nbrs, T, G, st)
-             : M.E2 == 100 ? launch_embed_fwd<25, 50, 100>(M, D, ti, pos, perm, box, nbrs, T, G, st)
-                           : launch_embed_fwd<32, 32, 64>(M, D, ti, pos, perm, box, nbrs, T, G, st);
-    if (rc) return rc;
-  }
-  return DPB_OK;
-}
-
 extern "C" int dpb_eval_descriptors(const dpb_model *m, int precision, const float *pos, const int32_t *perm,
                                     int natoms, int nframes, const int *type_count, const float *box,
                                     const int32_t *nbrs, const int *sel, float *T, float *G, int *err,
@@ -634,11 +674,16 @@ extern "C" int dpb_eval_descriptors(const dpb_model *m, int precision, const flo
   int rc = fill_sys(m, natoms, nframes, type_count, sel, D);
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
-  if (precision == DPB_PREC_FP32) return descriptors_fp32(m->dm, D, pos, perm, box, nbrs, T, G, st);
+  auto fp32 = [&]() {
+    char *w = (char *)workspace;
+    const SplitWs sw = split_ws(m->dm, (size_t)natoms * nframes, (size_t)nframes, w, w);
+    return embed_fwd_fp32(m->dm, D, pos, perm, box, nbrs, sw, split_block_atoms(D), T, G, st);
+  };
+  if (precision == DPB_PREC_FP32) return fp32();
   if (precision == DPB_PREC_MIXED) {
     if (!mixed_supported(m->dm)) return DPB_ERR_UNSUPPORTED;
     // the mixed form's embedding runs in the FP32 kernels for tables and untuned shapes
-    if (m->dm.ngrids > 0 || !m->dm.emb_tuned) return descriptors_fp32(m->dm, D, pos, perm, box, nbrs, T, G, st);
+    if (m->dm.ngrids > 0 || !m->dm.emb_tuned) return fp32();
     return mixed_descriptors_f32(m->dm, D, pos, perm, box, nbrs, T, G, err, workspace, st);
   }
   return DPB_ERR_INVALID_ARG;

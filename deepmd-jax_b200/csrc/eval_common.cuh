@@ -41,6 +41,10 @@ struct DevModel {
   const char *net_img[kMaxTypes * kMaxTypes];
   const float *net_small[kMaxTypes * kMaxTypes];
   int net_img_bytes, net_small_floats;
+  // per embedding net: the image of its FP16 hi / lo B tiles and the small FP32
+  // block of the FP32 form's tensor-core kernels (embed_split.cu, SplitDims)
+  const char *spl_img[kMaxTypes * kMaxTypes];
+  const float *spl_small[kMaxTypes * kMaxTypes];
   // compressed embedding (ngrids > 0): per net, poly_coeff (ngrids, 6, E2)
   // and the float32 srmin / interval width of the reference's table lookup
   int ngrids;

@@ -27,106 +27,6 @@ __device__ __forceinline__ float3 load_pos(const float *__restrict__ pos, const 
   return make_float3(p[0], p[1], p[2]);
 }
 
-template <int E0, int E1, int E2>
-struct EmbedDims {
-  static constexpr int NW = 2 * E0 + E0 * E1 + E1 + E1 * E2 + E2;  // floats per net
-  static constexpr int NQ = (E2 + 31) / 32;
-  static constexpr int Z1 = E1 / E0;
-  static constexpr int Z2 = E2 / E1;
-};
-
-// Load the weights of nets (ti, tj), tj < ntypes, into shared memory.
-template <int E0, int E1, int E2>
-__device__ void load_nets(const DevModel &M, int ti, float *wsm) {
-  using D = EmbedDims<E0, E1, E2>;
-  for (int tj = 0; tj < M.ntypes; ++tj) {
-    int k = ti * M.ntypes + tj;
-    float *w = wsm + tj * D::NW;
-    const float *src[6] = {M.ew[k][0], M.eb[k][0], M.ew[k][1], M.eb[k][1], M.ew[k][2], M.eb[k][2]};
-    const int len[6] = {E0, E0, E0 * E1, E1, E1 * E2, E2};
-    int o = 0;
-    for (int s = 0; s < 6; ++s) {
-      for (int e = threadIdx.x; e < len[s]; e += blockDim.x) w[o + e] = src[s][e];
-      o += len[s];
-    }
-  }
-}
-
-// ---------------------------------------------------------------- forward
-// One round of up to 32 compacted rows (row = lane).  Every layer runs
-// input-outer from activations staged per lane in shared memory
-// (h0s/h1s[k][lane]), so residual sources h[col / Z] are read with runtime
-// columns and no register array is indexed dynamically.  The contraction
-// T += R~^T h2 is accumulated per 32-column chunk in registers and added into
-// the warp's shared T (Ts[c][col]) once per round.
-template <int E0, int E1, int E2>
-__device__ __forceinline__ void embed_rows_fwd(const float *__restrict__ W, int n,
-                                               const float *__restrict__ rowbuf, float *__restrict__ h0s,
-                                               float *__restrict__ h1s, float *__restrict__ h2s,
-                                               float *__restrict__ Ts, int lane) {
-  using D = EmbedDims<E0, E1, E2>;
-  const float *w0 = W, *b0 = W + E0, *w1 = W + 2 * E0, *b1 = w1 + E0 * E1, *w2 = b1 + E1,
-              *b2 = w2 + E1 * E2;
-  const float st = lane < n ? rowbuf[lane * 12] : 0.f;
-#pragma unroll
-  for (int k = 0; k < E0; ++k) h0s[k * 32 + lane] = tanhf(fmaf(st, w0[k], b0[k]));
-#pragma unroll 1
-  for (int q = 0; q < (E1 + 31) / 32; ++q) {
-    float acc[32];
-#pragma unroll
-    for (int o = 0; o < 32; ++o) acc[o] = (q * 32 + o < E1) ? b1[q * 32 + o] : 0.f;
-#pragma unroll 2
-    for (int k = 0; k < E0; ++k) {
-      const float hv = h0s[k * 32 + lane];
-      const float *wr = w1 + k * E1 + q * 32;
-#pragma unroll
-      for (int o = 0; o < 32; ++o)
-        if (q * 32 + o < E1) acc[o] = fmaf(hv, wr[o], acc[o]);
-    }
-#pragma unroll
-    for (int o = 0; o < 32; ++o) {
-      const int col = q * 32 + o;
-      if (col < E1) h1s[col * 32 + lane] = tanhf(acc[o]) + h0s[(col / D::Z1) * 32 + lane];
-    }
-  }
-  __syncwarp();  // h2s aliases h0s
-#pragma unroll 1
-  for (int q = 0; q < D::NQ; ++q) {
-    float acc[32];
-#pragma unroll
-    for (int o = 0; o < 32; ++o) acc[o] = (q * 32 + o < E2) ? b2[q * 32 + o] : 0.f;
-#pragma unroll 2
-    for (int k = 0; k < E1; ++k) {
-      const float hv = h1s[k * 32 + lane];
-      const float *wr = w2 + k * E2 + q * 32;
-#pragma unroll
-      for (int o = 0; o < 32; ++o)
-        if (q * 32 + o < E2) acc[o] = fmaf(hv, wr[o], acc[o]);
-    }
-#pragma unroll
-    for (int o = 0; o < 32; ++o) {
-      const int col = q * 32 + o;
-      if (col < E2) h2s[lane * 33 + o] = tanhf(acc[o]) + h1s[(col / D::Z2) * 32 + lane];
-    }
-    __syncwarp();
-    const int col = q * 32 + lane;
-    if (col < E2) {
-      float Tq[10];
-#pragma unroll
-      for (int c = 0; c < 10; ++c) Tq[c] = 0.f;
-      for (int r = 0; r < n; ++r) {
-        const float hv = h2s[r * 33 + lane];
-        const float *R = rowbuf + r * 12 + 1;
-#pragma unroll
-        for (int c = 0; c < 10; ++c) Tq[c] = fmaf(R[c], hv, Tq[c]);
-      }
-#pragma unroll
-      for (int c = 0; c < 10; ++c) Ts[c * E2 + col] += Tq[c];
-    }
-    __syncwarp();
-  }
-}
-
 // ---------------------------------------------------------------- compressed embedding
 // The table lookup of the compressed embedding net (deepmd_jax/utils.py:126-151):
 // x = s~ - srmin; idx = trunc(x / delta); x0 = x - idx * delta; the gather
@@ -179,27 +79,20 @@ __device__ __forceinline__ void embed_rows_fwd_cmp(const float *__restrict__ coe
   __syncwarp();
 }
 
-template <int E0, int E1, int E2>
+template <int E2>
 __host__ __device__ constexpr int embed_fwd_warp_floats() {
-  return 64 * 12 + (32 * 33 > E0 * 32 ? 32 * 33 : E0 * 32) + E1 * 32 + 10 * E2;
+  return 64 * 12 + 10 * E2;
 }
 
-template <int E0, int E1, int E2, bool CMP>
+template <int E2>
 __global__ void __launch_bounds__(256) k_embed_fwd(DevModel M, SysDesc D, int ti, const float *__restrict__ pos,
                                                    const int32_t *__restrict__ perm, const float *__restrict__ box,
                                                    const int32_t *__restrict__ nbrs, float *__restrict__ Tout,
                                                    float *__restrict__ Gout) {
-  using ED = EmbedDims<E0, E1, E2>;
   extern __shared__ float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-  float *wsm = smem;
-  float *rowbuf = smem + (CMP ? 0 : M.ntypes * ED::NW) + warp * embed_fwd_warp_floats<E0, E1, E2>();
-  float *h2s = rowbuf + 64 * 12;  // aliases h0s
-  float *h0s = h2s;
-  float *h1s = h2s + (32 * 33 > E0 * 32 ? 32 * 33 : E0 * 32);
-  float *Ts = h1s + E1 * 32;
-  if (!CMP) load_nets<E0, E1, E2>(M, ti, wsm);
-  __syncthreads();
+  float *rowbuf = smem + warp * embed_fwd_warp_floats<E2>();
+  float *Ts = rowbuf + 64 * 12;
   const int f = blockIdx.y;
   const int a = blockIdx.x * wpb + warp;
   const int cnt_i = D.offs[ti + 1] - D.offs[ti];
@@ -217,7 +110,6 @@ __global__ void __launch_bounds__(256) k_embed_fwd(DevModel M, SysDesc D, int ti
   __syncwarp();
 
   for (int tj = 0; tj < D.ntypes; ++tj) {
-    const float *W = wsm + tj * ED::NW;
     const int32_t *nb = nbrs + g * D.S + D.col[tj];
     const int sel = D.sel[tj], cnt_j = D.offs[tj + 1] - D.offs[tj];
     int nbuf = 0;
@@ -253,11 +145,8 @@ __global__ void __launch_bounds__(256) k_embed_fwd(DevModel M, SysDesc D, int ti
       nbuf += __popc(m);
       __syncwarp();
       if (nbuf >= 32) {
-        if constexpr (CMP)
-          embed_rows_fwd_cmp<E2>(M.cmp_coeff[ti * M.ntypes + tj], M.cmp_srmin[ti * M.ntypes + tj],
-                                 M.cmp_delta[ti * M.ntypes + tj], M.ngrids, 32, rowbuf, Ts, lane);
-        else
-          embed_rows_fwd<E0, E1, E2>(W, 32, rowbuf, h0s, h1s, h2s, Ts, lane);
+        embed_rows_fwd_cmp<E2>(M.cmp_coeff[ti * M.ntypes + tj], M.cmp_srmin[ti * M.ntypes + tj],
+                               M.cmp_delta[ti * M.ntypes + tj], M.ngrids, 32, rowbuf, Ts, lane);
         const int rem = nbuf - 32;
         if (lane < rem)
           for (int c = 0; c < 12; ++c) rowbuf[lane * 12 + c] = rowbuf[(32 + lane) * 12 + c];
@@ -266,11 +155,8 @@ __global__ void __launch_bounds__(256) k_embed_fwd(DevModel M, SysDesc D, int ti
       }
     }
     if (nbuf > 0) {
-      if constexpr (CMP)
-        embed_rows_fwd_cmp<E2>(M.cmp_coeff[ti * M.ntypes + tj], M.cmp_srmin[ti * M.ntypes + tj],
-                               M.cmp_delta[ti * M.ntypes + tj], M.ngrids, nbuf, rowbuf, Ts, lane);
-      else
-        embed_rows_fwd<E0, E1, E2>(W, nbuf, rowbuf, h0s, h1s, h2s, Ts, lane);
+      embed_rows_fwd_cmp<E2>(M.cmp_coeff[ti * M.ntypes + tj], M.cmp_srmin[ti * M.ntypes + tj],
+                             M.cmp_delta[ti * M.ntypes + tj], M.ngrids, nbuf, rowbuf, Ts, lane);
     }
     __syncwarp();
   }
@@ -307,114 +193,6 @@ __global__ void __launch_bounds__(256) k_embed_fwd(DevModel M, SysDesc D, int ti
 }
 
 // ---------------------------------------------------------------- adjoint
-// Adjoint of one round of rows.  The row's embedding is recomputed with its
-// tangent along s~ (forward mode): h2 and dh2/ds~ give, against dE/dT,
-// u = dT.h2 = dE/dR~ and v = dT.dh2, so dE/ds~ = R~.v — no reverse sweep.
-template <int E0, int E1, int E2>
-__device__ __forceinline__ void embed_rows_bwd(const float *__restrict__ W, int n,
-                                               const float *__restrict__ rowbuf, const float *__restrict__ dT,
-                                               float *__restrict__ h1s, float *__restrict__ d1s,
-                                               float inv_std, float mean, int lane, float &fi0, float &fi1,
-                                               float &fi2, float (&vir)[9], float4 *__restrict__ F4,
-                                               size_t frame_base) {
-  using D = EmbedDims<E0, E1, E2>;
-  const float *w0 = W, *b0 = W + E0, *w1 = W + 2 * E0, *b1 = w1 + E0 * E1, *w2 = b1 + E1,
-              *b2 = w2 + E1 * E2;
-  const bool act = lane < n;
-  RowGeom gm;
-  int jj = 0;
-  if (act) {
-    const float *rb = rowbuf + lane * 8;
-    gm.x[0] = rb[0]; gm.x[1] = rb[1]; gm.x[2] = rb[2];
-    gm.r = rb[3]; gm.s = rb[4]; gm.dsdr = rb[5];
-    jj = __float_as_int(rb[6]);
-  } else {
-    gm.x[0] = gm.x[1] = gm.x[2] = 0.f; gm.r = 1.f; gm.s = 0.f; gm.dsdr = 0.f;
-  }
-  const float sn = gm.s * inv_std, st = (gm.s - mean) * inv_std;
-  const float inv_rp = 1.f / (gm.r + 1e-16f);
-  const float xh[3] = {gm.x[0] * inv_rp, gm.x[1] * inv_rp, gm.x[2] * inv_rp};
-  {
-    float h0[E0], d0[E0];
-#pragma unroll
-    for (int k = 0; k < E0; ++k) {
-      const float t = tanhf(fmaf(st, w0[k], b0[k]));
-      h0[k] = t;
-      d0[k] = (1.f - t * t) * w0[k];
-    }
-#pragma unroll
-    for (int o = 0; o < E1; ++o) {
-      float z = b1[o], dz = 0.f;
-#pragma unroll
-      for (int k = 0; k < E0; ++k) {
-        z = fmaf(h0[k], w1[k * E1 + o], z);
-        dz = fmaf(d0[k], w1[k * E1 + o], dz);
-      }
-      const float t = tanhf(z);
-      h1s[o * 32 + lane] = t + h0[o / D::Z1];
-      d1s[o * 32 + lane] = (1.f - t * t) * dz + d0[o / D::Z1];
-    }
-  }
-  __syncwarp();
-  float u[10], v[10];
-#pragma unroll
-  for (int c = 0; c < 10; ++c) u[c] = v[c] = 0.f;
-  constexpr int NQ16 = (E2 + 15) / 16;
-#pragma unroll 1
-  for (int q = 0; q < NQ16; ++q) {
-    float z[16], dz[16];
-#pragma unroll
-    for (int o = 0; o < 16; ++o) {
-      z[o] = (q * 16 + o < E2) ? b2[q * 16 + o] : 0.f;
-      dz[o] = 0.f;
-    }
-#pragma unroll 2
-    for (int k = 0; k < E1; ++k) {
-      const float hv = h1s[k * 32 + lane], dv = d1s[k * 32 + lane];
-      const float *wr = w2 + k * E2 + q * 16;
-#pragma unroll
-      for (int o = 0; o < 16; ++o)
-        if (q * 16 + o < E2) {
-          const float wv = wr[o];
-          z[o] = fmaf(hv, wv, z[o]);
-          dz[o] = fmaf(dv, wv, dz[o]);
-        }
-    }
-#pragma unroll
-    for (int o = 0; o < 16; ++o) {
-      const int col = q * 16 + o;
-      if (col < E2) {
-        const float t = tanhf(z[o]);
-        const int src = (col / D::Z2) * 32 + lane;
-        const float h2 = t + h1s[src];
-        const float dh2 = (1.f - t * t) * dz[o] + d1s[src];
-#pragma unroll
-        for (int c = 0; c < 10; ++c) {
-          const float dtc = dT[c * E2 + col];
-          u[c] = fmaf(dtc, h2, u[c]);
-          v[c] = fmaf(dtc, dh2, v[c]);
-        }
-      }
-    }
-  }
-  __syncwarp();
-  float R[10];
-  env_row(sn, xh, R);
-  float gst = 0.f;
-#pragma unroll
-  for (int c = 0; c < 10; ++c) gst = fmaf(R[c], v[c], gst);
-  float gx[3];
-  row_adjoint(gm, inv_std, u, gst, gx);
-  if (act) {
-    atomicAdd(&F4[frame_base + jj], make_float4(-gx[0], -gx[1], -gx[2], 0.f));
-    fi0 += gx[0]; fi1 += gx[1]; fi2 += gx[2];
-#pragma unroll
-    for (int p = 0; p < 3; ++p)
-#pragma unroll
-      for (int qq = 0; qq < 3; ++qq) vir[p * 3 + qq] -= gm.x[p] * gx[qq];
-  }
-}
-
 // Adjoint of one round of rows of a compressed net (row = lane): h and
 // dh/ds~ = dh/dx0 from the row's table entry (float4 loads along w), u =
 // dT.h, v = dT.dh, then the same env-row adjoint as the MLP path.
@@ -489,26 +267,24 @@ __device__ __forceinline__ void embed_rows_bwd_cmp(const float *__restrict__ coe
   }
 }
 
-template <int E0, int E1, int E2, bool CMP>
+template <int E2>
 __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti, const float *__restrict__ pos,
                                                    const int32_t *__restrict__ perm, const float *__restrict__ box,
                                                    const int32_t *__restrict__ nbrs, const float *__restrict__ Tin,
                                                    const float *__restrict__ dG, float4 *__restrict__ F4,
                                                    double *__restrict__ virial) {
-  using ED = EmbedDims<E0, E1, E2>;
+  constexpr int NQ = (E2 + 31) / 32;
   extern __shared__ float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const int A = M.A;
-  float *wsm = smem;
-  const int r1 = (A * E2 > 64 * 8 + 2 * E1 * 32) ? A * E2 : 64 * 8 + 2 * E1 * 32;
+  const int r1 = A * E2 > 64 * 8 ? A * E2 : 64 * 8;
   const int per_warp = r1 + 10 * E2 + 20 * A;
-  float *bufA = smem + (CMP ? 0 : M.ntypes * ED::NW) + warp * per_warp;  // dG, later rows + h1/dh1 staging
+  float *bufA = smem + warp * per_warp;  // dG, later rows
   float *bufB = bufA + r1;                                   // X, later dT
   float *Qs = bufB + 10 * E2;                                // 10 x A
   float *dQs = Qs + 10 * A;                                  // 10 x A
   __shared__ double vsm[9];
   if (threadIdx.x < 9) vsm[threadIdx.x] = 0.0;
-  if (!CMP) load_nets<E0, E1, E2>(M, ti, wsm);
   __syncthreads();
   const int f = blockIdx.y;
   const int a = blockIdx.x * wpb + warp;
@@ -543,9 +319,9 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
       dQs[e] = dq;
     }
     __syncwarp();
-    float dX[ED::NQ][10];
+    float dX[NQ][10];
 #pragma unroll
-    for (int q = 0; q < ED::NQ; ++q) {
+    for (int q = 0; q < NQ; ++q) {
       const int col = q * 32 + lane;
 #pragma unroll
       for (int c = 0; c < 10; ++c) dX[q][c] = 0.f;
@@ -575,7 +351,7 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
     }
     __syncwarp();
 #pragma unroll
-    for (int q = 0; q < ED::NQ; ++q) {
+    for (int q = 0; q < NQ; ++q) {
       const int col = q * 32 + lane;
       if (col < E2)
 #pragma unroll
@@ -591,12 +367,10 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
     const float inv_std = M.inv_std[ti], mean = M.mean[ti];
     const unsigned lt = (1u << lane) - 1u;
     float *rowbuf = bufA;  // 64 rows x 8 floats
-    float *h1s = bufA + 64 * 8, *d1s = h1s + E1 * 32;
     float fi0 = 0.f, fi1 = 0.f, fi2 = 0.f;
     const size_t frame_base = (size_t)f * D.N;
     for (int tj = 0; tj < D.ntypes; ++tj) {
-      const float *W = wsm + tj * ED::NW;
-      const int32_t *nb = nbrs + g * D.S + D.col[tj];
+        const int32_t *nb = nbrs + g * D.S + D.col[tj];
       const int sel = D.sel[tj], cnt_j = D.offs[tj + 1] - D.offs[tj];
       int nbuf = 0;
       const int total = sel * nim;
@@ -625,13 +399,9 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
         nbuf += __popc(m);
         __syncwarp();
         if (nbuf >= 32) {
-          if constexpr (CMP)
-            embed_rows_bwd_cmp<E2>(M.cmp_coeff[ti * M.ntypes + tj], M.cmp_srmin[ti * M.ntypes + tj],
-                                   M.cmp_delta[ti * M.ntypes + tj], M.ngrids, 32, rowbuf, bufB, inv_std, mean,
-                                   lane, fi0, fi1, fi2, vir, F4, frame_base);
-          else
-            embed_rows_bwd<E0, E1, E2>(W, 32, rowbuf, bufB, h1s, d1s, inv_std, mean, lane, fi0, fi1, fi2,
-                                       vir, F4, frame_base);
+          embed_rows_bwd_cmp<E2>(M.cmp_coeff[ti * M.ntypes + tj], M.cmp_srmin[ti * M.ntypes + tj],
+                                 M.cmp_delta[ti * M.ntypes + tj], M.ngrids, 32, rowbuf, bufB, inv_std, mean,
+                                 lane, fi0, fi1, fi2, vir, F4, frame_base);
           const int rem = nbuf - 32;
           if (lane < rem)
             for (int c = 0; c < 8; ++c) rowbuf[lane * 8 + c] = rowbuf[(32 + lane) * 8 + c];
@@ -640,13 +410,9 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
         }
       }
       if (nbuf > 0) {
-        if constexpr (CMP)
-          embed_rows_bwd_cmp<E2>(M.cmp_coeff[ti * M.ntypes + tj], M.cmp_srmin[ti * M.ntypes + tj],
-                                 M.cmp_delta[ti * M.ntypes + tj], M.ngrids, nbuf, rowbuf, bufB, inv_std, mean,
-                                 lane, fi0, fi1, fi2, vir, F4, frame_base);
-        else
-          embed_rows_bwd<E0, E1, E2>(W, nbuf, rowbuf, bufB, h1s, d1s, inv_std, mean, lane, fi0, fi1, fi2,
-                                     vir, F4, frame_base);
+        embed_rows_bwd_cmp<E2>(M.cmp_coeff[ti * M.ntypes + tj], M.cmp_srmin[ti * M.ntypes + tj],
+                               M.cmp_delta[ti * M.ntypes + tj], M.ngrids, nbuf, rowbuf, bufB, inv_std, mean,
+                               lane, fi0, fi1, fi2, vir, F4, frame_base);
       }
       __syncwarp();
     }
@@ -840,68 +606,46 @@ __global__ void k_finalize(int NF, int N, const float4 *__restrict__ F4, float *
   if (g < nE && !isfinite(energy[g])) atomicOr(status, DPB_ST_NONFINITE);
 }
 
-// Explicit instantiation helpers used by the C ABI dispatch.
-template <int E0, int E1, int E2>
-size_t embed_fwd_smem(int ntypes) {
-  return (size_t)(ntypes * EmbedDims<E0, E1, E2>::NW + 8 * embed_fwd_warp_floats<E0, E1, E2>()) * sizeof(float);
-}
-template <int E0, int E1, int E2>
-size_t embed_bwd_smem(int ntypes, int A) {
-  const int r1 = (A * E2 > 64 * 8 + 2 * E1 * 32) ? A * E2 : 64 * 8 + 2 * E1 * 32;
-  return (size_t)(ntypes * EmbedDims<E0, E1, E2>::NW + 8 * (r1 + 10 * E2 + 20 * A)) * sizeof(float);
-}
-
-template <int E0, int E1, int E2>
-int launch_embed_fwd(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
-                     const float *box, const int32_t *nbrs, float *T, float *G, cudaStream_t st) {
+template <int E2>
+int launch_embed_fwd_cmp(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
+                         const float *box, const int32_t *nbrs, float *T, float *G, cudaStream_t st) {
   const int cnt = D.offs[ti + 1] - D.offs[ti];
   if (cnt == 0) return DPB_OK;
   dim3 grid((cnt + 7) / 8, D.F);
-  if (M.ngrids > 0) {
-    size_t smem = embed_fwd_smem<E0, E1, E2>(0);
-    cudaFuncSetAttribute(k_embed_fwd<E0, E1, E2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_embed_fwd<E0, E1, E2, true><<<grid, 256, smem, st>>>(M, D, ti, pos, perm, box, nbrs, T, G);
-  } else {
-    size_t smem = embed_fwd_smem<E0, E1, E2>(M.ntypes);
-    cudaFuncSetAttribute(k_embed_fwd<E0, E1, E2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_embed_fwd<E0, E1, E2, false><<<grid, 256, smem, st>>>(M, D, ti, pos, perm, box, nbrs, T, G);
-  }
+  const size_t smem = (size_t)8 * embed_fwd_warp_floats<E2>() * sizeof(float);
+  cudaFuncSetAttribute(k_embed_fwd<E2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_embed_fwd<E2><<<grid, 256, smem, st>>>(M, D, ti, pos, perm, box, nbrs, T, G);
   count_launch();
   DPB_LAUNCH_CHECK();
   return DPB_OK;
 }
 
-template <int E0, int E1, int E2>
-int launch_embed_bwd(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
-                     const float *box, const int32_t *nbrs, const float *T, const float *dG, float4 *F4,
-                     double *virial, cudaStream_t st) {
+template <int E2>
+int launch_embed_bwd_cmp(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
+                         const float *box, const int32_t *nbrs, const float *T, const float *dG, float4 *F4,
+                         double *virial, cudaStream_t st) {
   const int cnt = D.offs[ti + 1] - D.offs[ti];
   if (cnt == 0) return DPB_OK;
   dim3 grid((cnt + 7) / 8, D.F);
-  if (M.ngrids > 0) {
-    size_t smem = embed_bwd_smem<E0, E1, E2>(0, M.A);
-    cudaFuncSetAttribute(k_embed_bwd<E0, E1, E2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_embed_bwd<E0, E1, E2, true><<<grid, 256, smem, st>>>(M, D, ti, pos, perm, box, nbrs, T, dG, F4, virial);
-  } else {
-    size_t smem = embed_bwd_smem<E0, E1, E2>(M.ntypes, M.A);
-    cudaFuncSetAttribute(k_embed_bwd<E0, E1, E2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_embed_bwd<E0, E1, E2, false><<<grid, 256, smem, st>>>(M, D, ti, pos, perm, box, nbrs, T, dG, F4, virial);
-  }
+  const int r1 = M.A * E2 > 64 * 8 ? M.A * E2 : 64 * 8;
+  const size_t smem = (size_t)8 * (r1 + 10 * E2 + 20 * M.A) * sizeof(float);
+  cudaFuncSetAttribute(k_embed_bwd<E2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  k_embed_bwd<E2><<<grid, 256, smem, st>>>(M, D, ti, pos, perm, box, nbrs, T, dG, F4, virial);
   count_launch();
   DPB_LAUNCH_CHECK();
   return DPB_OK;
 }
 
-template int launch_embed_fwd<25, 50, 100>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
-                                           const float *, const int32_t *, float *, float *, cudaStream_t);
-template int launch_embed_bwd<25, 50, 100>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
-                                           const float *, const int32_t *, const float *, const float *, float4 *,
-                                           double *, cudaStream_t);
-template int launch_embed_fwd<32, 32, 64>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
-                                          const float *, const int32_t *, float *, float *, cudaStream_t);
-template int launch_embed_bwd<32, 32, 64>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
-                                          const float *, const int32_t *, const float *, const float *, float4 *,
-                                          double *, cudaStream_t);
+template int launch_embed_fwd_cmp<100>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
+                                       const float *, const int32_t *, float *, float *, cudaStream_t);
+template int launch_embed_fwd_cmp<64>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
+                                      const float *, const int32_t *, float *, float *, cudaStream_t);
+template int launch_embed_bwd_cmp<100>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
+                                       const float *, const int32_t *, const float *, const float *, float4 *,
+                                       double *, cudaStream_t);
+template int launch_embed_bwd_cmp<64>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
+                                      const float *, const int32_t *, const float *, const float *, float4 *, double *,
+                                      cudaStream_t);
 
 int launch_sgemm(int Mrows, int Nc, int K, const float *A, int lda, RowMap rm, const float *B, const Epi &ep,
                  cudaStream_t st) {

@@ -1,6 +1,8 @@
 // Internal interfaces shared between the translation units of libdpb200.
 #pragma once
 #include "eval_common.cuh"
+#include <algorithm>
+#include <cmath>
 #include <vector>
 
 struct dpb_model {
@@ -16,6 +18,14 @@ struct dpb_model {
 };
 
 namespace dpb {
+// 2^k with x 2^k in (2^13, 2^14] (x > 0; 1 for x = 0 or non-finite), k
+// clamped to [-40, 40].
+inline float pow2_scale_to_2p14(double x) {
+  if (!(x > 0.0) || !std::isfinite(x)) return 1.f;
+  int k = 14 - (int)std::ceil(std::log2(x));
+  k = std::max(-40, std::min(40, k));
+  return std::ldexp(1.f, k);
+}
 int eval_impl(const dpb_model *m, int precision, const float *pos, const int32_t *perm, int natoms, int nframes,
               const int *type_count, const float *box, const int32_t *nbrs, const int *sel, double *energy,
               float *atom_energy, float *force, double *virial, uint32_t *status, void *workspace,

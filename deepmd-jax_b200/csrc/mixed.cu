@@ -1,6 +1,5 @@
 // Mixed-precision (BF16 tensor-core) evaluation path.
-#include "internal.cuh"
-#include "tc.cuh"
+#include "rows.cuh"
 
 namespace dpb {
 
@@ -111,20 +110,6 @@ struct HalfSplit {
   static_assert(S1 % 8 == 0 && S2 % 8 == 0 && H0LO1 % 2 == 0 && A0C % 8 == 0, "pair-aligned split");
 };
 
-constexpr int kBlkAtoms = 8;    // centre atoms per block
-constexpr int kRblkBytes = 128 * 128 * 2;
-
-__host__ __device__ constexpr int round1k(int x) { return (x + 1023) / 1024 * 1024; }
-
-// Bounded wait on the block's MMA barrier, made uniform across the block.
-#define MIX_WAIT()                                  \
-  do {                                              \
-    const bool w_ = tc::mbar_wait(&mbar, ph);       \
-    ph ^= 1;                                        \
-    ok = __syncthreads_and(w_ && ok) != 0;          \
-    tc::fence_after_sync();                         \
-  } while (0)
-
 // Asynchronous copy of one net's shared-memory image (BF16 B tiles and the
 // FP32 first layer / biases); completes at the caller's cp_async_wait.
 template <int E0, int E1, int E2>
@@ -135,13 +120,6 @@ __device__ __forceinline__ void mix_load_net(const DevModel &M, int k, char *net
   const float *sm = M.net_small[k];
   for (int e = threadIdx.x; e < D::NSMALL / 4; e += blockDim.x) tc::cp_async16(small + 4 * e, sm + 4 * e);
   tc::cp_async_commit();
-}
-
-// L2 prefetch of [base, base + bytes), one line per thread and step (the
-// persistent CTAs issue it for their next block while working on this one).
-__device__ __forceinline__ void prefetch_range_l2(const void *base, size_t bytes) {
-  const char *b = static_cast<const char *>(base);
-  for (size_t o = (size_t)threadIdx.x * 128; o < bytes; o += (size_t)blockDim.x * 128) tc::prefetch_l2(b + o);
 }
 
 // Row geometry of the mixed form: the guarded norm, s(r) of utils.py:29-32
@@ -197,245 +175,6 @@ __device__ __forceinline__ void mix_row_env(float4 rb, float rcut, float inv_std
   const float inv_rp = __fdividef(1.f, gm.r + 1e-16f);
   const float xh[3] = {gm.x[0] * inv_rp, gm.x[1] * inv_rp, gm.x[2] * inv_rp};
   env_row(sn, xh, R);
-}
-
-// One round of compaction over CPT * blockDim candidates (atom slot,
-// neighbour slot, image) of the block for neighbour type tj: thread t takes
-// the CPT consecutive candidates base + t * CPT + k, issues all of their
-// gathers (neighbour index, then position and user index from posS) before
-// using any, and the
-// kept rows are appended to rowbuf in candidate order (so rows stay sorted by
-// atom slot) as (x, y, z, packed), packed = (neighbour user index << 3) | slot.
-// With one image per pair (nim == 1, boxes wider than 2 rcut) the row's
-// displacement is the nearest image d - L rint(d / L), which equals the
-// reference's (d - L/2) mod L - L/2 (utils.py:24-26) up to rounding (the mixed
-// form is held to a tolerance, not to bits), and the keep test is |x| <
-// rcut + 1e-3 A: every row with s(r) != 0 is kept, and a kept row with
-// s(r) = 0 adds exact zeros (R~ = 0, ds/dr = 0).  With several images the
-// reference's displacement and s(r) decide.  The unread rows [rowstart, rowcount) of earlier rounds (fewer than
-// 128) are first moved to the front.
-template <int CPT>
-__device__ __forceinline__ void mix_compact_round(const SysDesc &D, const DevModel &M, int tj, int base, int total,
-                                                  int per_atom, int nim, int3 ni, float3 L, size_t g0,
-                                                  size_t frame_base, const float3 *ri_s,
-                                                  const float4 *__restrict__ posS, const int32_t *nbrs, float4 *rowbuf,
-                                                  int *wcnt, int &rowstart, int &rowcount) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (rowstart > 0) {
-    const int rem = rowcount - rowstart;  // < 128 <= blockDim
-    float4 carry = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (tid < rem) carry = rowbuf[rowstart + tid];
-    __syncthreads();
-    if (tid < rem) rowbuf[tid] = carry;
-    rowstart = 0;
-    rowcount = rem;
-  }
-  const int cnt_j = D.offs[tj + 1] - D.offs[tj];
-  const int p0 = base + tid * CPT;
-  int idx[CPT], slotk[CPT], mimgk[CPT];
-  int slot = p0 / per_atom, rem = p0 - slot * per_atom;  // advanced incrementally below
-#pragma unroll
-  for (int k = 0; k < CPT; ++k) {
-    const int p = p0 + k;
-    idx[k] = cnt_j;
-    slotk[k] = 0;
-    mimgk[k] = 0;
-    if (p < total) {
-      const int sidx = nim == 1 ? rem : rem / nim;
-      slotk[k] = slot;
-      mimgk[k] = rem - sidx * nim;
-      idx[k] = nbrs[(g0 + slot) * D.S + D.col[tj] + sidx] & DPB_NBR_INDEX_MASK;
-    }
-    if (++rem == per_atom) {
-      rem = 0;
-      ++slot;
-    }
-  }
-  int src[CPT];
-  float3 pj[CPT];
-#pragma unroll
-  for (int k = 0; k < CPT; ++k) {
-    src[k] = -1;
-    pj[k] = make_float3(0.f, 0.f, 0.f);
-    if (idx[k] < cnt_j) {
-      const float4 q = posS[frame_base + D.offs[tj] + idx[k]];
-      pj[k] = make_float3(q.x, q.y, q.z);
-      src[k] = __float_as_int(q.w);
-    }
-  }
-  float4 rv[CPT];
-  unsigned keep = 0;
-  if (nim == 1) {
-    const float3 inv_l = make_float3(1.f / L.x, 1.f / L.y, 1.f / L.z);
-    const float rk = M.rcut + 1e-3f, rk2 = rk * rk;
-#pragma unroll
-    for (int k = 0; k < CPT; ++k) {
-      rv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (src[k] >= 0) {
-        const float3 ri = ri_s[slotk[k]];
-        const float dx = pj[k].x - ri.x, dy = pj[k].y - ri.y, dz = pj[k].z - ri.z;
-        const float ax = fmaf(-L.x, rintf(dx * inv_l.x), dx), ay = fmaf(-L.y, rintf(dy * inv_l.y), dy),
-                    az = fmaf(-L.z, rintf(dz * inv_l.z), dz);
-        if (ax * ax + ay * ay + az * az < rk2) {
-          keep |= 1u << k;
-          rv[k] = make_float4(ax, ay, az, __int_as_float((src[k] << 3) | slotk[k]));
-        }
-      }
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < CPT; ++k) {
-      rv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (src[k] >= 0) {
-        const float3 x = rel_coord(ri_s[slotk[k]], pj[k], L, ni, mimgk[k]);
-        RowGeom gm;
-        row_geom(x, M.rcut, gm);
-        if (gm.s != 0.f) {
-          keep |= 1u << k;
-          rv[k] = make_float4(x.x, x.y, x.z, __int_as_float((src[k] << 3) | slotk[k]));
-        }
-      }
-    }
-  }
-  // block-wide exclusive scan of the per-thread counts
-  const int c = __popc(keep);
-  int incl = c;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += t;
-  }
-  if (lane == 31) wcnt[warp] = incl;
-  __syncthreads();
-  int off = 0, tot = 0;
-  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-    if (w < warp) off += wcnt[w];
-    tot += wcnt[w];
-  }
-  int o = rowcount + off + incl - c;
-#pragma unroll
-  for (int k = 0; k < CPT; ++k)
-    if (keep >> k & 1u) rowbuf[o++] = rv[k];
-  rowcount += tot;
-  __syncthreads();
-}
-
-// Row store of list mode (one image per pair, boxes wider than 2 rcut):
-// k_mix_rows compacts the neighbour rows of every block of 8 centre atoms and
-// neighbour type once per evaluation, rows of block g0 and type tj at rows_g
-// + g0 * kRowStoreCap + nb * col[tj] (in candidate order, so sorted by atom
-// slot, as mix_compact_round leaves them), their count at rcnt[g0 * ntypes +
-// tj].  The forward and the adjoint embedding kernels then stream them.
-constexpr int kRowStoreCap = 192;  // neighbour slots per atom the store holds (sum of sel)
-
-// The blocks whose rows the store holds.
-__device__ __forceinline__ bool row_store_covers(const SysDesc &D, const float4 *rows_g, int nim) {
-  return rows_g != nullptr && nim == 1 && D.S <= kRowStoreCap;
-}
-
-// One warp per (block of 8 centre atoms of type ti, neighbour type tj),
-// kRowsCpt rounds of 32 candidates (atom slot, list slot) at a time in
-// candidate order: all of their list entries are loaded, then all of their
-// neighbour positions gathered from posS, before any is used (the chain is
-// two dependent loads per round); the nearest-image displacement and keep
-// test are those of mix_compact_round (same arithmetic, so the same rows),
-// and the kept rows are appended round by round with a ballot.  Blocks
-// outside the store (several images) are left to the embedding kernels' own
-// compaction.
-constexpr int kRowsCpt = 4;
-
-__global__ void __launch_bounds__(256) k_mix_rows(DevModel M, SysDesc D, int ti, const float4 *__restrict__ posS,
-                                                 const float *__restrict__ box, const int32_t *__restrict__ nbrs,
-                                                 float4 *__restrict__ rows_g, int *__restrict__ rcnt) {
-  const int lane = threadIdx.x & 31;
-  const int wg = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int cnt_i = D.offs[ti + 1] - D.offs[ti];
-  const int nbpf = (cnt_i + kBlkAtoms - 1) / kBlkAtoms;
-  const int blk = wg / D.ntypes, tj = wg - blk * D.ntypes;
-  if (blk >= nbpf * D.F) return;
-  const int f = blk / nbpf, a0 = (blk - f * nbpf) * kBlkAtoms;
-  const int nb = min(kBlkAtoms, cnt_i - a0);
-  const size_t g0 = (size_t)f * D.N + D.offs[ti] + a0;
-  const size_t frame_base = (size_t)f * D.N;
-  const int bs = box_slot(D, g0, f);
-  const float3 L = make_float3(box[bs * 3], box[bs * 3 + 1], box[bs * 3 + 2]);
-  const int3 ni = image_range(L, M.rcut);
-  if (!row_store_covers(D, rows_g, (2 * ni.x + 1) * (2 * ni.y + 1) * (2 * ni.z + 1))) return;
-  const float3 inv_l = make_float3(1.f / L.x, 1.f / L.y, 1.f / L.z);
-  const float rk = M.rcut + 1e-3f, rk2 = rk * rk;
-  const int sel = D.sel[tj], cnt_j = D.offs[tj + 1] - D.offs[tj], total = nb * sel;
-  const int col = D.col[tj], jbase = D.offs[tj];
-  // the block's centre positions, one per lane
-  const float4 cl = lane < nb ? posS[g0 + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-  float4 *out = rows_g + g0 * kRowStoreCap + (size_t)nb * col;
-  int n = 0;
-  for (int base = 0; base < total; base += 32 * kRowsCpt) {
-    int idx[kRowsCpt], slot[kRowsCpt];
-#pragma unroll
-    for (int k = 0; k < kRowsCpt; ++k) {
-      const int p = base + 32 * k + lane;
-      slot[k] = p / sel;
-      idx[k] = p < total ? nbrs[(g0 + slot[k]) * D.S + col + (p - slot[k] * sel)] & DPB_NBR_INDEX_MASK : cnt_j;
-    }
-    float4 q[kRowsCpt];
-#pragma unroll
-    for (int k = 0; k < kRowsCpt; ++k)
-      q[k] = idx[k] < cnt_j ? posS[frame_base + jbase + idx[k]] : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int k = 0; k < kRowsCpt; ++k) {
-      const int sl = min(slot[k], kBlkAtoms - 1);
-      const float cx = __shfl_sync(0xffffffffu, cl.x, sl), cy = __shfl_sync(0xffffffffu, cl.y, sl),
-                  cz = __shfl_sync(0xffffffffu, cl.z, sl);
-      float4 rv = make_float4(0.f, 0.f, 0.f, 0.f);
-      bool keep = false;
-      if (idx[k] < cnt_j) {
-        const float dx = q[k].x - cx, dy = q[k].y - cy, dz = q[k].z - cz;
-        const float ax = fmaf(-L.x, rintf(dx * inv_l.x), dx), ay = fmaf(-L.y, rintf(dy * inv_l.y), dy),
-                    az = fmaf(-L.z, rintf(dz * inv_l.z), dz);
-        if (ax * ax + ay * ay + az * az < rk2) {
-          keep = true;
-          rv = make_float4(ax, ay, az, __int_as_float((__float_as_int(q[k].w) << 3) | slot[k]));
-        }
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, keep);
-      if (keep) out[n + __popc(m & ((1u << lane) - 1u))] = rv;
-      n += __popc(m);
-    }
-  }
-  if (lane == 0) rcnt[g0 * M.ntypes + tj] = n;
-}
-
-// One round of a row stream: the unread rows of earlier rounds move to the
-// front (as in mix_compact_round), then up to RPT * blockDim rows [base,
-// total) of the stored list are appended, RPT coalesced 16-byte loads per
-// thread issued before any store.
-template <int RPT>
-__device__ __forceinline__ void mix_stream_round(const float4 *__restrict__ src, int base, int total, float4 *rowbuf,
-                                                 int &rowstart, int &rowcount) {
-  const int tid = threadIdx.x;
-  if (rowstart > 0) {
-    const int rem = rowcount - rowstart;  // < 128 <= blockDim
-    float4 carry = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (tid < rem) carry = rowbuf[rowstart + tid];
-    __syncthreads();
-    if (tid < rem) rowbuf[tid] = carry;
-    rowstart = 0;
-    rowcount = rem;
-  }
-  const int n = min(RPT * (int)blockDim.x, total - base);
-  float4 v[RPT];
-#pragma unroll
-  for (int k = 0; k < RPT; ++k) {
-    const int i = tid + k * (int)blockDim.x;
-    if (i < n) v[k] = src[base + i];
-  }
-#pragma unroll
-  for (int k = 0; k < RPT; ++k) {
-    const int i = tid + k * (int)blockDim.x;
-    if (i < n) rowbuf[rowcount + i] = v[k];
-  }
-  rowcount += n;
-  __syncthreads();
 }
 
 // 8 floats times s as FP16, round to nearest, saturating at the largest
@@ -625,6 +364,7 @@ __device__ __forceinline__ float row_stilde(float4 rb, float rcut, float inv_std
 // TMEM across all tiles of both neighbour types.  The block epilogue writes
 // T / Nnbrs (FP32) and the descriptor G (BF16, dpmodel.py:74-78).  Only the
 // current neighbour type's net is resident (2 CTAs per SM).
+constexpr int kRblkBytes = 128 * 128 * 2;
 constexpr int kFwdThreads = 256;
 constexpr int kFwdCpt = 2;  // compaction candidates per thread, forward
 constexpr int kRowCapFwd = 128 + kFwdThreads * kFwdCpt;  // the carry (< 128) + one compaction round
@@ -2101,44 +1841,16 @@ static int launch_mix_dT(const DevModel &M, size_t NF, const float *T, const __h
   return DPB_OK;
 }
 
-// Positions in type-sorted order with each atom's frame-local user index:
-// posS[f N + k] = (r of atom perm[k] of frame f, perm[k]) - one 16-byte
-// gather per neighbour in the mixed embedding kernels.
-__global__ void k_pos_sorted(size_t NF, int N, const float *__restrict__ pos, const int32_t *__restrict__ perm,
-                             float4 *__restrict__ posS) {
-  const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g < NF) {
-    const size_t f = g / N;
-    const int k = (int)(g - f * N);
-    const int src = perm ? perm[k] : k;
-    const float *p = pos + (f * N + src) * 3;
-    posS[g] = make_float4(p[0], p[1], p[2], __int_as_float(src));
-  }
-}
-
-static int launch_pos_sorted(const SysDesc &D, const float *pos, const int32_t *perm, float4 *posS,
-                             cudaStream_t st) {
-  const size_t NF = (size_t)D.N * D.F;
-  k_pos_sorted<<<(unsigned)((NF + 255) / 256), 256, 0, st>>>(NF, D.N, pos, perm, posS);
-  count_launch();
-  DPB_LAUNCH_CHECK();
-  return DPB_OK;
-}
-
-// rows / rcnt (may be null): the row store, built here by k_mix_rows and
+// rows / rcnt (may be null): the row store, built here by k_rows and
 // streamed by the forward and the adjoint embedding kernels.
 int mixed_descriptors(const DevModel &M, const SysDesc &D, const float4 *posS, const float *box,
                       const int32_t *nbrs, float *T, __half *Gb, float4 *rows, int *rcnt, int *err,
                       cudaStream_t st) {
   if (M.ngrids > 0 || !M.emb_tuned) return DPB_ERR_UNSUPPORTED;  // the FP32 kernels give T and G
   prof_begin(PROF_MIXED_EMBED_FWD, st);
-  for (int ti = 0; ti < M.ntypes && rows; ++ti) {
-    const int cnt = D.offs[ti + 1] - D.offs[ti];
-    const size_t warps = (size_t)(cnt + kBlkAtoms - 1) / kBlkAtoms * D.F * D.ntypes;
-    if (!cnt) continue;
-    k_mix_rows<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(M, D, ti, posS, box, nbrs, rows, rcnt);
-    count_launch();
-    DPB_LAUNCH_CHECK();
+  if (rows) {
+    const int rc = launch_rows(M, D, kBlkAtoms, posS, box, nbrs, rows, rcnt, st);
+    if (rc) return rc;
   }
   for (int ti = 0; ti < M.ntypes; ++ti) {
     int rc = (M.E2 == 100)
@@ -2165,13 +1877,13 @@ __global__ void k_f32_to_f16(const float4 *__restrict__ a, uint2 *__restrict__ b
   }
 }
 
-template <int E0, int E1, int E2>
-int launch_embed_fwd(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
-                     const float *box, const int32_t *nbrs, float *T, float *G, cudaStream_t st);
-template <int E0, int E1, int E2>
-int launch_embed_bwd(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
-                     const float *box, const int32_t *nbrs, const float *T, const float *dG, float4 *F4,
-                     double *virial, cudaStream_t st);
+template <int E2>
+int launch_embed_fwd_cmp(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
+                         const float *box, const int32_t *nbrs, float *T, float *G, cudaStream_t st);
+template <int E2>
+int launch_embed_bwd_cmp(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
+                         const float *box, const int32_t *nbrs, const float *T, const float *dG, float4 *F4,
+                         double *virial, cudaStream_t st);
 int launch_embed_fwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
                          const int32_t *, float *, float *, cudaStream_t);
 int launch_embed_bwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
@@ -2191,8 +1903,8 @@ static int mixed_eval_compressed(const DevModel &M, const SysDesc &D, const floa
   prof_begin(PROF_EMBED_FWD, st);
   for (int ti = 0; ti < M.ntypes; ++ti) {
     rc = !M.emb_tuned   ? launch_embed_fwd_gen(M, D, ti, pos, perm, box, nbrs, T, dG, st)
-         : M.E2 == 100 ? launch_embed_fwd<25, 50, 100>(M, D, ti, pos, perm, box, nbrs, T, dG, st)
-                       : launch_embed_fwd<32, 32, 64>(M, D, ti, pos, perm, box, nbrs, T, dG, st);
+         : M.E2 == 100 ? launch_embed_fwd_cmp<100>(M, D, ti, pos, perm, box, nbrs, T, dG, st)
+                       : launch_embed_fwd_cmp<64>(M, D, ti, pos, perm, box, nbrs, T, dG, st);
     if (rc) return rc;
   }
   k_f32_to_f16<<<(unsigned)((NG / 4 + 255) / 256), 256, 0, st>>>(reinterpret_cast<const float4 *>(dG),
@@ -2207,8 +1919,8 @@ static int mixed_eval_compressed(const DevModel &M, const SysDesc &D, const floa
   prof_begin(PROF_EMBED_BWD, st);
   for (int ti = 0; ti < M.ntypes; ++ti) {
     rc = !M.emb_tuned   ? launch_embed_bwd_gen(M, D, ti, pos, perm, box, nbrs, T, dG, F4, virial, st)
-         : M.E2 == 100 ? launch_embed_bwd<25, 50, 100>(M, D, ti, pos, perm, box, nbrs, T, dG, F4, virial, st)
-                       : launch_embed_bwd<32, 32, 64>(M, D, ti, pos, perm, box, nbrs, T, dG, F4, virial, st);
+         : M.E2 == 100 ? launch_embed_bwd_cmp<100>(M, D, ti, pos, perm, box, nbrs, T, dG, F4, virial, st)
+                       : launch_embed_bwd_cmp<64>(M, D, ti, pos, perm, box, nbrs, T, dG, F4, virial, st);
     if (rc) return rc;
   }
   prof_end(PROF_EMBED_BWD, st);
