@@ -62,24 +62,28 @@ void split_net_image(int E2, const float *w0, const float *b0, const float *w1, 
                      const float *b2, double s_lo, double s_hi, std::vector<char> &img, std::vector<float> &small);
 int split_block_atoms(const SysDesc &D);
 int split_embed_fwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
-                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, cudaStream_t st);
+                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, float *gmax,
+                    cudaStream_t st);
 int split_embed_bwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
                     const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, const float *dG, float4 *F4,
                     double *virial, cudaStream_t st);
 template <int E2>
 int launch_embed_fwd_cmp(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
-                         const int32_t *, float *, float *, cudaStream_t);
+                         const int32_t *, float *, float *, float *, cudaStream_t);
 template <int E2>
 int launch_embed_bwd_cmp(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
                          const int32_t *, const float *, const float *, float4 *, double *, cudaStream_t);
-int launch_sgemm(int, int, int, const float *, int, RowMap, const float *, const Epi &, cudaStream_t);
+// fitting GEMMs on the tensor cores (gemm_split.cu)
+size_t gemm_tiles_halves(int N, int K);
+int launch_gemm_tiles(const float *w, int N, int K, int sn, int sk, float scale, __half *out);
+int launch_gemm_split(const GemmArgs &g, cudaStream_t st);
 // any embedding shape (eval_general.cu)
 int launch_embed_fwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
-                         const int32_t *, float *, float *, cudaStream_t);
+                         const int32_t *, float *, float *, float *, cudaStream_t);
 int launch_embed_bwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
                          const int32_t *, const float *, const float *, float4 *, double *, cudaStream_t);
-int launch_fit_energy(int, RowMap, int, const float *, const float *, const float *, const float *,
-                      const float *, float *, float *, double *, int, const int32_t *, cudaStream_t);
+int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, float *gZ, double *energy,
+                      const int32_t *seg, cudaStream_t st);
 int launch_finalize(int, int, const float4 *, float *, const float *, const int32_t *, float *, double *, int,
                     const float *, const int32_t *, uint32_t *, cudaStream_t);
 // mixed path (mixed.cu)
@@ -111,6 +115,16 @@ static int upload(dpb_model *m, const T *host, size_t n, const T **dev) {
   if (cudaMemcpy(p, host, n * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) return DPB_ERR_CUDA;
   *dev = (const T *)p;
   return DPB_OK;
+}
+
+// Stored weight tiles of one FP32 fitting GEMM, built on the device from the
+// uploaded matrix: B[n][k] = w[n sn + k sk].
+static int fit_tiles(dpb_model *m, const float *w, int N, int K, int sn, int sk, float scale, const __half **dev) {
+  void *p = nullptr;
+  if (cudaMalloc(&p, gemm_tiles_halves(N, K) * sizeof(__half)) != cudaSuccess) return DPB_ERR_CUDA;
+  m->allocs.push_back(p);
+  *dev = (const __half *)p;
+  return launch_gemm_tiles(w, N, K, sn, sk, scale, (__half *)p);
 }
 
 // B operand chunks of the mixed fitting kernel from a row-major matrix
@@ -279,7 +293,7 @@ extern "C" int dpb_model_create(const dpb_model_desc *d, dpb_model **out) {
     // per layer: max over inputs i of sum_o |W[i][o]|, max |dt| (1 without
     // residual), and max |w_out|: the bounds behind fit_gsc
     std::vector<double> rowsum(M.nfit + 1, 0.0), maxdt(M.nfit + 1, 1.0);
-    double wout_max = 0.0;
+    double wout_max = 0.0, hbound = 1.0;
     for (int l = 0; l <= M.nfit && rc == DPB_OK; ++l) {
       const int in = l == 0 ? K0 : M.FW[l - 1];
       const int outw = l == M.nfit ? 1 : M.FW[l];
@@ -292,10 +306,6 @@ extern "C" int dpb_model_create(const dpb_model_desc *d, dpb_model **out) {
       }
       rc = upload(m, kv.data(), kv.size(), &M.fw[t][l]);
       if (rc == DPB_OK) rc = upload(m, bv.data(), bv.size(), &M.fb[t][l]);
-      std::vector<float> kt((size_t)in * outw);
-      for (int i = 0; i < in; ++i)
-        for (int o = 0; o < outw; ++o) kt[(size_t)o * in + i] = kv[(size_t)i * outw + o];
-      if (rc == DPB_OK) rc = upload(m, kt.data(), kt.size(), &M.fwT[t][l]);
       const float *dt = (l < M.nfit && d->fit_dt) ? d->fit_dt[t * M.nfit + l] : nullptr;
       if (rc == DPB_OK && dt) rc = upload(m, dt, (size_t)outw, &M.fdt[t][l]);
       double wmax = 0.0;
@@ -309,8 +319,16 @@ extern "C" int dpb_model_create(const dpb_model_desc *d, dpb_model **out) {
       }
       if (dt)  // the kernel multiplies by dt or by 1: bound by both
         for (int o = 0; o < outw; ++o) maxdt[l] = std::max(maxdt[l], std::fabs((double)dt[o]));
-      if (l == M.nfit) wout_max = wmax;
-      else M.fit_wsc[t][l] = pow2_scale_to_2p14(wmax);
+      if (l == M.nfit) {
+        wout_max = wmax;
+      } else {
+        M.fit_wsc[t][l] = pow2_scale_to_2p14(wmax);
+        // |h_l| <= 1, plus max |dt| and the layer below's bound through a residual
+        hbound = dt ? maxdt[l] + hbound : 1.0;
+        M.fit_hsc[t][l] = pow2_scale_to_2p14(hbound);
+        if (rc == DPB_OK) rc = fit_tiles(m, M.fw[t][l], outw, in, 1, outw, M.fit_wsc[t][l], &M.fs_fwd[t][l]);
+        if (rc == DPB_OK) rc = fit_tiles(m, M.fw[t][l], in, outw, outw, 1, M.fit_wsc[t][l], &M.fs_adj[t][l]);
+      }
       if (rc == DPB_OK && M.mfw > 0) {
         // the tensor-core fitting's copy: every hidden width padded to mfw with zeros
         const int P = M.mfw, inp = l == 0 ? K0 : P, outp = l == M.nfit ? 1 : P;
@@ -424,11 +442,13 @@ static int fill_sys(const dpb_model *m, int natoms, int nframes, const int *type
   return DPB_OK;
 }
 
-// FP32 fitting chain (tiled SGEMMs with fused epilogues) for every centre
-// type: G -> per-atom energies (FP64 frame sums) and dE/dG written over G.
-// Hidden layer l has width FW[l]; a dt residual (utils.py:158-163) exists
-// only where FW[l] == FW[l-1], so every residual pairs equal widths.
-// w: scratch for the per-layer activations and adjoints.
+// FP32 fitting chain (tensor-core GEMMs of split operands with fused
+// epilogues, every centre type in one launch): G -> per-atom energies (FP64
+// frame sums) and dE/dG written over G.  Hidden layer l has width FW[l]; a dt
+// residual (utils.py:158-163) exists only where FW[l] == FW[l-1], so every
+// residual pairs equal widths.  Eatom holds each atom's largest |G| on entry (the
+// scale of layer 0's operand).  w: scratch for the per-layer activations and
+// adjoints.
 int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Eatom, double *energy, char *w,
                         cudaStream_t st) {
   const size_t NF = (size_t)D.N * D.F;
@@ -441,62 +461,89 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
   gz[1] = (float *)w; w += al(NF * FWM * 4);
   gh[0] = (float *)w; w += al(NF * FWM * 4);
   gh[1] = (float *)w; w += al(NF * FWM * 4);
-  int rc;
+  GemmArgs g{};
+  EnergyArgs en{};
+  int ty[kMaxTypes], n = 0;  // the types present
   for (int ti = 0; ti < M.ntypes; ++ti) {
     const int cnt = D.offs[ti + 1] - D.offs[ti];
     if (!cnt) continue;
-    const RowMap rm{cnt, D.N, D.offs[ti]};
-    const int Mrows = cnt * D.F;
-    for (int l = 0; l < L; ++l) {
-      const int out = M.FW[l], in = l == 0 ? K0 : M.FW[l - 1];
-      Epi ep{};
-      ep.bias = M.fb[ti][l];
-      ep.out1 = tb[l];
-      ep.out2 = hb[l];
-      ep.ld = out;
+    ty[n] = ti;
+    g.t[n].rm = en.t[n].rm = RowMap{cnt, D.N, D.offs[ti]};
+    g.t[n].Mrows = en.t[n].Mrows = cnt * D.F;
+    g.mt0[n + 1] = g.mt0[n] + (cnt * D.F + 127) / 128;
+    en.b0[n + 1] = en.b0[n] + (cnt * D.F + 7) / 8;
+    ++n;
+  }
+  g.ntypes = en.ntypes = n;
+  int rc;
+  for (int l = 0; l < L; ++l) {
+    g.A = l == 0 ? G : hb[l - 1];
+    g.lda = g.K = l == 0 ? K0 : M.FW[l - 1];
+    g.N = M.FW[l];
+    for (int k = 0; k < n; ++k) {
+      const int ti = ty[k];
+      GemmType &t = g.t[k];
+      t.B = M.fs_fwd[ti][l];
+      t.gmax = l == 0 ? Eatom : nullptr;
+      t.ascale = l == 0 ? 1.f : M.fit_hsc[ti][l - 1];
+      t.wscale = M.fit_wsc[ti][l];
+      t.ep = Epi{};
+      t.ep.bias = M.fb[ti][l];
+      t.ep.out1 = tb[l];
+      t.ep.out2 = hb[l];
+      t.ep.ld = g.N;
+      t.ep.mode = EPI_TANH;
       if (l > 0 && M.fdt[ti][l]) {
-        ep.mode = EPI_TANH_RES;
-        ep.dt = M.fdt[ti][l];
-        ep.hprev = hb[l - 1];
-      } else {
-        ep.mode = EPI_TANH;
+        t.ep.mode = EPI_TANH_RES;
+        t.ep.dt = M.fdt[ti][l];
+        t.ep.hprev = hb[l - 1];
       }
-      if (l == 0) rc = launch_sgemm(Mrows, out, in, G, K0, rm, M.fw[ti][0], ep, st);
-      else rc = launch_sgemm(Mrows, out, in, hb[l - 1], in, rm, M.fw[ti][l], ep, st);
-      if (rc) return rc;
     }
-    int cur = 0;
-    rc = launch_fit_energy(Mrows, rm, M.FW[L - 1], hb[L - 1], tb[L - 1], M.fw[ti][L], M.fb[ti][L],
-                           M.fdt[ti][L - 1], Eatom, gz[cur], energy, D.N, D.seg, st);
-    if (rc) return rc;
-    for (int l = L - 1; l >= 1; --l) {
-      // gH_{l-1} = gZ_l W_l^T (+ gH_l through layer l's residual)
-      const int out = M.FW[l - 1], in = M.FW[l];
-      Epi ep{};
-      ep.ld = out;
-      ep.tin = tb[l - 1];
+    if ((rc = launch_gemm_split(g, st))) return rc;
+  }
+  int cur = 0;
+  en.FWl = M.FW[L - 1];
+  en.N = D.N;
+  for (int k = 0; k < n; ++k) {
+    en.t[k].wfin = M.fw[ty[k]][L];
+    en.t[k].bfin = M.fb[ty[k]][L];
+    en.t[k].dtl = M.fdt[ty[k]][L - 1];
+  }
+  if ((rc = launch_fit_energy(en, hb[L - 1], tb[L - 1], Eatom, gz[cur], energy, D.seg, st))) return rc;
+  for (int l = L - 1; l >= 0; --l) {
+    // l >= 1: gH_{l-1} = gZ_l W_l^T (+ gH_l through layer l's residual); l = 0: dE/dG
+    g.A = gz[cur];
+    g.lda = g.K = M.FW[l];
+    g.N = l == 0 ? K0 : M.FW[l - 1];
+    for (int k = 0; k < n; ++k) {
+      const int ti = ty[k];
+      GemmType &t = g.t[k];
+      t.B = M.fs_adj[ti][l];
+      t.gmax = nullptr;
+      t.ascale = M.fit_gsc[ti][l];
+      t.wscale = M.fit_wsc[ti][l];
+      t.ep = Epi{};
+      t.ep.ld = g.N;
+      if (l == 0) {
+        t.ep.mode = EPI_STORE;
+        t.ep.out1 = G;
+        continue;
+      }
+      t.ep.tin = tb[l - 1];
       if (M.fdt[ti][l]) {
-        if (l == L - 1) ep.gvec = M.fw[ti][L];
-        else ep.gmat = gh[cur];
+        if (l == L - 1) t.ep.gvec = M.fw[ti][L];
+        else t.ep.gmat = gh[cur];
       }
-      ep.out1 = gz[cur ^ 1];
+      t.ep.out1 = gz[cur ^ 1];
+      t.ep.mode = EPI_GRAD;
       if (l - 1 > 0 && M.fdt[ti][l - 1]) {
-        ep.mode = EPI_GRAD_RES;
-        ep.dt = M.fdt[ti][l - 1];
-        ep.out2 = gh[cur ^ 1];
-      } else {
-        ep.mode = EPI_GRAD;
+        t.ep.mode = EPI_GRAD_RES;
+        t.ep.dt = M.fdt[ti][l - 1];
+        t.ep.out2 = gh[cur ^ 1];
       }
-      rc = launch_sgemm(Mrows, out, in, gz[cur], in, rm, M.fwT[ti][l], ep, st);
-      if (rc) return rc;
-      cur ^= 1;
     }
-    Epi ep{};
-    ep.mode = EPI_STORE;
-    ep.out1 = G;
-    ep.ld = K0;
-    rc = launch_sgemm(Mrows, K0, M.FW[0], gz[cur], M.FW[0], rm, M.fwT[ti][0], ep, st);
-    if (rc) return rc;
+    if ((rc = launch_gemm_split(g, st))) return rc;
+    cur ^= 1;
   }
   return DPB_OK;
 }
@@ -527,18 +574,18 @@ static SplitWs split_ws(const DevModel &M, size_t NF, size_t nE, char *base, cha
 // tables and other shapes in the FP32 kernels.
 static int embed_fwd_fp32(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm,
                           const float *box, const int32_t *nbrs, const SplitWs &sw, int ba, float *T, float *G,
-                          cudaStream_t st) {
+                          float *gmax, cudaStream_t st) {
   int rc = DPB_OK;
   if (M.ngrids == 0 && M.emb_tuned) {
     rc = launch_pos_sorted(D, pos, perm, sw.posS, st);
     if (!rc && sw.rows && D.S <= kRowStoreCap) rc = launch_rows(M, D, ba, sw.posS, box, nbrs, sw.rows, sw.rcnt, st);
-    if (!rc) rc = split_embed_fwd(M, D, ba, sw.posS, box, nbrs, sw.rows, sw.rcnt, T, G, st);
+    if (!rc) rc = split_embed_fwd(M, D, ba, sw.posS, box, nbrs, sw.rows, sw.rcnt, T, G, gmax, st);
     return rc;
   }
   for (int ti = 0; ti < M.ntypes && !rc; ++ti)
-    rc = !M.emb_tuned   ? launch_embed_fwd_gen(M, D, ti, pos, perm, box, nbrs, T, G, st)
-         : M.E2 == 100 ? launch_embed_fwd_cmp<100>(M, D, ti, pos, perm, box, nbrs, T, G, st)
-                       : launch_embed_fwd_cmp<64>(M, D, ti, pos, perm, box, nbrs, T, G, st);
+    rc = !M.emb_tuned   ? launch_embed_fwd_gen(M, D, ti, pos, perm, box, nbrs, T, G, gmax, st)
+         : M.E2 == 100 ? launch_embed_fwd_cmp<100>(M, D, ti, pos, perm, box, nbrs, T, G, gmax, st)
+                       : launch_embed_fwd_cmp<64>(M, D, ti, pos, perm, box, nbrs, T, G, gmax, st);
   return rc;
 }
 
@@ -553,7 +600,7 @@ static int eval_fp32(const DevModel &M, const SysDesc &D, const float *pos, cons
   const int ba = split_block_atoms(D);
   int rc;
   prof_begin(PROF_EMBED_FWD, st);
-  rc = embed_fwd_fp32(M, D, pos, perm, box, nbrs, sw, ba, T, G, st);
+  rc = embed_fwd_fp32(M, D, pos, perm, box, nbrs, sw, ba, T, G, Eatom, st);
   if (rc) return rc;
   prof_end(PROF_EMBED_FWD, st);
   prof_begin(PROF_FIT, st);
@@ -677,7 +724,7 @@ extern "C" int dpb_eval_descriptors(const dpb_model *m, int precision, const flo
   auto fp32 = [&]() {
     char *w = (char *)workspace;
     const SplitWs sw = split_ws(m->dm, (size_t)natoms * nframes, (size_t)nframes, w, w);
-    return embed_fwd_fp32(m->dm, D, pos, perm, box, nbrs, sw, split_block_atoms(D), T, G, st);
+    return embed_fwd_fp32(m->dm, D, pos, perm, box, nbrs, sw, split_block_atoms(D), T, G, nullptr, st);
   };
   if (precision == DPB_PREC_FP32) return fp32();
   if (precision == DPB_PREC_MIXED) {

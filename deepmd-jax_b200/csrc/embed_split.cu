@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_fwd(DevModel M, SysD
                                                                const int32_t *__restrict__ nbrs,
                                                                const float4 *__restrict__ rows_g,
                                                                const int *__restrict__ rcnt, float *__restrict__ Tout,
-                                                               float *__restrict__ Gout) {
+                                                               float *__restrict__ Gout, float *__restrict__ gmax) {
   using SD = SplitDims<E0, E1, E2>;
   using SM = SplitFwdSmem<E0, E1, E2>;
   extern __shared__ __align__(1024) char smem[];
@@ -382,6 +382,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_fwd(DevModel M, SysD
   __shared__ int wcnt[kSplitThreads / 32];
   __shared__ int seg_s[5];  // first row of each slot in the staged tile
   __shared__ float3 ri_s[kBlkAtoms];
+  __shared__ int gmax_s[4];  // largest |G| per slot (float bits)
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tbase_s;
   const int tid = threadIdx.x, warp = tid >> 5;
@@ -643,6 +644,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_fwd(DevModel M, SysD
     // Q[slot][a][12] staged behind X
     const int A = M.A;
     float *Qs = Xs + 4 * 10 * E2;
+    if (tid < 4) gmax_s[tid] = 0;
     for (int e = tid; e < nb * 160; e += kSplitThreads) {
       const int slot = e / 160, aa = (e - slot * 160) / 10, c = e - slot * 160 - aa * 10;
       if (aa < A) {
@@ -667,6 +669,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_fwd(DevModel M, SysD
       x[0] = tc::add2(x[0], tc::pk(M.tbias[w], M.tbias[w + 1]));
       const float *Q = Qs + slot * 16 * 12;
       float *Gs = Gout + (g0 + slot) * (size_t)A * E2 + w;
+      float gm = 0.f;
       for (int aa = 0; aa < A; ++aa, Q += 12) {
         const float4 qa = *reinterpret_cast<const float4 *>(Q), qb = *reinterpret_cast<const float4 *>(Q + 4);
         const float2 qc = *reinterpret_cast<const float2 *>(Q + 8);
@@ -681,9 +684,12 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_fwd(DevModel M, SysD
         v = tc::fma2(x[8], tc::pk1(qc.x), v);
         v = tc::fma2(x[9], tc::pk1(qc.y), v);
         *reinterpret_cast<f2 *>(Gs + (size_t)aa * E2) = v;
+        gm = fmaxf(gm, fmaxf(fabsf(lo_of(v)), fabsf(hi_of(v))));
       }
+      atomicMax(&gmax_s[slot], __float_as_int(gm));  // gm >= 0: the bits order as the values
     }
     __syncthreads();
+    if (gmax && tid < nb) gmax[g0 + tid] = __int_as_float(gmax_s[tid]);
   }
   if (!ok) {
     // a tensor-core wait gave up: NaN descriptors reach the energy and the status word
@@ -1134,12 +1140,13 @@ int split_block_atoms(const SysDesc &D) {
 
 template <int E0, int E1, int E2>
 static int launch_fwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
-                      const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, cudaStream_t st) {
+                      const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, float *gmax,
+                    cudaStream_t st) {
   const int nblk = blocks_total(D, ba), smem = SplitFwdSmem<E0, E1, E2>::total;
   if (!nblk) return DPB_OK;
   DPB_CUDA_TRY(cudaFuncSetAttribute(k_split_fwd<E0, E1, E2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int grid = std::min(nblk, 2 * split_sms());
-  k_split_fwd<E0, E1, E2><<<grid, kSplitThreads, smem, st>>>(M, D, ba, posS, box, nbrs, rows, rcnt, T, G);
+  k_split_fwd<E0, E1, E2><<<grid, kSplitThreads, smem, st>>>(M, D, ba, posS, box, nbrs, rows, rcnt, T, G, gmax);
   count_launch();
   DPB_LAUNCH_CHECK();
   return DPB_OK;
@@ -1167,9 +1174,10 @@ static int launch_bwd(const DevModel &M, const SysDesc &D, int ba, const float4 
 }
 
 int split_embed_fwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
-                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, cudaStream_t st) {
-  return M.E2 == 100 ? launch_fwd<25, 50, 100>(M, D, ba, posS, box, nbrs, rows, rcnt, T, G, st)
-                     : launch_fwd<32, 32, 64>(M, D, ba, posS, box, nbrs, rows, rcnt, T, G, st);
+                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, float *gmax,
+                    cudaStream_t st) {
+  return M.E2 == 100 ? launch_fwd<25, 50, 100>(M, D, ba, posS, box, nbrs, rows, rcnt, T, G, gmax, st)
+                     : launch_fwd<32, 32, 64>(M, D, ba, posS, box, nbrs, rows, rcnt, T, G, gmax, st);
 }
 
 int split_embed_bwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,

@@ -32,8 +32,11 @@ struct DevModel {
   const float *fw[kMaxTypes][kMaxFitLayers + 1];
   const float *fb[kMaxTypes][kMaxFitLayers + 1];
   const float *fdt[kMaxTypes][kMaxFitLayers];
-  // transposed fitting kernels (out,in) for the adjoint GEMMs
-  const float *fwT[kMaxTypes][kMaxFitLayers + 1];
+  // stored weight tiles of the FP32 form's fitting GEMMs (gemm_split.cu): layer
+  // l forward (B = W_l^T) and adjoint (B = W_l), times fit_wsc; fit_hsc is the
+  // operand scale of the activations of layer l
+  const __half *fs_fwd[kMaxTypes][kMaxFitLayers], *fs_adj[kMaxTypes][kMaxFitLayers];
+  float fit_hsc[kMaxTypes][kMaxFitLayers];
   // per embedding net: the shared-memory image of its FP16 B tiles (layer 1
   // and layer 2, K-major, the layer's bias as the K row after the inputs,
   // zero padded to multiples of 16) and of its first layer (w0, b0 in FP32),
@@ -136,6 +139,35 @@ struct Epi {
   const float *gmat;    // per atom addend (or NULL)
   float *out1, *out2;   // per atom, ld
   int ld;
+};
+
+// One centre type's part of a fitting GEMM over the atoms of every type
+// (gemm_split.cu): rows, weights, operand scales and epilogue.
+struct GemmType {
+  int Mrows;
+  RowMap rm;
+  const __half *B;      // stored weight tiles
+  const float *gmax;    // per atom max |A| (row scale), or NULL: ascale for every row
+  float ascale, wscale;
+  Epi ep;
+};
+struct GemmArgs {
+  const float *A;       // per atom, lda
+  int lda, K, N, ntypes;
+  int mt0[kMaxTypes + 1];  // first 128-row tile of each type
+  GemmType t[kMaxTypes];
+};
+
+// One centre type's part of the energy kernel.
+struct EnergyType {
+  int Mrows;
+  RowMap rm;
+  const float *wfin, *bfin, *dtl;
+};
+struct EnergyArgs {
+  int ntypes, FWl, N;
+  int b0[kMaxTypes + 1];  // first block of each type
+  EnergyType t[kMaxTypes];
 };
 
 }  // namespace dpb

@@ -88,7 +88,7 @@ template <int E2>
 __global__ void __launch_bounds__(256) k_embed_fwd(DevModel M, SysDesc D, int ti, const float *__restrict__ pos,
                                                    const int32_t *__restrict__ perm, const float *__restrict__ box,
                                                    const int32_t *__restrict__ nbrs, float *__restrict__ Tout,
-                                                   float *__restrict__ Gout) {
+                                                   float *__restrict__ Gout, float *__restrict__ gmax) {
   extern __shared__ float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   float *rowbuf = smem + warp * embed_fwd_warp_floats<E2>();
@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(256) k_embed_fwd(DevModel M, SysDesc D, int ti
   // Q[4+m][a] = tensor_3to6(X[1:4][A+a])[m] + X[4+m][A+a]
   const int A = M.A;
   float *Gg = Gout + g * (size_t)A * E2;
+  float gm = 0.f;
   for (int aa = 0; aa < A; ++aa) {
     float Q[10];
 #pragma unroll
@@ -188,7 +189,13 @@ __global__ void __launch_bounds__(256) k_embed_fwd(DevModel M, SysDesc D, int ti
 #pragma unroll
       for (int c = 0; c < 10; ++c) v = fmaf(Q[c], Ts[c * E2 + col], v);
       Gg[aa * E2 + col] = v;
+      gm = fmaxf(gm, fabsf(v));
     }
+  }
+  if (gmax) {  // the fitting GEMM's row scale
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) gm = fmaxf(gm, __shfl_xor_sync(0xffffffffu, gm, o));
+    if (lane == 0) gmax[g] = gm;
   }
 }
 
@@ -432,143 +439,47 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
   }
 }
 
-// ---------------------------------------------------------------- fitting (SGEMM chain)
-constexpr int GB_M = 64, GB_N = 64, GB_K = 16;
-
-__global__ void __launch_bounds__(256) k_sgemm(int Mrows, int Nc, int K, const float *__restrict__ A, int lda,
-                                               RowMap rm, const float *__restrict__ B, Epi ep) {
-  __shared__ float As[GB_K][GB_M + 4];
-  __shared__ __align__(16) float Bs[GB_K][GB_N];
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int m0 = blockIdx.y * GB_M, n0 = blockIdx.x * GB_N;
-  float acc[4][4] = {};
-  // A tile loader: 64 rows x 16 k, one float4 (4 k) per thread
-  const int la_r = tid >> 2, la_k = (tid & 3) * 4;
-  const int ar = m0 + la_r;
-  const float *Arow = ar < Mrows ? A + rm.atom(ar) * (size_t)lda : nullptr;
-  // B tile loader: 16 k x 64 n, one float4 (4 n) per thread
-  const int lb_k = tid >> 4, lb_n = (tid & 15) * 4;
-  for (int k0 = 0; k0 < K; k0 += GB_K) {
-    float4 av = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (Arow) {
-      const int kk = k0 + la_k;
-      if (kk + 3 < K) av = *reinterpret_cast<const float4 *>(Arow + kk);
-      else {
-        float t[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int u = 0; u < 4; ++u) if (kk + u < K) t[u] = Arow[kk + u];
-        av = make_float4(t[0], t[1], t[2], t[3]);
-      }
-    }
-    As[la_k + 0][la_r] = av.x; As[la_k + 1][la_r] = av.y;
-    As[la_k + 2][la_r] = av.z; As[la_k + 3][la_r] = av.w;
-    {
-      const int kk = k0 + lb_k, nn = n0 + lb_n;
-      float t[4] = {0.f, 0.f, 0.f, 0.f};
-      if (kk < K) {
-        if (nn + 3 < Nc && ((Nc & 3) == 0)) {
-          float4 bv = *reinterpret_cast<const float4 *>(B + (size_t)kk * Nc + nn);
-          t[0] = bv.x; t[1] = bv.y; t[2] = bv.z; t[3] = bv.w;
-        } else {
-          for (int u = 0; u < 4; ++u) if (nn + u < Nc) t[u] = B[(size_t)kk * Nc + nn + u];
-        }
-      }
-      *reinterpret_cast<float4 *>(&Bs[lb_k][lb_n]) = make_float4(t[0], t[1], t[2], t[3]);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < GB_K; ++k) {
-      float a4[4], b4[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) a4[u] = As[k][ty * 4 + u];
-      const float4 bv = *reinterpret_cast<const float4 *>(&Bs[k][tx * 4]);
-      b4[0] = bv.x; b4[1] = bv.y; b4[2] = bv.z; b4[3] = bv.w;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = fmaf(a4[u], b4[v], acc[u][v]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int r = m0 + ty * 4 + u;
-    if (r >= Mrows) continue;
-    const size_t at = rm.atom(r) * (size_t)ep.ld;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int n = n0 + tx * 4 + v;
-      if (n >= Nc) continue;
-      const float x = acc[u][v];
-      switch (ep.mode) {
-        case EPI_STORE: ep.out1[at + n] = x; break;
-        case EPI_TANH: {
-          const float t = tanhf(x + ep.bias[n]);
-          ep.out1[at + n] = t;
-          if (ep.out2) ep.out2[at + n] = t;
-          break;
-        }
-        case EPI_TANH_RES: {
-          const float t = tanhf(x + ep.bias[n]);
-          ep.out1[at + n] = t;
-          ep.out2[at + n] = t * ep.dt[n] + ep.hprev[at + n];
-          break;
-        }
-        case EPI_GRAD_RES: {
-          const float gh = x + (ep.gvec ? ep.gvec[n] : ep.gmat[at + n]);
-          const float t = ep.tin[at + n];
-          ep.out2[at + n] = gh;
-          ep.out1[at + n] = gh * ep.dt[n] * (1.f - t * t);
-          break;
-        }
-        case EPI_GRAD: {
-          const float gh = x + (ep.gvec ? ep.gvec[n] : (ep.gmat ? ep.gmat[at + n] : 0.f));
-          const float t = ep.tin[at + n];
-          ep.out1[at + n] = gh * (1.f - t * t);
-          break;
-        }
-      }
-    }
-  }
-}
-
-// Per-atom energy E = H . w + b' and the first adjoint gZ of the last hidden
-// layer (64 atoms per block); per-frame energies reduced in FP64, one atomic
-// per (block, frame).
-__global__ void __launch_bounds__(256) k_fit_energy(int Mrows, RowMap rm, int FWl, const float *__restrict__ H,
-                                                    const float *__restrict__ tl, const float *__restrict__ wfin,
-                                                    const float *__restrict__ bfin, const float *__restrict__ dtl,
-                                                    float *__restrict__ Eatom, float *__restrict__ gZ,
-                                                    double *__restrict__ energy, int N,
+// ---------------------------------------------------------------- fitting energy
+// Per-atom energy E = H . w + b' and the first adjoint gate of the last hidden
+// layer, gZ = w dt (1 - t^2): a warp per atom, 8 atoms per block (64 atoms per
+// block with 8 in turn per warp took 27 us at 192 atoms, all latency); energies
+// reduced in FP64, one atomic per run of one energy row.
+__global__ void __launch_bounds__(256) k_fit_energy(EnergyArgs g, const float *__restrict__ H,
+                                                    const float *__restrict__ tl, float *__restrict__ Eatom,
+                                                    float *__restrict__ gZ, double *__restrict__ energy,
                                                     const int32_t *__restrict__ seg) {
-  __shared__ double es[64];
-  __shared__ int fs[64];
+  __shared__ double es[8];
+  __shared__ int fs[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int k = 0; k < 8; ++k) {
-    const int slot = warp * 8 + k;
-    const int r = blockIdx.x * 64 + slot;
-    if (r >= Mrows) {
-      if (lane == 0) { es[slot] = 0.0; fs[slot] = -1; }
-      continue;
-    }
-    const size_t at = rm.atom(r);
+  int ti = 0;
+#pragma unroll
+  for (int t = 1; t < kMaxTypes; ++t)
+    if (t < g.ntypes && (int)blockIdx.x >= g.b0[t]) ti = t;
+  const EnergyType &et = g.t[ti];
+  const int r = ((int)blockIdx.x - g.b0[ti]) * 8 + warp;
+  if (r < et.Mrows) {
+    const size_t at = et.rm.atom(r);
     float s = 0.f;
-    for (int n = lane; n < FWl; n += 32) {
-      s = fmaf(H[at * FWl + n], wfin[n], s);
-      const float t = tl[at * FWl + n];
-      gZ[at * FWl + n] = wfin[n] * (dtl ? dtl[n] : 1.f) * (1.f - t * t);
+    for (int n = lane; n < g.FWl; n += 32) {
+      const float w = et.wfin[n], t = tl[at * g.FWl + n];
+      s = fmaf(H[at * g.FWl + n], w, s);
+      gZ[at * g.FWl + n] = w * (et.dtl ? et.dtl[n] : 1.f) * (1.f - t * t);
     }
-    s = warp_sum(s) + bfin[0];
+    s = warp_sum(s) + et.bfin[0];
     if (lane == 0) {
       Eatom[at] = s;
-      es[slot] = (double)s;
-      fs[slot] = energy_slot(seg, at, N);
+      es[warp] = (double)s;
+      fs[warp] = energy_slot(seg, at, g.N);
     }
+  } else if (lane == 0) {
+    es[warp] = 0.0;
+    fs[warp] = -1;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     double run = 0.0;
     int cf = fs[0];
-    for (int k = 0; k < 64; ++k) {
+    for (int k = 0; k < 8; ++k) {
       if (fs[k] != cf) {
         if (cf >= 0) atomicAdd(&energy[cf], run);
         run = 0.0;
@@ -608,13 +519,13 @@ __global__ void k_finalize(int NF, int N, const float4 *__restrict__ F4, float *
 
 template <int E2>
 int launch_embed_fwd_cmp(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
-                         const float *box, const int32_t *nbrs, float *T, float *G, cudaStream_t st) {
+                         const float *box, const int32_t *nbrs, float *T, float *G, float *gmax, cudaStream_t st) {
   const int cnt = D.offs[ti + 1] - D.offs[ti];
   if (cnt == 0) return DPB_OK;
   dim3 grid((cnt + 7) / 8, D.F);
   const size_t smem = (size_t)8 * embed_fwd_warp_floats<E2>() * sizeof(float);
   cudaFuncSetAttribute(k_embed_fwd<E2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  k_embed_fwd<E2><<<grid, 256, smem, st>>>(M, D, ti, pos, perm, box, nbrs, T, G);
+  k_embed_fwd<E2><<<grid, 256, smem, st>>>(M, D, ti, pos, perm, box, nbrs, T, G, gmax);
   count_launch();
   DPB_LAUNCH_CHECK();
   return DPB_OK;
@@ -637,9 +548,9 @@ int launch_embed_bwd_cmp(const DevModel &M, const SysDesc &D, int ti, const floa
 }
 
 template int launch_embed_fwd_cmp<100>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
-                                       const float *, const int32_t *, float *, float *, cudaStream_t);
+                                       const float *, const int32_t *, float *, float *, float *, cudaStream_t);
 template int launch_embed_fwd_cmp<64>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
-                                      const float *, const int32_t *, float *, float *, cudaStream_t);
+                                      const float *, const int32_t *, float *, float *, float *, cudaStream_t);
 template int launch_embed_bwd_cmp<100>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
                                        const float *, const int32_t *, const float *, const float *, float4 *,
                                        double *, cudaStream_t);
@@ -647,22 +558,11 @@ template int launch_embed_bwd_cmp<64>(const DevModel &, const SysDesc &, int, co
                                       const float *, const int32_t *, const float *, const float *, float4 *, double *,
                                       cudaStream_t);
 
-int launch_sgemm(int Mrows, int Nc, int K, const float *A, int lda, RowMap rm, const float *B, const Epi &ep,
-                 cudaStream_t st) {
-  if (Mrows == 0) return DPB_OK;
-  dim3 grid((Nc + GB_N - 1) / GB_N, (Mrows + GB_M - 1) / GB_M);
-  k_sgemm<<<grid, 256, 0, st>>>(Mrows, Nc, K, A, lda, rm, B, ep);
-  count_launch();
-  DPB_LAUNCH_CHECK();
-  return DPB_OK;
-}
-
-int launch_fit_energy(int Mrows, RowMap rm, int FWl, const float *H, const float *tl, const float *wfin,
-                      const float *bfin, const float *dtl, float *Eatom, float *gZ, double *energy, int N,
+int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, float *gZ, double *energy,
                       const int32_t *seg, cudaStream_t st) {
-  if (Mrows == 0) return DPB_OK;
-  k_fit_energy<<<(Mrows + 63) / 64, 256, 0, st>>>(Mrows, rm, FWl, H, tl, wfin, bfin, dtl, Eatom, gZ, energy, N,
-                                                  seg);
+  const int nb = g.b0[g.ntypes];
+  if (nb == 0) return DPB_OK;
+  k_fit_energy<<<nb, 256, 0, st>>>(g, H, tl, Eatom, gZ, energy, seg);
   count_launch();
   DPB_LAUNCH_CHECK();
   return DPB_OK;

@@ -210,7 +210,8 @@ template <bool CMP>
 __global__ void __launch_bounds__(256) k_embed_fwd_gen(DevModel M, GenNet G, SysDesc D, int ti,
                                                        const float *__restrict__ pos, const int32_t *__restrict__ perm,
                                                        const float *__restrict__ box, const int32_t *__restrict__ nbrs,
-                                                       float *__restrict__ Tout, float *__restrict__ Gout) {
+                                                       float *__restrict__ Tout, float *__restrict__ Gout,
+                                                       float *__restrict__ gmax) {
   extern __shared__ float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   float *wsm = smem;
@@ -303,6 +304,7 @@ __global__ void __launch_bounds__(256) k_embed_fwd_gen(DevModel M, GenNet G, Sys
   // G[a][w] = sum_c Q[c][a] X[c][w] (dpmodel.py:74-78)
   const int A = M.A;
   float *Gg = Gout + g * (size_t)A * E;
+  float gm = 0.f;
   for (int aa = 0; aa < A; ++aa) {
     float Q[10];
 #pragma unroll
@@ -319,7 +321,13 @@ __global__ void __launch_bounds__(256) k_embed_fwd_gen(DevModel M, GenNet G, Sys
 #pragma unroll
       for (int c = 0; c < 10; ++c) v = fmaf(Q[c], Ts[c * E + col], v);
       Gg[aa * E + col] = v;
+      gm = fmaxf(gm, fabsf(v));
     }
+  }
+  if (gmax) {  // the fitting GEMM's row scale
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) gm = fmaxf(gm, __shfl_xor_sync(0xffffffffu, gm, o));
+    if (lane == 0) gmax[g] = gm;
   }
 }
 
@@ -688,7 +696,7 @@ static int gen_warps(size_t fixed_floats, size_t per_warp_floats, size_t *smem) 
 }
 
 int launch_embed_fwd_gen(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
-                         const float *box, const int32_t *nbrs, float *T, float *G, cudaStream_t st) {
+                         const float *box, const int32_t *nbrs, float *T, float *G, float *gmax, cudaStream_t st) {
   const int cnt = D.offs[ti + 1] - D.offs[ti];
   if (cnt == 0) return DPB_OK;
   const GenNet net = gen_net(M);
@@ -699,10 +707,10 @@ int launch_embed_fwd_gen(const DevModel &M, const SysDesc &D, int ti, const floa
   dim3 grid((cnt + wpb - 1) / wpb, D.F);
   if (cmp) {
     DPB_CUDA_TRY(cudaFuncSetAttribute(k_embed_fwd_gen<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_embed_fwd_gen<true><<<grid, 32 * wpb, smem, st>>>(M, net, D, ti, pos, perm, box, nbrs, T, G);
+    k_embed_fwd_gen<true><<<grid, 32 * wpb, smem, st>>>(M, net, D, ti, pos, perm, box, nbrs, T, G, gmax);
   } else {
     DPB_CUDA_TRY(cudaFuncSetAttribute(k_embed_fwd_gen<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_embed_fwd_gen<false><<<grid, 32 * wpb, smem, st>>>(M, net, D, ti, pos, perm, box, nbrs, T, G);
+    k_embed_fwd_gen<false><<<grid, 32 * wpb, smem, st>>>(M, net, D, ti, pos, perm, box, nbrs, T, G, gmax);
   }
   count_launch();
   DPB_LAUNCH_CHECK();

@@ -1879,13 +1879,13 @@ __global__ void k_f32_to_f16(const float4 *__restrict__ a, uint2 *__restrict__ b
 
 template <int E2>
 int launch_embed_fwd_cmp(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
-                         const float *box, const int32_t *nbrs, float *T, float *G, cudaStream_t st);
+                         const float *box, const int32_t *nbrs, float *T, float *G, float *gmax, cudaStream_t st);
 template <int E2>
 int launch_embed_bwd_cmp(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
                          const float *box, const int32_t *nbrs, const float *T, const float *dG, float4 *F4,
                          double *virial, cudaStream_t st);
 int launch_embed_fwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
-                         const int32_t *, float *, float *, cudaStream_t);
+                         const int32_t *, float *, float *, float *, cudaStream_t);
 int launch_embed_bwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
                          const int32_t *, const float *, const float *, float4 *, double *, cudaStream_t);
 
@@ -1902,9 +1902,9 @@ static int mixed_eval_compressed(const DevModel &M, const SysDesc &D, const floa
   int rc;
   prof_begin(PROF_EMBED_FWD, st);
   for (int ti = 0; ti < M.ntypes; ++ti) {
-    rc = !M.emb_tuned   ? launch_embed_fwd_gen(M, D, ti, pos, perm, box, nbrs, T, dG, st)
-         : M.E2 == 100 ? launch_embed_fwd_cmp<100>(M, D, ti, pos, perm, box, nbrs, T, dG, st)
-                       : launch_embed_fwd_cmp<64>(M, D, ti, pos, perm, box, nbrs, T, dG, st);
+    rc = !M.emb_tuned   ? launch_embed_fwd_gen(M, D, ti, pos, perm, box, nbrs, T, dG, nullptr, st)
+         : M.E2 == 100 ? launch_embed_fwd_cmp<100>(M, D, ti, pos, perm, box, nbrs, T, dG, nullptr, st)
+                       : launch_embed_fwd_cmp<64>(M, D, ti, pos, perm, box, nbrs, T, dG, nullptr, st);
     if (rc) return rc;
   }
   k_f32_to_f16<<<(unsigned)((NG / 4 + 255) / 256), 256, 0, st>>>(reinterpret_cast<const float4 *>(dG),
