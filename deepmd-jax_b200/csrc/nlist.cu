@@ -8,14 +8,23 @@
 // indices in ascending order, type-local, padded with N, and flags overflow
 // when more than sel_j exist.
 //
-// Layout: cells are binned per frame and each cell slot also holds its
-// atom's canonical position and index as one float4 (cell order), so a
-// candidate is one coalesced 16-byte load.  A warp owns one centre atom,
-// centres taken in cell order so that the warps of a block share their
-// neighbourhood in L1; it walks the 27 (or fewer, for 2-cell or 1-cell axes)
-// neighbouring cells, appends hits per type into shared memory with ballots,
-// then ranks the hits (indices are distinct, so rank = number of smaller
-// hits) and writes the sorted prefix into the centre's own row.
+// Layout: cells are binned per frame and each cell slot holds its atom's
+// canonical position and index as one float4 (cell order), so a candidate is
+// one coalesced 16-byte load.  A warp owns one centre atom, centres taken in
+// cell order so that the warps of a block share their neighbourhood in L1.
+// Cells are at least rc / 2 wide (at least rc where that would leave cells
+// mostly empty).  Each lane takes one z-row of the 5 x 5 (3 x 3) rows around the
+// centre, drops it if it lies outside the cutoff sphere and else cuts it to the
+// sphere's chord; the rows' candidates are then walked as one flat sequence, 32
+// per round with every lane busy.  Hits are appended per type into shared memory
+// with ballots, sorted in registers, and the sorted prefix is written into the
+// centre's own row.
+//
+// What bounds it: instruction issue (79 % of slots, the ALU pipe 69 % busy).
+// With cells of rc, 98,304 atoms of liquid water at rc 6.3 A had 964 candidates in
+// 36 rounds per centre: 505 us.  Cells of rc / 2 with the sphere cuts took it to
+// 274 us, sorting in registers to 240 us, branch-free displacements to 217 us; 32
+// frames of 1,536 atoms 474 -> 114 us.
 #include "dpb_common.cuh"
 #include <algorithm>
 #include <climits>
@@ -26,24 +35,33 @@ namespace dpb {
 struct NlGrid {
   int nc[3];
   int ncell;      // per frame
-  int image_mode; // 1: explicit images (min(L) < 2 rc)
-  int nimg[3];    // image range per axis in image mode
+  int reach;      // cells on each side of the centre's that can hold neighbours
+  int image_mode; // 1: some L < 2 rc, brute force over the frame's atoms
 };
 
-static NlGrid make_grid(const float box[3], float rc) {
+static NlGrid cell_grid(const float box[3], float rc, int reach) {
   NlGrid g;
+  g.reach = reach;
   g.image_mode = 0;
+  long long n = 1;
   for (int d = 0; d < 3; ++d) {
-    int n = (int)floorf(box[d] / rc);
-    g.nc[d] = std::max(1, std::min(n, 512));
+    g.nc[d] = std::max(1, std::min((int)floorf(box[d] * (float)reach / rc), 512));
+    while (g.nc[d] > 1 && (double)box[d] * reach < (double)rc * g.nc[d]) --g.nc[d];
+    n *= g.nc[d];
     if (box[d] < 2.f * rc) g.image_mode = 1;
-    g.nimg[d] = (int)floorf(rc / box[d] + 0.5f);  // images with |minimg + m L| < rc
   }
   if (g.image_mode) {
     g.nc[0] = g.nc[1] = g.nc[2] = 1;
+    n = 1;
   }
-  g.ncell = g.nc[0] * g.nc[1] * g.nc[2];
+  g.ncell = (int)n;
   return g;
+}
+
+// Cells of rc / 2 where they hold an atom each on average, else of rc.
+static NlGrid make_grid(const float box[3], float rc, int natoms) {
+  const NlGrid fine = cell_grid(box, rc, 2);
+  return fine.ncell <= natoms ? fine : cell_grid(box, rc, 1);
 }
 
 // A non-null gate makes every kernel of the build a no-op unless *gate != 0,
@@ -82,6 +100,7 @@ __global__ void nl_canon_kernel(const float *__restrict__ pos, const int32_t *__
   canon[(size_t)g * 3 + 0] = c0;
   canon[(size_t)g * 3 + 1] = c1;
   canon[(size_t)g * 3 + 2] = c2;
+  if (!cell_count) return;  // image mode
   // cell bins of the reference box (canonical coordinates live in [0, ref))
   int ix = min(max((int)(c0 / RB.x * nc.x), 0), nc.x - 1);
   int iy = min(max((int)(c1 / RB.y * nc.y), 0), nc.y - 1);
@@ -91,46 +110,79 @@ __global__ void nl_canon_kernel(const float *__restrict__ pos, const int32_t *__
   atomicAdd(&cell_count[f * (nc.x * nc.y * nc.z) + cell], 1);
 }
 
-// Exclusive scan of n ints with one block (n up to a few million).
-__global__ void nl_scan_kernel(const int *__restrict__ in, int *__restrict__ out, int n,
-                               const unsigned *__restrict__ gate) {
+// Exclusive scan of n ints with one block, 16 per thread and pass (four 16-byte
+// loads in flight: 4 per thread took 14 us for the 29,791 cells of 98,304 atoms,
+// one load latency and two barriers per 4,096 cells).
+__global__ void __launch_bounds__(1024) nl_scan_kernel(const int *__restrict__ in, int *__restrict__ out, int n,
+                                                      const unsigned *__restrict__ gate) {
   if (gate && *gate == 0u) return;
-  __shared__ int part[1024];
-  int t = threadIdx.x;
-  int per = (n + blockDim.x - 1) / blockDim.x;
-  int b = t * per, e = min(b + per, n);
-  int s = 0;
-  for (int i = b; i < e; ++i) s += in[i];
-  part[t] = s;
-  __syncthreads();
-  for (int o = 1; o < (int)blockDim.x; o <<= 1) {
-    int v = t >= o ? part[t - o] : 0;
+  __shared__ int part[32];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  int run = 0;
+  for (int base = 0; base < n; base += 16384) {
+    const int i = base + 16 * t;
+    int v[16], mine = 0;
+    if (i + 16 <= n) {
+#pragma unroll
+      for (int k = 0; k < 16; k += 4) {
+        const int4 q = *reinterpret_cast<const int4 *>(in + i + k);
+        v[k] = q.x; v[k + 1] = q.y; v[k + 2] = q.z; v[k + 3] = q.w;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) v[k] = i + k < n ? in[i + k] : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) mine += v[k];
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    if (lane == 31) part[warp] = incl;
     __syncthreads();
-    part[t] += v;
+    int w = part[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w += u;
+    }
+    const int before = __shfl_sync(0xffffffffu, w, warp ? warp - 1 : 0), total = __shfl_sync(0xffffffffu, w, 31);
+    int e = run + (warp ? before : 0) + incl - mine;
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+      const int u = v[k];
+      v[k] = e;
+      e += u;
+    }
+    if (i + 16 <= n) {
+#pragma unroll
+      for (int k = 0; k < 16; k += 4)
+        *reinterpret_cast<int4 *>(out + i + k) = make_int4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        if (i + k < n) out[i + k] = v[k];
+    }
+    run += total;
     __syncthreads();
   }
-  int run = t ? part[t - 1] : 0;
-  for (int i = b; i < e; ++i) {
-    out[i] = run;
-    run += in[i];
-  }
-  if (t == blockDim.x - 1) out[n] = part[t];
+  if (t == 0) out[n] = run;
 }
 
 __global__ void nl_scatter_kernel(const int *__restrict__ atom_cell, const int *__restrict__ cell_start,
-                                  int *__restrict__ cursor, int *__restrict__ cell_atoms,
-                                  const float *__restrict__ canon, float4 *__restrict__ cell_pos, int N, int F,
-                                  int ncell, const unsigned *__restrict__ gate) {
+                                  int *__restrict__ cursor, const float *__restrict__ canon,
+                                  float4 *__restrict__ cell_pos, int N, int F, int ncell,
+                                  const unsigned *__restrict__ gate) {
   if (gate && *gate == 0u) return;
   int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= N * F) return;
   int f = g / N;
   int c = f * ncell + atom_cell[g];
-  int slot = atomicAdd(&cursor[c], 1);
-  const int q = cell_start[c] + slot;
-  cell_atoms[q] = g - f * N;  // frame-local sorted index
+  const int q = cell_start[c] + atomicAdd(&cursor[c], 1);
   cell_pos[q] = make_float4(canon[(size_t)g * 3], canon[(size_t)g * 3 + 1], canon[(size_t)g * 3 + 2],
-                            __int_as_float(g - f * N));
+                            __int_as_float(g - f * N));  // frame-local sorted index
 }
 
 struct NlParams {
@@ -141,8 +193,9 @@ struct NlParams {
   float3 L;      // reference box (canonical frame)
   float rc2;
   int3 nc;
-  int image_mode;
-  int3 nimg;
+  float3 h, inv_h;  // cell sizes
+  float rcm2;    // squared cutoff with a margin, for the row cuts
+  int reach, image_mode;
 };
 
 // Append the hits of one 32-candidate round into the per-type lists; the
@@ -164,45 +217,80 @@ __device__ __forceinline__ void append_hits(bool hit, int t, int key, int ntypes
   }
 }
 
-// Rank of each of a lane's KPL keys (lane, lane + 32, ...) among the nn
-// distinct keys of a hit list padded with INT_MAX to nn4 (a multiple of 4),
-// read four at a time; the keys with rank < sel go to out[rank] - off.
-template <int KPL>
-__device__ __forceinline__ void rank_write(const int *__restrict__ L_, int nn, int nn4, int sel, int off,
+// Sorts up to 32 R distinct keys of a hit list ascending in registers (bitonic,
+// element lane R + r: strides below R stay within a lane) and writes the first
+// sel of them minus off.  Counting each key's smaller ones instead took about
+// 650 instructions per centre (35 + 70 keys), this about 300.
+template <int R>
+__device__ __forceinline__ void sort_write(const int *__restrict__ L_, int nn, int sel, int off,
                                            int32_t *__restrict__ out) {
   const int lane = threadIdx.x & 31;
-  int key[KPL], rank[KPL];
+  int v[R];
 #pragma unroll
-  for (int k = 0; k < KPL; ++k) {
-    key[k] = lane + 32 * k < nn ? L_[lane + 32 * k] : INT_MAX;
-    rank[k] = 0;
+  for (int r = 0; r < R; ++r) v[r] = lane * R + r < nn ? L_[lane * R + r] : INT_MAX;
+#pragma unroll
+  for (int k = 2; k <= 32 * R; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+      if (j >= R) {  // partner element in another lane
+        const bool keep_min = ((lane * R & j) == 0) == ((lane * R & k) == 0);
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int o = __shfl_xor_sync(0xffffffffu, v[r], j / R);
+          v[r] = keep_min ? min(v[r], o) : max(v[r], o);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if ((r & j) == 0) {
+            const bool up = ((lane * R + r) & k) == 0;
+            const int lo = min(v[r], v[r | j]), hi = max(v[r], v[r | j]);
+            v[r] = up ? lo : hi;
+            v[r | j] = up ? hi : lo;
+          }
+      }
+    }
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int e = lane * R + r;
+    if (e < nn && e < sel) out[e] = v[r] - off;
   }
-  for (int e2 = 0; e2 < nn4; e2 += 4) {
-    const int4 v = *reinterpret_cast<const int4 *>(L_ + e2);
-#pragma unroll
-    for (int k = 0; k < KPL; ++k)
-      rank[k] += (v.x < key[k]) + (v.y < key[k]) + (v.z < key[k]) + (v.w < key[k]);
-  }
-#pragma unroll
-  for (int k = 0; k < KPL; ++k)
-    if (lane + 32 * k < nn && rank[k] < sel) out[rank[k]] = key[k] - off;
+}
+
+// jax_md.space.periodic displacement of one axis, mod(ci - cj + L/2, L) - L/2 in
+// float32.  Canonical coordinates lie in [0, L), so the argument lies in (-L/2,
+// 3L/2) and its mod is one exact or correctly rounded add (jmod in branch-free
+// form).
+__device__ __forceinline__ float canon_disp(float ci, float cj, float L, float h) {
+  const float t = __fadd_rn(__fsub_rn(ci, cj), h);
+  const float w = t < 0.f ? L : t >= L ? -L : 0.f;
+  return __fsub_rn(__fadd_rn(t, w), h);
 }
 
 __device__ __forceinline__ bool pair_hit(float3 ci, float3 cj, float3 L, float rc2) {
-  // jax_md.space.periodic displacement, centre minus neighbour, float32
-  float hx = 0.5f * L.x, hy = 0.5f * L.y, hz = 0.5f * L.z;
-  float dx = __fsub_rn(jmod(__fadd_rn(__fsub_rn(ci.x, cj.x), hx), L.x), hx);
-  float dy = __fsub_rn(jmod(__fadd_rn(__fsub_rn(ci.y, cj.y), hy), L.y), hy);
-  float dz = __fsub_rn(jmod(__fadd_rn(__fsub_rn(ci.z, cj.z), hz), L.z), hz);
-  float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+  const float dx = canon_disp(ci.x, cj.x, L.x, 0.5f * L.x), dy = canon_disp(ci.y, cj.y, L.y, 0.5f * L.y),
+              dz = canon_disp(ci.z, cj.z, L.z, 0.5f * L.z);
+  const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
   return d2 < rc2;
 }
 
-// 40 registers: 48 resident warps per SM at every launch shape (128-512
+// First offset and number of the cells to visit along an axis of nc cells: every
+// cell once where fewer than 2 reach + 1 exist.
+__device__ __forceinline__ int2 nl_span(int nc, int reach) {
+  return nc >= 2 * reach + 1 ? make_int2(-reach, 2 * reach + 1) : make_int2(-((nc - 1) / 2), nc);
+}
+
+// Distance (in cells) from a point at fraction fr of its cell to the cells at
+// offset o; 0 where the axis has so few cells that o stands for two images.
+__device__ __forceinline__ float nl_gap(int o, float fr, int nc, int reach) {
+  const float d = o > 0 ? (float)o - fr : o < 0 ? fr - (float)(o + 1) : 0.f;
+  return nc >= 2 * reach + 1 ? fmaxf(d, 0.f) : 0.f;
+}
+
+// 48 registers: 40 resident warps per SM at every launch shape (128-512
 // threads), with nothing spilled.
-__global__ void __maxnreg__(40) nl_search_kernel(NlParams P, const float *__restrict__ canon,
+__global__ void __maxnreg__(48) nl_search_kernel(NlParams P, const float *__restrict__ canon,
                                                  const int *__restrict__ cell_start,
-                                                 const int *__restrict__ cell_atoms,
                                                  const float4 *__restrict__ cell_pos,
                                                  int32_t *__restrict__ nbrs,
                                                  int32_t *__restrict__ counts,
@@ -212,96 +300,116 @@ __global__ void __maxnreg__(40) nl_search_kernel(NlParams P, const float *__rest
   extern __shared__ __align__(16) int smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int wpb = blockDim.x >> 5;
-  int *lists = smem + warp * P.ntypes * P.cap;
-  const int gc = blockIdx.x * wpb + warp;  // position in cell order
+  int4 *rows = reinterpret_cast<int4 *>(smem) + warp * 32;  // the rows' (first candidate, range 1, its length, range 2)
+  int *lists = smem + wpb * 128 + warp * P.ntypes * P.cap;
+  const int gc = blockIdx.x * wpb + warp;  // position in cell order (image mode: in sorted order)
   if (gc >= P.N * P.F) return;
-  const int f = gc / P.N, i = cell_atoms[gc];  // frame-local sorted index of the centre
-  const int g = f * P.N + i;
+  const int f = gc / P.N;
   const float *cf = canon + (size_t)f * P.N * 3;
-  float3 ci = make_float3(cf[i * 3], cf[i * 3 + 1], cf[i * 3 + 2]);
+  int i = gc - f * P.N;  // frame-local sorted index of the centre
+  float3 ci;
   int cnt[kMaxTypes] = {0, 0, 0, 0};
 
   if (!P.image_mode) {
-    const int ncell = P.nc.x * P.nc.y * P.nc.z;
+    const float4 c4 = cell_pos[gc];
+    i = __float_as_int(c4.w);
+    ci = make_float3(c4.x, c4.y, c4.z);
+    const int ncell = P.nc.x * P.nc.y * P.nc.z, nz = P.nc.z;
     const int *cs = cell_start + f * ncell;
-    int ix = min(max((int)(ci.x / P.L.x * P.nc.x), 0), P.nc.x - 1);
-    int iy = min(max((int)(ci.y / P.L.y * P.nc.y), 0), P.nc.y - 1);
-    int iz = min(max((int)(ci.z / P.L.z * P.nc.z), 0), P.nc.z - 1);
-    int lox = P.nc.x >= 3 ? -1 : 0, hix = P.nc.x >= 2 ? 1 : 0;
-    int loy = P.nc.y >= 3 ? -1 : 0, hiy = P.nc.y >= 2 ? 1 : 0;
-    int loz = P.nc.z >= 3 ? -1 : 0, hiz = P.nc.z >= 2 ? 1 : 0;
-    // candidates of [b, e) of cell order, 32 per round
-    auto scan = [&](int b, int e) {
-      for (int base = b; base < e; base += 32) {
-        const int q = base + lane;
-        bool hit = false;
-        int j = 0, t = 0;
-        if (q < e) {
-          const float4 v = cell_pos[q];
-          j = __float_as_int(v.w);
-          hit = (j != i) && pair_hit(ci, make_float3(v.x, v.y, v.z), P.L, P.rc2);
-          t = type_of(j, P.offs, P.ntypes);
+    const int ix = min(max((int)(ci.x / P.L.x * P.nc.x), 0), P.nc.x - 1);
+    const int iy = min(max((int)(ci.y / P.L.y * P.nc.y), 0), P.nc.y - 1);
+    const int iz = min(max((int)(ci.z / P.L.z * P.nc.z), 0), P.nc.z - 1);
+    const int2 sx = nl_span(P.nc.x, P.reach), sy = nl_span(P.nc.y, P.reach), sz = nl_span(nz, P.reach);
+    // ---- this lane's z-row: one or two ranges of cell order
+    int b1 = 0, n1 = 0, b2 = 0, n2 = 0;
+    if (lane < sx.y * sy.y) {
+      const int rx = lane / sy.y, ox = sx.x + rx, oy = sy.x + lane - rx * sy.y;
+      const float gx = nl_gap(ox, ci.x * P.inv_h.x - (float)ix, P.nc.x, P.reach) * P.h.x;
+      const float gy = nl_gap(oy, ci.y * P.inv_h.y - (float)iy, P.nc.y, P.reach) * P.h.y;
+      const float rem = P.rcm2 - gx * gx - gy * gy;
+      if (rem > 0.f) {
+        int z0 = iz + sz.x, z1 = z0 + sz.y - 1;
+        if (nz >= 2 * P.reach + 1) {  // the chord of the sphere
+          const float zc = ci.z * P.inv_h.z, zr = sqrtf(rem) * P.inv_h.z;
+          z0 = max(z0, (int)floorf(zc - zr));
+          z1 = min(z1, (int)floorf(zc + zr));
         }
-        append_hits(hit, t, j, P.ntypes, P.cap, cnt, lists);
-      }
-    };
-    // ix + o lies in [-1, nc], so one conditional add or subtract is the
-    // periodic wrap.  With three or more cells along z the cells iz-1..iz+1
-    // of a row are one range of cell order, or two where the row wraps, so
-    // a round takes 32 candidates of the row rather than of one cell (the
-    // visiting order only matters past cap hits, already an overflow).
-    for (int ox = lox; ox <= hix; ++ox) {
-      int cx = ix + ox;
-      cx += cx < 0 ? P.nc.x : 0;
-      cx -= cx >= P.nc.x ? P.nc.x : 0;
-      for (int oy = loy; oy <= hiy; ++oy) {
-        int cy = iy + oy;
+        // ix + ox lies in [-nc, 2 nc), so one conditional add or subtract wraps it
+        int cx = ix + ox, cy = iy + oy;
+        cx += cx < 0 ? P.nc.x : 0;
+        cx -= cx >= P.nc.x ? P.nc.x : 0;
         cy += cy < 0 ? P.nc.y : 0;
         cy -= cy >= P.nc.y ? P.nc.y : 0;
-        const int cxy = (cx * P.nc.y + cy) * P.nc.z, nz = P.nc.z;
-        if (nz >= 3) {
-          if (iz >= 1 && iz <= nz - 2) {
-            scan(cs[cxy + iz - 1], cs[cxy + iz + 2]);
-          } else if (iz == 0) {
-            scan(cs[cxy], cs[cxy + 2]);
-            scan(cs[cxy + nz - 1], cs[cxy + nz]);
-          } else {
-            scan(cs[cxy + nz - 2], cs[cxy + nz]);
-            scan(cs[cxy], cs[cxy + 1]);
-          }
-        } else {
-          for (int oz = loz; oz <= hiz; ++oz) {
-            int cz = iz + oz;
-            cz -= cz >= nz ? nz : 0;
-            scan(cs[cxy + cz], cs[cxy + cz + 1]);
-          }
+        const int *row = cs + (cx * P.nc.y + cy) * nz;
+        int a0 = z0, a1 = z1;
+        if (z0 < 0) {
+          a0 = z0 + nz;
+          a1 = nz - 1;
+          b2 = row[0];
+          n2 = row[z1 + 1] - b2;
+        } else if (z1 >= nz) {
+          a1 = nz - 1;
+          b2 = row[0];
+          n2 = row[z1 - nz + 1] - b2;
         }
+        b1 = row[a0];
+        n1 = row[a1 + 1] - b1;
       }
     }
+    // ---- the rows with candidates, in order, as one flat sequence
+    const int n = n1 + n2;
+    int incl = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += u;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31), start = incl - n;
+    const unsigned live = __ballot_sync(0xffffffffu, n > 0), lt = (1u << lane) - 1u, le = lt | (1u << lane);
+    if (n > 0) rows[__popc(live & lt)] = make_int4(start, b1, n1, b2);
+    __syncwarp();
+    int before = 0;  // rows that start before this round
+    for (int base = 0; base < total; base += 32) {
+      // bit l: a row starts at candidate base + l
+      const unsigned off = (unsigned)(start - base);
+      const unsigned starts = __reduce_or_sync(0xffffffffu, n > 0 && off < 32u ? 1u << off : 0u);
+      const int p = base + lane;
+      bool hit = false;
+      int j = 0, t = 0;
+      if (p < total) {
+        const int4 r = rows[before + __popc(starts & le) - 1];
+        const int k = p - r.x;
+        const float4 v = cell_pos[k < r.z ? r.y + k : r.w + k - r.z];
+        j = __float_as_int(v.w);
+        hit = (j != i) && pair_hit(ci, make_float3(v.x, v.y, v.z), P.L, P.rc2);
+        t = type_of(j, P.offs, P.ntypes);
+      }
+      before += __popc(starts);
+      append_hits(hit, t, j, P.ntypes, P.cap, cnt, lists);
+    }
   } else {
-    // small box: j is listed once if any periodic image lies within rc
-    const int nx = 2 * P.nimg.x + 1, ny = 2 * P.nimg.y + 1, nz = 2 * P.nimg.z + 1;
-    const int nim = nx * ny * nz;
+    // Some L < 2 rc: j is listed once if any periodic image lies within rc.
+    // For j != i that is the nearest image (|d + m L| >= |d| per axis for every m,
+    // in floating point too: d + L >= L / 2 >= |d| before rounding, which is
+    // monotonic); for j == i the nearest image that is not the atom itself.
+    ci = make_float3(cf[i * 3], cf[i * 3 + 1], cf[i * 3 + 2]);
+    const float ls = fminf(P.L.x, fminf(P.L.y, P.L.z));
+    const bool self = ls * ls < P.rc2;
     for (int base = 0; base < P.N; base += 32) {
       const int j = base + lane;
       bool hit = false;
       int t = 0;
       if (j < P.N) {
-        const float3 cj = make_float3(cf[j * 3], cf[j * 3 + 1], cf[j * 3 + 2]);
-        const float3 d0 = make_float3(shift_ortho(cj.x - ci.x, P.L.x), shift_ortho(cj.y - ci.y, P.L.y),
-                                      shift_ortho(cj.z - ci.z, P.L.z));
-        for (int m = 0; m < nim && !hit; ++m) {
-          const int a = m / (ny * nz) - P.nimg.x, bb = (m / nz) % ny - P.nimg.y, cc = m % nz - P.nimg.z;
-          if (j == i && a == 0 && bb == 0 && cc == 0) continue;
-          const float x = d0.x + a * P.L.x, y = d0.y + bb * P.L.y, z = d0.z + cc * P.L.z;
-          hit = x * x + y * y + z * z < P.rc2;
-        }
+        const float x = shift_ortho(cf[j * 3] - ci.x, P.L.x), y = shift_ortho(cf[j * 3 + 1] - ci.y, P.L.y),
+                    z = shift_ortho(cf[j * 3 + 2] - ci.z, P.L.z);
+        hit = j == i ? self : x * x + y * y + z * z < P.rc2;
         t = type_of(j, P.offs, P.ntypes);
       }
       append_hits(hit, t, j, P.ntypes, P.cap, cnt, lists);
     }
   }
-  // rank-sort each type's hits and write the sel_t smallest
+  const int g = f * P.N + i;
+  // sort each type's hits and write the sel_t smallest
   const int S = P.col[P.ntypes];
   int32_t *out = nbrs + (size_t)g * S;
   bool ovf = false;
@@ -310,16 +418,14 @@ __global__ void __maxnreg__(40) nl_search_kernel(NlParams P, const float *__rest
     const int n = t == 0 ? cnt[0] : t == 1 ? cnt[1] : t == 2 ? cnt[2] : cnt[3];
     if (counts && lane == 0) counts[(size_t)g * P.ntypes + t] = n;
     ovf |= (n > P.sel[t]) || (n > P.cap);
-    const int nn = min(n, P.cap), nn4 = (nn + 3) & ~3;  // cap is a multiple of 4
-    int *L_ = lists + t * P.cap;
-    if (lane < nn4 - nn) L_[nn + lane] = INT_MAX;
+    const int nn = min(n, P.cap);
+    const int *L_ = lists + t * P.cap;
     __syncwarp();
     int32_t *o = out + P.col[t];
     const int sel = P.sel[t], off = P.offs[t];
-    if (nn <= 32) rank_write<1>(L_, nn, nn4, sel, off, o);
-    else if (nn <= 64) rank_write<2>(L_, nn, nn4, sel, off, o);
-    else if (nn <= 96) rank_write<3>(L_, nn, nn4, sel, off, o);
-    else if (nn <= 128) rank_write<4>(L_, nn, nn4, sel, off, o);
+    if (nn <= 32) sort_write<1>(L_, nn, sel, off, o);
+    else if (nn <= 64) sort_write<2>(L_, nn, sel, off, o);
+    else if (nn <= 128) sort_write<4>(L_, nn, sel, off, o);
     else  // long lists (large sel): one key per lane at a time, few registers
       for (int e = lane; e < nn; e += 32) {
         const int key = L_[e];
@@ -338,13 +444,17 @@ using namespace dpb;
 
 static size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 
+static size_t nlist_bytes(size_t NF, size_t C) {
+  return align_up(C * 4) * 2 + align_up((C + 1) * 4) + align_up(NF * 4) + align_up(NF * 16) + align_up(NF * 12);
+}
+
+// Enough for both cell sizes of make_grid, and monotonic in rc: a caller may
+// size the workspace at a slightly smaller cutoff than it builds with.
 extern "C" int dpb_nlist_workspace_bytes(int natoms, int nframes, const float box[3], float rc,
                                          size_t *bytes) {
   if (!bytes || natoms <= 0 || nframes <= 0 || !box || rc <= 0) return DPB_ERR_INVALID_ARG;
-  NlGrid g = make_grid(box, rc);
-  size_t NF = (size_t)natoms * nframes, C = (size_t)g.ncell * nframes;
-  *bytes = align_up(C * 4) * 2 + align_up((C + 1) * 4) + align_up(NF * 4) * 2 + align_up(NF * 16) +
-           align_up(NF * 12);
+  const int ncell = std::max(cell_grid(box, rc, 1).ncell, std::min(cell_grid(box, rc, 2).ncell, natoms));
+  *bytes = nlist_bytes((size_t)natoms * nframes, (size_t)ncell * nframes);
   return DPB_OK;
 }
 
@@ -363,11 +473,13 @@ int nlist_build_impl(const float *pos, const int32_t *perm, int natoms, int nfra
   // jax_md receives rcut * max(ref/box) as float32 and squares it in float32
   float smax = std::max(rb[0] / box[0], std::max(rb[1] / box[1], rb[2] / box[2]));
   float rc_eff = rc * smax;
-  NlGrid g = make_grid(rb, rc_eff);
-  if (g.image_mode && (g.nimg[0] > 4 || g.nimg[1] > 4 || g.nimg[2] > 4)) return DPB_ERR_UNSUPPORTED;
-  size_t need = 0;
-  dpb_nlist_workspace_bytes(natoms, nframes, rb, rc_eff, &need);
-  if (!workspace || ws_bytes < need) return DPB_ERR_WORKSPACE;
+  NlGrid g = make_grid(rb, rc_eff, natoms);
+  if (g.image_mode)
+    for (int d = 0; d < 3; ++d)  // more than 4 images of an axis within reach
+      if ((int)floorf(rc_eff / rb[d] + 0.5f) > 4) return DPB_ERR_UNSUPPORTED;
+  const size_t NF = (size_t)natoms * nframes;
+  if (ws_bytes < nlist_bytes(NF, (size_t)g.ncell * nframes)) g = cell_grid(rb, rc_eff, 1);
+  if (!workspace || ws_bytes < nlist_bytes(NF, (size_t)g.ncell * nframes)) return DPB_ERR_WORKSPACE;
   NlParams P;
   P.N = natoms; P.F = nframes; P.ntypes = ntypes;
   int smax_sel = 0, off = 0, col = 0;
@@ -390,37 +502,46 @@ int nlist_build_impl(const float *pos, const int32_t *perm, int natoms, int nfra
   P.rc2 = rc_eff * rc_eff;
   P.nc = make_int3(g.nc[0], g.nc[1], g.nc[2]);
   P.image_mode = g.image_mode;
-  P.nimg = make_int3(g.nimg[0], g.nimg[1], g.nimg[2]);
+  P.reach = g.reach;
+  P.h = make_float3(rb[0] / g.nc[0], rb[1] / g.nc[1], rb[2] / g.nc[2]);
+  P.inv_h = make_float3(1.f / P.h.x, 1.f / P.h.y, 1.f / P.h.z);
+  const float rcm = rc_eff * 1.0001f + 1e-3f;  // far above the rounding of coordinates and bins
+  P.rcm2 = rcm * rcm;
 
-  size_t NF = (size_t)natoms * nframes, C = (size_t)g.ncell * nframes;
+  const size_t C = (size_t)g.ncell * nframes;
   char *w = (char *)workspace;
   int *cell_count = (int *)w; w += align_up(C * 4);
   int *cursor = (int *)w; w += align_up(C * 4);
   int *cell_start = (int *)w; w += align_up((C + 1) * 4);
   int *atom_cell = (int *)w; w += align_up(NF * 4);
-  int *cell_atoms = (int *)w; w += align_up(NF * 4);
   float4 *cell_pos = (float4 *)w; w += align_up(NF * 16);
   float *canon = ref_pos ? ref_pos : (float *)w;
 
-  nl_zero_kernel<<<(int)((C + 255) / 256), 256, 0, stream>>>(cell_count, (int)C, cursor, (int)C, gate);
   float3 L = make_float3(box[0], box[1], box[2]);
   float3 scale = make_float3(rb[0] / box[0], rb[1] / box[1], rb[2] / box[2]);
   int nb = (int)((NF + 255) / 256);
+  if (!g.image_mode) {
+    nl_zero_kernel<<<(int)((C + 255) / 256), 256, 0, stream>>>(cell_count, (int)C, cursor, (int)C, gate);
+    count_launch();
+  }
   nl_canon_kernel<<<nb, 256, 0, stream>>>(pos, perm, natoms, nframes, L, scale, P.L, P.nc, canon, atom_cell,
-                                          cell_count, gate, dbox);
-  nl_scan_kernel<<<1, 1024, 0, stream>>>(cell_count, cell_start, (int)C, gate);
-  nl_scatter_kernel<<<nb, 256, 0, stream>>>(atom_cell, cell_start, cursor, cell_atoms, canon, cell_pos, natoms,
-                                            nframes, g.ncell, gate);
+                                          g.image_mode ? nullptr : cell_count, gate, dbox);
+  if (!g.image_mode) {
+    nl_scan_kernel<<<1, 1024, 0, stream>>>(cell_count, cell_start, (int)C, gate);
+    nl_scatter_kernel<<<nb, 256, 0, stream>>>(atom_cell, cell_start, cursor, canon, cell_pos, natoms, nframes,
+                                              g.ncell, gate);
+    count_launch(2);
+  }
   if (nl_warps != 4 && nl_warps != 8 && nl_warps != 16) return DPB_ERR_INVALID_ARG;
   const int wpb = nl_warps, threads = 32 * wpb;  // centres (warps) per block
-  size_t smem = (size_t)wpb * ntypes * cap * 4;
+  size_t smem = (size_t)wpb * (512 + (size_t)ntypes * cap * 4);
   if (smem > 200 * 1024) return DPB_ERR_UNSUPPORTED;  // hit lists of this many warps do not fit
   if (smem > 48 * 1024) {
     DPB_CUDA_TRY(cudaFuncSetAttribute(nl_search_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   }
-  nl_search_kernel<<<(int)((NF + wpb - 1) / wpb), threads, smem, stream>>>(P, canon, cell_start, cell_atoms,
-                                                                           cell_pos, nbrs, counts, status, gate);
-  count_launch(5);
+  nl_search_kernel<<<(int)((NF + wpb - 1) / wpb), threads, smem, stream>>>(P, canon, cell_start, cell_pos, nbrs,
+                                                                           counts, status, gate);
+  count_launch(2);
   DPB_LAUNCH_CHECK();
   return DPB_OK;
 }
