@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_fwd(DevModel M, SysD
   __shared__ int gmax_s[4];  // largest |G| per slot (float bits)
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tbase_s;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tc::warp_index();
   const int row = tid & 127, half = tid >> 7;
   if (tid == 0) tc::mbar_init(&mbar, 1);
   if (warp == 0) tc::tmem_alloc(&tbase_s, 256);
@@ -542,7 +542,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_fwd(DevModel M, SysD
             tc::fence_proxy_async();  // the net image, copied with cp.async
             tc::fence_before_sync();
             __syncthreads();
-            if (tid == 0) {
+            if (warp == 0 && tc::elect_one()) {
               tc::fence_after_sync();
               split_mma<SD::K1>(tX, tY, w1_u, SD::W1B, idesc1);
               tc::commit(&mbar);
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_fwd(DevModel M, SysD
           tc::tmem_wait_st();
           tc::fence_before_sync();
           __syncthreads();
-          if (tid == 0) {
+          if (warp == 0 && tc::elect_one()) {
             tc::fence_after_sync();
             split_mma<SD::K2>(tX, tY, w2_u, SD::W2B, idesc2);
             split_mma<SD::K2>(tX + SD::NP, tY, w2_u + 2 * SD::W2B, SD::W2B, idesc2);
@@ -858,7 +858,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
   __shared__ double vir_s[9];
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tbase_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tc::warp_index(), lane = tid & 31;
   const int row = tid & 127, half = tid >> 7;
   if (tid < 9) vir_s[tid] = 0.0;
   if (tid == 0) tc::mbar_init(&mbar, 1);
@@ -968,7 +968,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
             tc::fence_proxy_async();
             tc::fence_before_sync();
             __syncthreads();
-            if (tid == 0) {
+            if (warp == 0 && tc::elect_one()) {
               tc::fence_after_sync();
               split_mma<SD::K1>(tX, tY, w1_u, SD::W1B, idesc1);
               split_mma<SD::K1>(tX + SD::N1, tY + SD::K1, w1_u, SD::W1B, idesc1);
@@ -988,7 +988,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
             tc::tmem_wait_st();
             tc::fence_before_sync();
             __syncthreads();  // A1 written (pass 0); the accumulators of pass 0 read (pass 1)
-            if (tid == 0) {
+            if (warp == 0 && tc::elect_one()) {
               tc::fence_after_sync();
               const uint32_t wp = w2_u + pass * 2 * SD::W2B;
               split_mma<SD::K2>(tX, tY, wp, SD::W2B, idesc2);

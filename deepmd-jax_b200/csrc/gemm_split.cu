@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_split(const __grid_con
   __shared__ uint32_t tbase_s;
   __shared__ int abort_s;
   volatile int *abort = &abort_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tc::warp_index(), lane = tid & 31;
   const int nc = (g.K + kGemmK - 1) / kGemmK;
   const int ntile = (g.N + NW - 1) / NW * g.mt0[g.ntypes];
   if (tid == 0) {
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_split(const __grid_con
 
   if (warp == 17) {
     // ================= weights: NW of the 128 rows of a stored tile per chunk
-    if (lane == 0) {
+    if (tc::elect_one()) {
       int issued = 0;
       for (int tile = blockIdx.x; tile < ntile && ok; tile += gridDim.x) {
         const GemmTilePos p = gemm_tile<NW>(g, tile);
@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_split(const __grid_con
     }
   } else if (warp == 16) {
     // ================= MMA issuer
-    if (lane == 0) {
+    if (tc::elect_one()) {
       int last = -1;
       uint32_t last_ph = 0;
       for (int tile = blockIdx.x; tile < ntile && ok; tile += gridDim.x) {

@@ -370,7 +370,7 @@ constexpr int kFwdCpt = 2;  // compaction candidates per thread, forward
 constexpr int kRowCapFwd = 128 + kFwdThreads * kFwdCpt;  // the carry (< 128) + one compaction round
 
 template <int E0, int E1, int E2>
-__global__ void __launch_bounds__(kFwdThreads, 2) k_mix_embed_fwd(DevModel M, SysDesc D, int ti,
+__global__ void __launch_bounds__(kFwdThreads, 2) k_mix_embed_fwd(DevModel M, SysDesc D, int wave,
                                                                   const float4 *__restrict__ posS,
                                                                   const float *__restrict__ box,
                                                                   const int32_t *__restrict__ nbrs,
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_mix_embed_fwd(DevModel M, Sy
   __shared__ float3 ri_s[kBlkAtoms];
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tbase_s;
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tc::warp_index();
   const int row = tid & 127, half = tid >> 7;
 
   for (int e = tid; e < kRblkBytes / 16; e += kFwdThreads) reinterpret_cast<uint4 *>(rblk)[e] = make_uint4(0, 0, 0, 0);
@@ -405,10 +405,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_mix_embed_fwd(DevModel M, Sy
   uint32_t ph = 0;
   bool ok = true;
 
-  const int cnt_i = D.offs[ti + 1] - D.offs[ti];
-  const int nbpf = (cnt_i + kBlkAtoms - 1) / kBlkAtoms;
-  const int nblk = nbpf * D.F;
-  const float inv_std = M.inv_std[ti], mean = M.mean[ti];
+  const int nblk = blocks_total(D, kBlkAtoms);
   const uint32_t idesc1 = tc::idesc_f16(128, MD::N1, 0, 0);
   const uint32_t idesc2 = tc::idesc_f16(128, MD::N2, 0, 0);
   const uint32_t idesc3 = tc::idesc_f16(128, MD::N2, 1, 1);
@@ -418,16 +415,16 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_mix_embed_fwd(DevModel M, Sy
   int loaded_net = -1;
 
   for (int blk = blockIdx.x; blk < nblk && ok; blk += gridDim.x) {
-    const int f = blk / nbpf, a0 = (blk - f * nbpf) * kBlkAtoms;
-    const int nb = min(kBlkAtoms, cnt_i - a0);
-    const size_t g0 = (size_t)f * D.N + D.offs[ti] + a0;
+    const BlkPos bp = block_pos(D, kBlkAtoms, blk);
+    const int ti = bp.ti, f = bp.f, nb = bp.nb;
+    const size_t g0 = bp.g0;
     const size_t frame_base = (size_t)f * D.N;
+    const float inv_std = M.inv_std[ti], mean = M.mean[ti];
     if (blk + (int)gridDim.x < nblk) {  // the next block's neighbour rows
-      const int bn = blk + gridDim.x, fn = bn / nbpf, an = (bn - fn * nbpf) * kBlkAtoms;
-      const size_t gn = (size_t)fn * D.N + D.offs[ti] + an;
-      const int nbn = min(kBlkAtoms, cnt_i - an);
-      if (rows_g != nullptr && D.S <= kRowStoreCap) prefetch_range_l2(rows_g + gn * kRowStoreCap, (size_t)nbn * D.S * 16);
-      else prefetch_range_l2(nbrs + gn * D.S, (size_t)nbn * D.S * 4);
+      const BlkPos bn = block_pos(D, kBlkAtoms, blk + gridDim.x);
+      if (rows_g != nullptr && D.S <= kRowStoreCap)
+        prefetch_range_l2(rows_g + bn.g0 * kRowStoreCap, (size_t)bn.nb * D.S * 16);
+      else prefetch_range_l2(nbrs + bn.g0 * D.S, (size_t)bn.nb * D.S * 4);
     }
     const int bs = box_slot(D, g0, f);  // the block's 8 atoms share one frame
     const float3 L = make_float3(box[bs * 3], box[bs * 3 + 1], box[bs * 3 + 2]);
@@ -444,8 +441,11 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_mix_embed_fwd(DevModel M, Sy
     bool pending = false;
     int my_slot = -1;
     int rowstart = 0, rowcount = 0;
-    // alternate the neighbour-type order between blocks so the resident net carries over
-    const int tj0 = (loaded_net >= 0) ? loaded_net - ti * M.ntypes : 0;
+    // The neighbour types' order rotates from one wave of `wave` blocks of a centre
+    // type to the next, so that the resident net mostly carries over; it depends on
+    // the block alone, so T's rounding does not depend on the launch.
+    const int local = blk - bp.first, turn = local / min(blocks_of_type(D, ti, kBlkAtoms), wave);
+    const int tj0 = turn * (D.ntypes - 1) % D.ntypes;
     for (int tt = 0; tt < D.ntypes && ok; ++tt) {
       const int tj = (tj0 + tt) % D.ntypes;
       const int sel = D.sel[tj];
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_mix_embed_fwd(DevModel M, Sy
           tc::fence_proxy_async();
           tc::fence_before_sync();
           __syncthreads();
-          if (tid == 0) {
+          if (warp == 0 && tc::elect_one()) {
             tc::fence_after_sync();
 #pragma unroll
             for (int ks = 0; ks < MD::K1 / 16; ++ks)
@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_mix_embed_fwd(DevModel M, Sy
           tc::fence_proxy_async();
           tc::fence_before_sync();
           __syncthreads();
-          if (tid == 0) {
+          if (warp == 0 && tc::elect_one()) {
             tc::fence_after_sync();
 #pragma unroll
             for (int ks = 0; ks < MD::K2 / 16; ++ks)
@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_mix_embed_fwd(DevModel M, Sy
           tc::fence_proxy_async();
           tc::fence_before_sync();
           __syncthreads();
-          if (tid == 0) {
+          if (warp == 0 && tc::elect_one()) {
             tc::fence_after_sync();
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks)
@@ -675,17 +675,16 @@ static int num_sms() {
 }
 
 template <int E0, int E1, int E2>
-int launch_mix_embed_fwd(const DevModel &M, const SysDesc &D, int ti, const float4 *posS,
+int launch_mix_embed_fwd(const DevModel &M, const SysDesc &D, const float4 *posS,
                          const float *box, const int32_t *nbrs, float *T, __half *G, const float4 *rows_g,
                          const int *rcnt, int *err, cudaStream_t st) {
-  const int cnt = D.offs[ti + 1] - D.offs[ti];
-  if (cnt == 0) return DPB_OK;
-  const int nblk = (cnt + kBlkAtoms - 1) / kBlkAtoms * D.F;
+  const int nblk = blocks_total(D, kBlkAtoms);
+  if (nblk == 0) return DPB_OK;
   const size_t smem = mix_fwd_smem<E0, E1, E2>();
   DPB_CUDA_TRY(cudaFuncSetAttribute(k_mix_embed_fwd<E0, E1, E2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)smem));
-  const int grid = nblk < 2 * num_sms() ? nblk : 2 * num_sms();
-  k_mix_embed_fwd<E0, E1, E2><<<grid, kFwdThreads, smem, st>>>(M, D, ti, posS, box, nbrs, T, G, rows_g, rcnt,
+  const int wave = 2 * num_sms(), grid = nblk < wave ? nblk : wave;
+  k_mix_embed_fwd<E0, E1, E2><<<grid, kFwdThreads, smem, st>>>(M, D, wave, posS, box, nbrs, T, G, rows_g, rcnt,
                                                                 err);
   count_launch();
   DPB_LAUNCH_CHECK();
@@ -949,7 +948,7 @@ constexpr int kRowCapBwd = 128 + kBwdThreads * kBwdCpt;
 constexpr int kDtbRows = 16 * kBlkAtoms;  // DTB rows: 16 per atom slot
 
 template <int E0, int E1, int E2>
-__global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, SysDesc D, int ti,
+__global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, SysDesc D,
                                                                   const float4 *__restrict__ posS,
                                                                   const float *__restrict__ box,
                                                                   const int32_t *__restrict__ nbrs,
@@ -976,7 +975,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
   __shared__ double vir_s[9];
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tbase_s;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tc::warp_index(), lane = tid & 31;
   const int row = tid & 127, half = tid >> 7;
 
   if (tid < 9) vir_s[tid] = 0.0;
@@ -1009,10 +1008,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
     __syncthreads();
   };
 
-  const int cnt_i = D.offs[ti + 1] - D.offs[ti];
-  const int nbpf = (cnt_i + kBlkAtoms - 1) / kBlkAtoms;
-  const int nblk = nbpf * D.F;
-  const float inv_std = M.inv_std[ti], mean = M.mean[ti];
+  const int nblk = blocks_total(D, kBlkAtoms);
   const uint32_t idesc1 = tc::idesc_f16(128, MD::N1, 0, 0);
   const uint32_t idesc2 = tc::idesc_f16(128, MD::N2, 0, 0);
   const uint32_t opb_u = tc::smem_u32(opb), dtb_u = tc::smem_u32(dtb);
@@ -1023,17 +1019,17 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
   int loaded_net = -1;
 
   for (int blk = blockIdx.x; blk < nblk && ok; blk += gridDim.x) {
-    const int f = blk / nbpf, a0 = (blk - f * nbpf) * kBlkAtoms;
-    const int nb = min(kBlkAtoms, cnt_i - a0);
-    const size_t g0 = (size_t)f * D.N + D.offs[ti] + a0;
+    const BlkPos bp = block_pos(D, kBlkAtoms, blk);
+    const int ti = bp.ti, f = bp.f, nb = bp.nb;
+    const size_t g0 = bp.g0;
     const size_t frame_base = (size_t)f * D.N;
+    const float inv_std = M.inv_std[ti], mean = M.mean[ti];
     if (blk + (int)gridDim.x < nblk) {  // the next block's neighbour rows and dE/dT rows
-      const int bn = blk + gridDim.x, fn = bn / nbpf, an = (bn - fn * nbpf) * kBlkAtoms;
-      const size_t gn = (size_t)fn * D.N + D.offs[ti] + an;
-      const int nbn = min(kBlkAtoms, cnt_i - an);
-      if (rows_g != nullptr && D.S <= kRowStoreCap) prefetch_range_l2(rows_g + gn * kRowStoreCap, (size_t)nbn * D.S * 16);
-      else prefetch_range_l2(nbrs + gn * D.S, (size_t)nbn * D.S * 4);
-      prefetch_range_l2(dTh + gn * 10 * MD::N2, (size_t)nbn * 10 * MD::N2 * 2);
+      const BlkPos bn = block_pos(D, kBlkAtoms, blk + gridDim.x);
+      if (rows_g != nullptr && D.S <= kRowStoreCap)
+        prefetch_range_l2(rows_g + bn.g0 * kRowStoreCap, (size_t)bn.nb * D.S * 16);
+      else prefetch_range_l2(nbrs + bn.g0 * D.S, (size_t)bn.nb * D.S * 4);
+      prefetch_range_l2(dTh + bn.g0 * 10 * MD::N2, (size_t)bn.nb * 10 * MD::N2 * 2);
     }
     const int bs = box_slot(D, g0, f);  // the block's 8 atoms share one frame
     if (bs != vframe) {
@@ -1063,7 +1059,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
     tc::cp_async_commit();
     __syncthreads();
     int rowstart = 0, rowcount = 0;
-    const int tj0 = (loaded_net >= 0) ? loaded_net - ti * M.ntypes : 0;
+    const int tj0 = (loaded_net >= 0 && loaded_net / M.ntypes == ti) ? loaded_net - ti * M.ntypes : 0;
     for (int tt = 0; tt < D.ntypes && ok; ++tt) {
       const int tj = (tj0 + tt) % D.ntypes;
       const int sel = D.sel[tj];
@@ -1105,7 +1101,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
             tc::fence_proxy_async();
             tc::fence_before_sync();
             __syncthreads();
-            if (tid == 0) {
+            if (warp == 0 && tc::elect_one()) {
               tc::fence_after_sync();
 #pragma unroll
               for (int ks = 0; ks < MD::K1 / 16; ++ks) {
@@ -1129,7 +1125,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
           tc::fence_proxy_async();
           tc::fence_before_sync();
           __syncthreads();
-          if (tid == 0) {
+          if (warp == 0 && tc::elect_one()) {
             tc::fence_after_sync();
 #pragma unroll
             for (int ks = 0; ks < MD::K2 / 16; ++ks) {
@@ -1150,7 +1146,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
           tc::fence_proxy_async();
           tc::fence_before_sync();
           __syncthreads();
-          if (tid == 0) {
+          if (warp == 0 && tc::elect_one()) {
             tc::fence_after_sync();
             const uint32_t idesc3 = tc::idesc_f16(128, 16 * (smax - smin + 1), 0, 0);
 #pragma unroll
@@ -1269,23 +1265,20 @@ size_t mix_bwd_smem() {
 }
 
 template <int E0, int E1, int E2>
-int launch_mix_embed_bwd(const DevModel &M, const SysDesc &D, int ti, const float4 *posS,
+int launch_mix_embed_bwd(const DevModel &M, const SysDesc &D, const float4 *posS,
                          const float *box, const int32_t *nbrs, const __half *dTh, const float *dTs,
                          const float4 *rows_g, const int *rcnt, float4 *F4, double *virial, int *err,
                          cudaStream_t st) {
-  using MD = MixDims<E0, E1, E2>;
-  const int cnt = D.offs[ti + 1] - D.offs[ti];
-  if (cnt == 0) return DPB_OK;
+  // one launch over every centre type and frame: a CTA's blocks run through the
+  // frames of a type in increasing order, and it flushes its virial sum to a
+  // frame's row before it moves on to the next frame (flush_virial)
+  const int nblk = blocks_total(D, kBlkAtoms);
+  if (nblk == 0) return DPB_OK;
   const size_t smem = mix_bwd_smem<E0, E1, E2>();
   DPB_CUDA_TRY(cudaFuncSetAttribute(k_mix_embed_bwd<E0, E1, E2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)smem));
-  // one launch over every frame: a CTA's blocks run through the frames in
-  // increasing order, and it flushes its virial sum to a frame's row before it
-  // moves on to the next frame (flush_virial), so the frames of PIMD beads or
-  // of a batch share one full-width grid
-  const int nblk = (cnt + kBlkAtoms - 1) / kBlkAtoms * D.F;
   const int grid = nblk < 2 * num_sms() ? nblk : 2 * num_sms();
-  k_mix_embed_bwd<E0, E1, E2><<<grid, kBwdThreads, smem, st>>>(M, D, ti, posS, box, nbrs, dTh, dTs, rows_g, rcnt, F4,
+  k_mix_embed_bwd<E0, E1, E2><<<grid, kBwdThreads, smem, st>>>(M, D, posS, box, nbrs, dTh, dTs, rows_g, rcnt, F4,
                                                                 virial, err);
   count_launch();
   DPB_LAUNCH_CHECK();
@@ -1379,14 +1372,20 @@ __device__ __forceinline__ FitGemm fit_gemm_info(const DevModel &M, int ti, int 
   return G;
 }
 
+// The 128-row tiles of every centre type in one launch: t0[k] is the first tile
+// of the k-th type present, ti[k] its index.
+struct FitTiles {
+  int n, ti[kMaxTypes], t0[kMaxTypes + 1], rows[kMaxTypes];
+  RowMap rm[kMaxTypes];
+};
+
 template <int FW, typename DGT, bool DEEP>
-__global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, int ti,
-                                                           int Mrows, RowMap rm,
+__global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, FitTiles ft,
                                                            const __half *__restrict__ Gh,
                                                            DGT *__restrict__ dGout, float *__restrict__ scratch,
                                                            float *__restrict__ Eatom, double *__restrict__ energy,
                                                            int N, int *__restrict__ err,
-                                                           const int32_t *__restrict__ seg, int tile0) {
+                                                           const int32_t *__restrict__ seg) {
   using C = FitCfg<FW, DEEP>;
   constexpr int ST = C::ST;
   static_assert(FW % 16 == 0 && FW <= 256, "fit width");
@@ -1397,7 +1396,7 @@ __global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, int ti,
   __shared__ uint32_t tbase_s;
   __shared__ int abort_s;
   __shared__ float esum_s[128];  // the second half's energy partial per atom
-  const int tid = threadIdx.x, warp = tid >> 5;
+  const int tid = threadIdx.x, warp = tc::warp_index();
   const int L = M.nfit, K0 = M.A * M.E2;
   const int NG = 2 * L - 1 + (K0 + kFitDgN - 1) / kFitDgN;
   volatile int *abort = &abort_s;
@@ -1421,11 +1420,17 @@ __global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, int ti,
   __syncthreads();
   tc::fence_after_sync();
   const uint32_t td = tbase_s;
-  const int r0 = blockIdx.x * 128, nrows = min(128, Mrows - r0);
+  int tk = 0;
+#pragma unroll
+  for (int k = 1; k < kMaxTypes; ++k)
+    if (k < ft.n && (int)blockIdx.x >= ft.t0[k]) tk = k;
+  const int ti = ft.ti[tk];
+  const RowMap rm = ft.rm[tk];
+  const int r0 = ((int)blockIdx.x - ft.t0[tk]) * 128, nrows = min(128, ft.rows[tk] - r0);
 
   if (warp == 9) {
     // ================= weight producer (one thread): bulk copies into free stages
-    if ((tid & 31) == 0) {
+    if (tc::elect_one()) {
       const uint32_t ring_u = tc::smem_u32(ring);
       int p = 0;  // chunks issued
       bool ok = true;
@@ -1444,7 +1449,7 @@ __global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, int ti,
     }
   } else if (warp == 8) {
     // ================= MMA issuer (one thread)
-    if ((tid & 31) == 0) {
+    if (tc::elect_one()) {
       const uint32_t ring_u = tc::smem_u32(ring), ha_u = tc::smem_u32(HA);
       int q = 0;  // chunks multiplied
       uint32_t epid_n = 0;
@@ -1518,7 +1523,7 @@ __global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, int ti,
     // per-CTA scratch tile [slot][n][thread] (coalesced): slots 0..L-2 tanh
     // values, L..2L-2 layer outputs (hidden layers below the last), 2L the
     // residual adjoint
-    float *tile = scratch + ((size_t)tile0 + blockIdx.x) * 128 * (size_t)(2 * L + 1) * FW + row;
+    float *tile = scratch + (size_t)blockIdx.x * 128 * (size_t)(2 * L + 1) * FW + row;
 #define FIT_SCR(slot, n) tile[((size_t)(slot) * FW + (n)) * 128]
     // L2 prefetch of one scratch slot of this warp's 32 rows and this half's
     // columns (one 128-byte line per column), issued before a layer's
@@ -1739,19 +1744,21 @@ int launch_mix_fit(const DevModel &M, const SysDesc &D, const __half *Gb, DGT *d
   if (!M.fit_bt[0][kFitBtDg]) return DPB_ERR_UNSUPPORTED;
   DPB_CUDA_TRY(
       cudaFuncSetAttribute(k_mix_fit<FW, DGT, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
-  int tile0 = 0;  // scratch tiles of 128 rows, consecutive over the centre types
+  FitTiles ft{};  // scratch tiles of 128 rows are numbered as the launch's tiles
   for (int ti = 0; ti < M.ntypes; ++ti) {
     const int cnt = D.offs[ti + 1] - D.offs[ti];
     if (!cnt) continue;
-    const RowMap rm{cnt, D.N, D.offs[ti]};
-    const int Mrows = cnt * D.F;
-    const int ntile = (Mrows + 127) / 128;
-    k_mix_fit<FW, DGT, DEEP><<<ntile, kFitThreads, C::SMEM, st>>>(M, ti, Mrows, rm, Gb, dG, scratch, Eatom, energy, D.N, err,
-                                                        D.seg, tile0);
-    tile0 += ntile;
-    count_launch();
-    DPB_LAUNCH_CHECK();
+    ft.ti[ft.n] = ti;
+    ft.rm[ft.n] = RowMap{cnt, D.N, D.offs[ti]};
+    ft.rows[ft.n] = cnt * D.F;
+    ft.t0[ft.n + 1] = ft.t0[ft.n] + (cnt * D.F + 127) / 128;
+    ++ft.n;
   }
+  if (ft.n == 0) return DPB_OK;
+  k_mix_fit<FW, DGT, DEEP><<<ft.t0[ft.n], kFitThreads, C::SMEM, st>>>(M, ft, Gb, dG, scratch, Eatom, energy, D.N, err,
+                                                                      D.seg);
+  count_launch();
+  DPB_LAUNCH_CHECK();
   return DPB_OK;
 }
 
@@ -1852,12 +1859,10 @@ int mixed_descriptors(const DevModel &M, const SysDesc &D, const float4 *posS, c
     const int rc = launch_rows(M, D, kBlkAtoms, posS, box, nbrs, rows, rcnt, st);
     if (rc) return rc;
   }
-  for (int ti = 0; ti < M.ntypes; ++ti) {
-    int rc = (M.E2 == 100)
-                 ? launch_mix_embed_fwd<25, 50, 100>(M, D, ti, posS, box, nbrs, T, Gb, rows, rcnt, err, st)
-                 : launch_mix_embed_fwd<32, 32, 64>(M, D, ti, posS, box, nbrs, T, Gb, rows, rcnt, err, st);
-    if (rc) return rc;
-  }
+  const int rc = (M.E2 == 100)
+                     ? launch_mix_embed_fwd<25, 50, 100>(M, D, posS, box, nbrs, T, Gb, rows, rcnt, err, st)
+                     : launch_mix_embed_fwd<32, 32, 64>(M, D, posS, box, nbrs, T, Gb, rows, rcnt, err, st);
+  if (rc) return rc;
   prof_end(PROF_MIXED_EMBED_FWD, st);
   return DPB_OK;
 }
@@ -2029,14 +2034,11 @@ int mixed_eval(const DevModel &M, const SysDesc &D, const float *pos, const int3
   if (rc) return rc;
   prof_end(PROF_MIXED_DT, st);
   prof_begin(PROF_MIXED_EMBED_BWD, st);
-  for (int ti = 0; ti < M.ntypes; ++ti) {
-    rc = (M.E2 == 100)
-             ? launch_mix_embed_bwd<25, 50, 100>(M, D, ti, posS, box, nbrs, mw.dTh, mw.dTs, mw.rows, mw.rcnt, F4,
-                                                 virial, err, st)
-             : launch_mix_embed_bwd<32, 32, 64>(M, D, ti, posS, box, nbrs, mw.dTh, mw.dTs, mw.rows, mw.rcnt, F4,
-                                               virial, err, st);
-    if (rc) return rc;
-  }
+  rc = (M.E2 == 100) ? launch_mix_embed_bwd<25, 50, 100>(M, D, posS, box, nbrs, mw.dTh, mw.dTs, mw.rows, mw.rcnt, F4,
+                                                         virial, err, st)
+                     : launch_mix_embed_bwd<32, 32, 64>(M, D, posS, box, nbrs, mw.dTh, mw.dTs, mw.rows, mw.rcnt, F4,
+                                                        virial, err, st);
+  if (rc) return rc;
   prof_end(PROF_MIXED_EMBED_BWD, st);
   return DPB_OK;
 }

@@ -24,6 +24,7 @@ __host__ __device__ constexpr int round1k(int x) { return (x + 1023) / 1024 * 10
 // blocks are numbered type after type, frame after frame within a type.
 struct BlkPos {
   int ti, f, nb;  // centre type, frame, atoms of the block
+  int first;      // number of the type's first block
   size_t g0;      // its first atom (f * N + sorted index)
 };
 __host__ __device__ __forceinline__ int blocks_of_type(const SysDesc &D, int ti, int ba) {
@@ -36,12 +37,13 @@ __host__ __device__ __forceinline__ int blocks_total(const SysDesc &D, int ba) {
 }
 __device__ __forceinline__ BlkPos block_pos(const SysDesc &D, int ba, int blk) {
   BlkPos b;
-  b.ti = 0;
+  b.ti = b.first = 0;
   int n = blocks_of_type(D, 0, ba);
 #pragma unroll
   for (int t = 1; t < kMaxTypes; ++t)
     if (t < D.ntypes && b.ti == t - 1 && blk >= n) {
       blk -= n;
+      b.first += n;
       b.ti = t;
       n = blocks_of_type(D, t, ba);
     }

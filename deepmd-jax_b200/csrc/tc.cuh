@@ -50,6 +50,23 @@ __host__ __device__ constexpr uint32_t idesc_f16(int M, int N, int a_mn, int b_m
          ((uint32_t)(M >> 4) << 24);
 }
 
+// True in one thread of a converged warp.  MMAs, commits and bulk copies are
+// issued under this (in a warp-uniform branch): their operands are uniform
+// registers, and under a plain `tid == 0` the compiler serialises over the
+// warp's possible operand values, 328 clocks per MMA instead of the 65 (N =
+// 128) or 118 (N = 240) that the MMA itself takes.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "elect.sync _|P, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(p));
+  return p != 0;
+}
+// The warp's index as a warp-uniform value.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 // tcgen05.mma kind::f16 issued by one thread: D (TMEM) (+)= A . B with FP32
 // accumulation; A and B are both BF16 or both FP16, as the instruction
 // descriptor says (idesc_bf16 / idesc_f16).
