@@ -1294,39 +1294,53 @@ int launch_mix_embed_bwd(const DevModel &M, const SysDesc &D, const float4 *posS
 //   g >= 2L - 1      dE/dG columns [128 p, 128 p + 128), p = g - (2L - 1), B: rows of W_0
 // Warp roles (320 threads): warps 0-7 are the epilogue, two threads per atom
 // (warps w and w + 4 share TMEM lane quarter w and take the two halves of
-// every layer's columns), which also stream layer 0's G rows into the ring
-// with cp.async; lane 0 of warp 8 issues the MMAs and lane 0 of warp 9 the
-// bulk (TMA) copies of the weights, each waiting only on its own barriers so
-// MMAs queue back to back.  Operands
-// pass through a ring of K = 16 stages (full / empty mbarriers), so the
-// weights of the next GEMM are already in flight while the epilogue of the
-// current one runs; the dE/dG passes alternate between two TMEM accumulators
-// so that the epilogue of pass p overlaps the MMAs of pass p + 1.
-// A stage holds the A chunk as [k8 (2)][row (128)][8 bf16] and the B chunk as
-// [k8 (2)][row (br)][8 bf16] (K-major core matrices, no swizzle: LBO = rows x
-// 16 B between the two K halves, SBO = 128 B between 8-row groups).  The
-// weights are stored pre-tiled in exactly this chunk layout (DevModel::fit_bt,
-// built at model creation), so a B chunk is one contiguous cp.async.bulk.
+// every layer's columns), which also stream layer 0's G rows; one
+// thread of warp 8 issues the MMAs and one of warp 9 the bulk (TMA) copies of
+// the weights, each waiting only on its own barriers so MMAs queue back to
+// back.  The weights pass through a ring of stages of KC K = 16 steps (full /
+// empty mbarriers), so those of the next GEMM are already in flight while the
+// epilogue of the current one runs; layer 0's A operand passes through a second
+// ring in the space that the activations take later.  The dE/dG passes
+// alternate between two TMEM accumulators so that the epilogue of pass p
+// overlaps the MMAs of pass p + 1.
+// A K = 16 step of the weights is [k8 (2)][row][8 fp16] (K-major core matrices,
+// no swizzle: LBO = rows x 16 B between the two K halves, SBO = 128 B between
+// 8-row groups).  The weights are stored pre-tiled in exactly this
+// layout (DevModel::fit_bt, built at model creation), so a stage is one
+// contiguous cp.async.bulk.
 // Epilogues run in FP32 on the CUDA cores: tanh, dt-residuals, the energy dot
 // product (FP64 segment sums) and the adjoint gates; tanh values and residual
-// sources go to a per-atom FP32 scratch, the BF16 activation of the next GEMM
-// stays in shared memory.  2 CTAs per SM, 256 TMEM columns each.
+// sources go to a per-atom FP32 scratch, the FP16 activation of the next GEMM
+// stays in shared memory, as do the biases, dt and output weights.
+//
+// What bounds it: the chain of a tile, GEMM after epilogue.  One tile of width 240
+// and K0 = 1600 took 153 us: the single issuing thread spent 470 clocks per step
+// on its wait and MMA (branches and uniform operands serialised, see
+// tc::elect_one), layer 0's ring ran empty at every stage, and each 8 columns of
+// an epilogue waited on L2 for 32 bytes of biases.  It takes 80 us: layer 0 16,
+// the six hidden GEMMs and epilogues 6 each, the dE/dG passes 25.  98,304 atoms
+// took 609 us and take 505 us.
 constexpr int kFitThreads = 320;
 constexpr int kFitEpi = 256;                 // epilogue threads: 2 per atom
 constexpr int kFitDgN = 128;                 // N of one dE/dG pass
-constexpr int kFitStageA = 2 * 128 * 16;     // A chunk bytes (K = 16)
+constexpr int kFitStepA = 2 * 128 * 16;      // A bytes of a K = 16 step
 
-// Ring depth: the shallow ring fits two CTAs per SM (one CTA's epilogue
-// overlaps the other's MMAs); the deep ring keeps 12 stages of weights in
-// flight for one CTA per SM.  dpb_md_autotune times both.
+// Pipeline shape: the shallow one (stages of two steps) fits two CTAs per SM
+// (one CTA's epilogue overlaps the other's MMAs); the deep one has stages of
+// four steps and more weights in flight, for one CTA per SM.  dpb_md_autotune
+// times both.
 template <int FW, bool DEEP>
 struct FitCfg {
   static constexpr int BR = FW > kFitDgN ? FW : kFitDgN;  // rows of the largest B box
-  static constexpr int STAGE = kFitStageA + 2 * BR * 16;
-  static constexpr int ST = DEEP ? 12 : (FW > 128 ? 4 : 8);
+  static constexpr int KC = DEEP ? 4 : 2;                 // K = 16 steps per stage
+  static constexpr int STAGE = KC * BR * 32, STAGEA = KC * kFitStepA;
   static constexpr int HAB = 128 * FW * 2;
-  static constexpr size_t SMEM = (size_t)round1k(HAB) + (size_t)ST * STAGE;
-  static_assert(SMEM <= 220 * 1024, "fitting ring");
+  static constexpr int RA = HAB > 3 * STAGEA ? HAB : 3 * STAGEA;  // activations, and layer 0's A ring
+  static constexpr int NA = RA / STAGEA < 8 ? RA / STAGEA : 8;
+  static constexpr int ST = DEEP ? (FW > 240 ? 4 : 5) : (FW > 240 ? 2 : 3);
+  // biases and dt of every layer, output weights
+  static size_t smem(int L) { return (size_t)RA + (size_t)ST * STAGE + (size_t)(2 * L + 1) * FW * 4; }
+  static_assert(RA + ST * STAGE + (2 * kMaxFitLayers + 1) * FW * 4 <= 226 * 1024, "fitting ring");
 };
 
 // Bounded mbarrier wait that also gives up once another role of the CTA gave
@@ -1341,11 +1355,25 @@ __device__ __forceinline__ bool fit_wait(uint64_t *bar, uint32_t parity, volatil
   return false;
 }
 
+// The same for a whole warp, one lane polling.
+__device__ __forceinline__ bool fit_wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort) {
+  bool ok = true;
+  if ((threadIdx.x & 31) == 0) ok = fit_wait(bar, parity, abort);
+  return __all_sync(0xffffffffu, ok);
+}
+
+// One arrival per warp, after its lanes' work.  (Polling and arriving by one lane
+// instead of all: 49,152 atoms in two CTAs per SM 315 -> 276 us.)
+__device__ __forceinline__ void fit_arrive_warp(uint64_t *bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) tc::mbar_arrive(bar);
+}
+
 // Epilogue -> issuer hand-over: TMEM reads done, shared-memory operand written.
 __device__ __forceinline__ void fit_signal(uint64_t *bar) {
   tc::fence_before_sync();
   tc::fence_proxy_async();
-  tc::mbar_arrive(bar);
+  fit_arrive_warp(bar);
 }
 
 struct FitGemm {
@@ -1380,19 +1408,20 @@ struct FitTiles {
 };
 
 template <int FW, typename DGT, bool DEEP>
-__global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, FitTiles ft,
+__global__ void __launch_bounds__(kFitThreads, DEEP ? 1 : 2) k_mix_fit(DevModel M, FitTiles ft,
                                                            const __half *__restrict__ Gh,
                                                            DGT *__restrict__ dGout, float *__restrict__ scratch,
                                                            float *__restrict__ Eatom, double *__restrict__ energy,
                                                            int N, int *__restrict__ err,
                                                            const int32_t *__restrict__ seg) {
   using C = FitCfg<FW, DEEP>;
-  constexpr int ST = C::ST;
+  constexpr int ST = C::ST, KC = C::KC, NA = C::NA;
   static_assert(FW % 16 == 0 && FW <= 256, "fit width");
   extern __shared__ __align__(1024) char smem[];
-  char *HA = smem;                        // 128 x FW bf16, K-major (kmajor_off)
-  char *ring = smem + round1k(C::HAB);    // ST stages
-  __shared__ __align__(8) uint64_t full[ST], fullA[ST], empty[ST], accf, accfD[2], epid, accfree[2];
+  char *HA = smem;              // 128 x FW fp16, K-major (kmajor_off); during layer 0 its A ring
+  char *ring = smem + C::RA;    // ST stages
+  float *cst = reinterpret_cast<float *>(ring + ST * C::STAGE);  // bias[l], dt[l], w_out
+  __shared__ __align__(8) uint64_t full[ST], empty[ST], fullA[NA], emptyA[NA], accf, accfD[2], epid, accfree[2];
   __shared__ uint32_t tbase_s;
   __shared__ int abort_s;
   __shared__ float esum_s[128];  // the second half's energy partial per atom
@@ -1403,57 +1432,83 @@ __global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, FitTiles
   if (tid == 0) {
     for (int s = 0; s < ST; ++s) {
       tc::mbar_init(&full[s], 1);
-      tc::mbar_init(&fullA[s], kFitEpi);
       tc::mbar_init(&empty[s], 1);
+    }
+    for (int s = 0; s < NA; ++s) {
+      tc::mbar_init(&fullA[s], kFitEpi / 32);
+      tc::mbar_init(&emptyA[s], 1);
     }
     tc::mbar_init(&accf, 1);
     tc::mbar_init(&accfD[0], 1);
     tc::mbar_init(&accfD[1], 1);
-    tc::mbar_init(&epid, kFitEpi);
-    tc::mbar_init(&accfree[0], kFitEpi);
-    tc::mbar_init(&accfree[1], kFitEpi);
+    tc::mbar_init(&epid, kFitEpi / 32);
+    tc::mbar_init(&accfree[0], kFitEpi / 32);
+    tc::mbar_init(&accfree[1], kFitEpi / 32);
     abort_s = 0;
     tc::fence_mbar_init();
   }
-  if (warp == 0) tc::tmem_alloc(&tbase_s, 256);
-  tc::fence_before_sync();
-  __syncthreads();
-  tc::fence_after_sync();
-  const uint32_t td = tbase_s;
   int tk = 0;
 #pragma unroll
   for (int k = 1; k < kMaxTypes; ++k)
     if (k < ft.n && (int)blockIdx.x >= ft.t0[k]) tk = k;
   const int ti = ft.ti[tk];
   const RowMap rm = ft.rm[tk];
+  static_assert(FW <= kFitThreads, "one column per thread");
+  if (tid < FW) {  // every load in flight before the first store
+    float v[2 * kMaxFitLayers + 1];
+#pragma unroll
+    for (int l = 0; l < kMaxFitLayers; ++l) {
+      v[2 * l] = l < L ? M.mfb[ti][l][tid] : 0.f;
+      v[2 * l + 1] = l < L && M.mfdt[ti][l] ? M.mfdt[ti][l][tid] : 1.f;
+    }
+    v[2 * kMaxFitLayers] = M.mfwout[ti][tid];
+#pragma unroll
+    for (int l = 0; l < kMaxFitLayers; ++l)
+      if (l < L) {
+        cst[l * FW + tid] = v[2 * l];
+        cst[(L + l) * FW + tid] = v[2 * l + 1];
+      }
+    cst[2 * L * FW + tid] = v[2 * kMaxFitLayers];
+  }
+  if (warp == 0) tc::tmem_alloc(&tbase_s, 256);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t td = tbase_s;
   const int r0 = ((int)blockIdx.x - ft.t0[tk]) * 128, nrows = min(128, ft.rows[tk] - r0);
 
   if (warp == 9) {
     // ================= weight producer (one thread): bulk copies into free stages
     if (tc::elect_one()) {
       const uint32_t ring_u = tc::smem_u32(ring);
-      int p = 0;  // chunks issued
+      int p = 0, s = 0;  // stages filled, current stage
+      uint32_t ph = 1;   // parity of its previous use
       bool ok = true;
       for (int g = 0; g < NG && ok; ++g) {
         const FitGemm gi = fit_gemm_info<FW>(M, ti, g, L, K0);
-        const uint32_t bytes = (uint32_t)gi.br * 32u;
-        for (int k = 0; k < gi.nk; ++k, ++p) {
-          const int s = p % ST;
-          if (p >= ST && !(ok = fit_wait(&empty[s], ((p / ST) - 1) & 1, abort))) break;
+        const char *src = gi.src;
+        for (int k = 0; k < gi.nk; k += KC, ++p) {
+          if (p >= ST && !(ok = fit_wait(&empty[s], ph, abort))) break;
+          const uint32_t bytes = (uint32_t)min(KC, gi.nk - k) * gi.br * 32u;
           tc::mbar_arrive_expect_tx(&full[s], bytes);
-          tc::bulk_load(ring_u + s * C::STAGE + kFitStageA, gi.src + (size_t)k * bytes, bytes, &full[s]);
+          tc::bulk_load(ring_u + s * C::STAGE, src, bytes, &full[s]);
+          src += bytes;
+          if (++s == ST) {
+            s = 0;
+            ph ^= 1;
+          }
         }
       }
-      // copies still in flight only after a give-up: the last ST issued chunks
+      // copies still in flight only after a give-up: the last ST filled stages
       for (int c = p > ST ? p - ST : 0; c < p; ++c) tc::mbar_wait(&full[c % ST], (c / ST) & 1);
     }
   } else if (warp == 8) {
     // ================= MMA issuer (one thread)
     if (tc::elect_one()) {
       const uint32_t ring_u = tc::smem_u32(ring), ha_u = tc::smem_u32(HA);
-      int q = 0;  // chunks multiplied
-      uint32_t epid_n = 0;
-      bool ok = true;
+      int s = 0, sa = 0;
+      uint32_t ph = 0, pha = 0, epid_n = 0;
+      bool ok = true, any = false;
       for (int g = 0; g < NG && ok; ++g) {
         const FitGemm gi = fit_gemm_info<FW>(M, ti, g, L, K0);
         if (g >= 1 && g <= 2 * L - 1) {  // A operand (and the accumulator) handed back by the epilogue
@@ -1465,25 +1520,49 @@ __global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, FitTiles
         }
         if (!ok) break;
         tc::fence_after_sync();
-        const uint32_t idesc = tc::idesc_f16(128, gi.N, 0, 0);
-        for (int k = 0; k < gi.nk; ++k, ++q) {
-          const int s = q % ST;
-          const uint32_t par = (q / ST) & 1;
-          ok = fit_wait(&full[s], par, abort) && (g != 0 || fit_wait(&fullA[s], par, abort));
+        const uint32_t idesc = tc::idesc_f16(128, gi.N, 0, 0), d = td + gi.col, bl = (uint32_t)gi.br * 16,
+                       bstep = (uint32_t)gi.br * 32;
+        // one stage's steps: A at a0 + j astep
+        auto steps = [&](int n, uint32_t a0, uint32_t astep, uint32_t albo, uint32_t asbo, bool acc) {
+          const uint32_t b0 = ring_u + s * C::STAGE;
+          if (n == KC) {
+#pragma unroll
+            for (int j = 0; j < KC; ++j)
+              tc::mma_f16kind(d, tc::make_desc(a0 + j * astep, albo, asbo), tc::make_desc(b0 + j * bstep, bl, 128), idesc,
+                              (j > 0 || acc) ? 1u : 0u);
+          } else {
+            for (int j = 0; j < n; ++j)
+              tc::mma_f16kind(d, tc::make_desc(a0 + j * astep, albo, asbo), tc::make_desc(b0 + j * bstep, bl, 128), idesc,
+                              (j > 0 || acc) ? 1u : 0u);
+          }
+          tc::commit(&empty[s]);
+        };
+        for (int k = 0; k < gi.nk; k += KC) {
+          ok = fit_wait(&full[s], ph, abort) && (g != 0 || fit_wait(&fullA[sa], pha, abort));
           if (!ok) break;
           tc::fence_after_sync();
-          const uint32_t st_u = ring_u + s * C::STAGE;
-          const uint64_t ad = (g == 0) ? tc::make_desc(st_u, 128 * 16, 128)
-                                       : tc::make_desc(ha_u + tc::kmajor_off(0, 16 * k, FW), 128, (FW / 8) * 128);
-          const uint64_t bd = tc::make_desc(st_u + kFitStageA, (uint32_t)gi.br * 16, 128);
-          tc::mma_f16kind(td + gi.col, ad, bd, idesc, k > 0 ? 1u : 0u);
-          tc::commit(&empty[s]);
+          any = true;
+          const int n = min(KC, gi.nk - k);
+          if (g == 0) {
+            steps(n, ha_u + sa * C::STAGEA, tc::kmajor_off(0, 16, 16 * KC), 128, 16 * KC * 16, k > 0);
+            tc::commit(&emptyA[sa]);
+            if (++sa == NA) {
+              sa = 0;
+              pha ^= 1;
+            }
+          } else {
+            steps(n, ha_u + tc::kmajor_off(0, 16 * k, FW), tc::kmajor_off(0, 16, FW), 128, (FW / 8) * 128, k > 0);
+          }
+          if (++s == ST) {
+            s = 0;
+            ph ^= 1;
+          }
         }
         if (!ok) break;
         tc::commit(g < 2 * L - 1 ? &accf : &accfD[(g - (2 * L - 1)) & 1]);
       }
-      // the last MMAs complete before the CTA exits
-      if (q > 0) tc::mbar_wait(&empty[(q - 1) % ST], ((q - 1) / ST) & 1);
+      // the last MMAs complete before the CTA exits: the stage before s
+      if (any) tc::mbar_wait(&empty[s ? s - 1 : ST - 1], s ? ph : ph ^ 1);
     }
   } else {
     // ================= epilogue warps: two threads per atom = TMEM lane; half
@@ -1497,25 +1576,51 @@ __global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, FitTiles
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
     const int cb = half * FH, ce = cb + FH;  // this half's hidden columns
     bool ok = true;
-    // ---- layer 0's A operand: this atom's G row (each half copies its 16
-    // bytes of every 32-byte K chunk), ST - 1 chunks in flight
+    // ---- layer 0's A operand: an instruction loads 64 bytes of 8 rows (whole
+    // sectors, and stores without bank conflicts; a thread per row took 1,700
+    // clocks per stage), PF stages ahead in registers.  (With asynchronous copies signalled NA - 1 stages later the
+    // ring ran empty at every stage: 2,100 clocks each against 470 of its MMAs.)
     {
-      const int nch0 = K0 / 16;
-      const char *grow = reinterpret_cast<const char *>(Gh + me * (size_t)K0);
-      for (int c = 0; c < nch0 + ST - 1; ++c) {
-        if (c < nch0) {
-          const int s = c % ST;
-          if (c >= ST && !(ok = __all_sync(0xffffffffu, fit_wait(&empty[s], ((c / ST) - 1) & 1, abort)))) break;
-          char *dst = ring + s * C::STAGE + half * 128 * 16 + row * 16;
-          if (act) tc::cp_async16(dst, grow + c * 32 + half * 16);
-          else *reinterpret_cast<uint4 *>(dst) = make_uint4(0, 0, 0, 0);
-        }
-        tc::cp_async_commit();
-        const int cc = c - (ST - 1);
-        if (cc >= 0) {
-          tc::cp_async_wait<ST - 1>();
+      constexpr int PF = 8 / KC;
+      const int nk0 = K0 / 16, nst = (nk0 + KC - 1) / KC;
+      // instruction q: rows 8 (q & 1) + lane % 8 of the warp's 16, 8-wide K groups 4 (q >> 1) + lane / 8
+      const int lane = tid & 31, k8 = lane >> 3, r_first = 16 * warp + (lane & 7);
+      const char *grow[2];
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int r = r_first + 8 * q;
+        grow[q] = r < nrows ? reinterpret_cast<const char *>(Gh + rm.atom(r0 + r) * (size_t)K0) + k8 * 16 : nullptr;
+      }
+      char *dst0 = HA + tc::kmajor_off(r_first, 8 * k8, 16 * KC);
+      uint4 v[PF][KC];
+      auto load = [&](int c, uint4 (&x)[KC]) {
+#pragma unroll
+        for (int q = 0; q < KC; ++q)
+          x[q] = grow[q & 1] && c * KC + 2 * (q >> 1) + (k8 >> 1) < nk0
+                     ? *reinterpret_cast<const uint4 *>(grow[q & 1] + c * KC * 32 + (q >> 1) * 64)
+                     : make_uint4(0, 0, 0, 0);
+      };
+#pragma unroll
+      for (int p = 0; p < PF; ++p) load(p, v[p]);
+      int s = 0;
+      uint32_t ph = 1;  // parity of the stage's previous use
+      for (int c0 = 0; c0 < nst && ok; c0 += PF) {
+#pragma unroll
+        for (int p = 0; p < PF; ++p) {
+          const int c = c0 + p;
+          if (c >= nst || !ok) continue;
+          if (c >= NA && !(ok = fit_wait_warp(&emptyA[s], ph, abort))) continue;
+          char *dst = dst0 + s * C::STAGEA;
+#pragma unroll
+          for (int q = 0; q < KC; ++q)
+            *reinterpret_cast<uint4 *>(dst + tc::kmajor_off(8 * (q & 1), 32 * (q >> 1), 16 * KC)) = v[p][q];
+          load(c + PF, v[p]);
           tc::fence_proxy_async();
-          tc::mbar_arrive(&fullA[cc % ST]);
+          fit_arrive_warp(&fullA[s]);
+          if (++s == NA) {
+            s = 0;
+            ph ^= 1;
+          }
         }
       }
     }
@@ -1535,60 +1640,65 @@ __global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, FitTiles
     // ---- forward; the last layer's epilogue also forms the atom energy and
     // the first adjoint gate g = w_out dt (1 - t^2), the A operand of adjoint
     // layer L-1 (its t and h never go to the scratch)
-    const float *wf = M.mfwout[ti];
     float e_sum = 0.f;
     for (int l = 0; l < L && ok; ++l) {
-      if (M.mfdt[ti][l]) prefetch_slot(L + l - 1);
-      ok = __all_sync(0xffffffffu, fit_wait(&accf, accf_n & 1, abort));
+      if (M.mfdt[ti][l]) prefetch_slot(M.mfdt[ti][l - 1] ? L + l - 1 : l - 1);
+      ok = fit_wait_warp(&accf, accf_n & 1, abort);
       ++accf_n;
       if (!ok) break;
       tc::fence_after_sync();
       const bool last = l == L - 1;
-      const float *bias = M.mfb[ti][l], *dt = M.mfdt[ti][l];
+      const float *dt = M.mfdt[ti][l];
       const float usc = 1.f / M.fit_wsc[ti][l];         // a power of two: exact
       const float gsc = last ? M.fit_gsc[ti][l] : 1.f;  // the gate's operand scale
-      // residual sources of the current chunk, loaded one chunk ahead so the
-      // scratch reads overlap the TMEM loads and the previous chunk's math
-      float hp[8];
+      // residual sources of two chunks of 8 columns, each reloaded for the chunk
+      // after next as soon as it is used
+      const bool res = dt != nullptr;
+      const int hs = res && !M.mfdt[ti][l - 1] ? l - 1 : L + l - 1;  // the layer below's output
+      const float *cb_ = cst + l * FW, *cd_ = cst + (L + l) * FW, *cw_ = cst + 2 * L * FW;
+      float hp[2][8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) hp[i] = dt ? FIT_SCR(L + l - 1, cb + i) : 0.f;
-      for (int c0 = cb; c0 < ce; c0 += 8) {
-        uint32_t r[8];
-        tc::tmem_ld8_issue(td + lane_off + c0, r);
-        float hn[8];
+      for (int q = 0; q < 2; ++q)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) hn[i] = (dt && c0 + 8 < ce) ? FIT_SCR(L + l - 1, c0 + 8 + i) : 0.f;
-        float bv[8], dv[8], wv[8];
-#pragma unroll
-        for (int i = 0; i < 8; i += 4) {
-          const float4 b4 = __ldg(reinterpret_cast<const float4 *>(bias + c0 + i));
-          bv[i] = b4.x; bv[i + 1] = b4.y; bv[i + 2] = b4.z; bv[i + 3] = b4.w;
-          const float4 d4 =
-              dt ? __ldg(reinterpret_cast<const float4 *>(dt + c0 + i)) : make_float4(1.f, 1.f, 1.f, 1.f);
-          dv[i] = d4.x; dv[i + 1] = d4.y; dv[i + 2] = d4.z; dv[i + 3] = d4.w;
-          const float4 w4 = last ? __ldg(reinterpret_cast<const float4 *>(wf + c0 + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
-          wv[i] = w4.x; wv[i + 1] = w4.y; wv[i + 2] = w4.z; wv[i + 3] = w4.w;
-        }
-        tc::tmem_wait();
+        for (int i = 0; i < 8; ++i) hp[q][i] = (res && cb + 8 * q < ce) ? FIT_SCR(hs, cb + 8 * q + i) : 0.f;
+      auto chunk = [&](int c0, const uint32_t (&r)[8], float (&h_prev)[8]) {
         float hv[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int n = c0 + i;
-          const float t = tc::tanh_fast(fmaf(__uint_as_float(r[i]), usc, bv[i]));
-          float h = t;
-          if (dt) h = t * dv[i] + hp[i];
-          if (!last) {
-            hv[i] = h;
-            FIT_SCR(l, n) = t;
-            FIT_SCR(L + l, n) = h;
-          } else {
-            e_sum = fmaf(h, wv[i], e_sum);
-            hv[i] = wv[i] * dv[i] * (1.f - t * t);
+        for (int q = 0; q < 8; q += 4) {
+          const float4 b4 = *reinterpret_cast<const float4 *>(cb_ + c0 + q);
+          const float4 d4 = *reinterpret_cast<const float4 *>(cd_ + c0 + q);
+          const float4 w4 = last ? *reinterpret_cast<const float4 *>(cw_ + c0 + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float bv[4] = {b4.x, b4.y, b4.z, b4.w}, dv[4] = {d4.x, d4.y, d4.z, d4.w},
+                      wv[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int i = q + e, n = c0 + i;
+            const float t = tc::tanh_fast(fmaf(__uint_as_float(r[i]), usc, bv[e]));
+            float h = t;
+            if (res) h = t * dv[e] + h_prev[i];
+            if (!last) {
+              hv[i] = h;
+              FIT_SCR(l, n) = t;
+              if (res) FIT_SCR(L + l, n) = h;  // without a residual h is t
+            } else {
+              e_sum = fmaf(h, wv[e], e_sum);
+              hv[i] = wv[e] * dv[e] * (1.f - t * t);
+            }
           }
         }
+        if (res && c0 + 16 < ce) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) hp[i] = hn[i];
+          for (int i = 0; i < 8; ++i) h_prev[i] = FIT_SCR(hs, c0 + 16 + i);
+        }
         *reinterpret_cast<uint4 *>(HA + tc::kmajor_off(row, c0, FW)) = pack8h(hv, gsc);
+      };
+      for (int c0 = cb; c0 < ce; c0 += 16) {
+        uint32_t ra[8], rb[8];
+        tc::tmem_ld8_issue(td + lane_off + c0, ra);
+        if (c0 + 8 < ce) tc::tmem_ld8_issue(td + lane_off + c0 + 8, rb);
+        tc::tmem_wait();
+        chunk(c0, ra, hp[0]);
+        if (c0 + 8 < ce) chunk(c0 + 8, rb, hp[1]);
       }
       fit_signal(&epid);
     }
@@ -1621,55 +1731,57 @@ __global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, FitTiles
     for (int l = L - 1; l >= 1 && ok; --l) {
       if (M.mfdt[ti][l] != nullptr && l != L - 1) prefetch_slot(2 * L);
       prefetch_slot(l - 1);
-      ok = __all_sync(0xffffffffu, fit_wait(&accf, accf_n & 1, abort));
+      ok = fit_wait_warp(&accf, accf_n & 1, abort);
       ++accf_n;
       if (!ok) break;
       tc::fence_after_sync();
       const bool res_l = M.mfdt[ti][l] != nullptr, res_lm1 = (l - 1 > 0) && M.mfdt[ti][l - 1] != nullptr;
-      const float *dtm1 = M.mfdt[ti][l - 1];
       const bool use_gh = res_l && l != L - 1;
       const float usc = 1.f / (M.fit_wsc[ti][l] * M.fit_gsc[ti][l]), gsc = M.fit_gsc[ti][l - 1];
-      float ghc[8], tcur[8];
+      // dt of layer l - 1 (1 without residual), output weights
+      const float *cd_ = cst + (L + l - 1) * FW, *cw_ = cst + 2 * L * FW;
+      float ghc[2][8], tcur[2][8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        ghc[i] = use_gh ? FIT_SCR(2 * L, cb + i) : 0.f;
-        tcur[i] = FIT_SCR(l - 1, cb + i);
-      }
-      for (int c0 = cb; c0 < ce; c0 += 8) {
-        uint32_t r[8];
-        tc::tmem_ld8_issue(td + lane_off + c0, r);
-        float ghn[8], tn[8];
+      for (int q = 0; q < 2; ++q)
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          ghn[i] = (use_gh && c0 + 8 < ce) ? FIT_SCR(2 * L, c0 + 8 + i) : 0.f;
-          tn[i] = (c0 + 8 < ce) ? FIT_SCR(l - 1, c0 + 8 + i) : 0.f;
+          const bool in = cb + 8 * q < ce;
+          ghc[q][i] = (use_gh && in) ? FIT_SCR(2 * L, cb + 8 * q + i) : 0.f;
+          tcur[q][i] = in ? FIT_SCR(l - 1, cb + 8 * q + i) : 0.f;
         }
-        float wv[8], dv[8];
-#pragma unroll
-        for (int i = 0; i < 8; i += 4) {
-          const float4 w4 = __ldg(reinterpret_cast<const float4 *>(wf + c0 + i));
-          wv[i] = w4.x; wv[i + 1] = w4.y; wv[i + 2] = w4.z; wv[i + 3] = w4.w;
-          const float4 d4 =
-              res_lm1 ? __ldg(reinterpret_cast<const float4 *>(dtm1 + c0 + i)) : make_float4(1.f, 1.f, 1.f, 1.f);
-          dv[i] = d4.x; dv[i + 1] = d4.y; dv[i + 2] = d4.z; dv[i + 3] = d4.w;
-        }
-        tc::tmem_wait();
+      auto chunk = [&](int c0, const uint32_t (&r)[8], float (&gh)[8], float (&tt)[8]) {
         float gz[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int n = c0 + i;
-          float g = __uint_as_float(r[i]) * usc;
-          if (res_l) g += (l == L - 1) ? wv[i] : ghc[i];
-          const float t = tcur[i];
-          gz[i] = g * dv[i] * (1.f - t * t);
-          if (res_lm1) FIT_SCR(2 * L, n) = g;
-        }
+        for (int q = 0; q < 8; q += 4) {
+          const float4 w4 = *reinterpret_cast<const float4 *>(cw_ + c0 + q);
+          const float4 d4 = res_lm1 ? *reinterpret_cast<const float4 *>(cd_ + c0 + q) : make_float4(1.f, 1.f, 1.f, 1.f);
+          const float wv[4] = {w4.x, w4.y, w4.z, w4.w}, dv[4] = {d4.x, d4.y, d4.z, d4.w};
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          ghc[i] = ghn[i];
-          tcur[i] = tn[i];
+          for (int e = 0; e < 4; ++e) {
+            const int i = q + e, n = c0 + i;
+            float g = __uint_as_float(r[i]) * usc;
+            if (res_l) g += (l == L - 1) ? wv[e] : gh[i];
+            const float t = tt[i];
+            gz[i] = g * dv[e] * (1.f - t * t);
+            if (res_lm1) FIT_SCR(2 * L, n) = g;
+          }
+        }
+        if (c0 + 16 < ce) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            if (use_gh) gh[i] = FIT_SCR(2 * L, c0 + 16 + i);
+            tt[i] = FIT_SCR(l - 1, c0 + 16 + i);
+          }
         }
         *reinterpret_cast<uint4 *>(HA + tc::kmajor_off(row, c0, FW)) = pack8h(gz, gsc);
+      };
+      for (int c0 = cb; c0 < ce; c0 += 16) {
+        uint32_t ra[8], rb[8];
+        tc::tmem_ld8_issue(td + lane_off + c0, ra);
+        if (c0 + 8 < ce) tc::tmem_ld8_issue(td + lane_off + c0 + 8, rb);
+        tc::tmem_wait();
+        chunk(c0, ra, ghc[0], tcur[0]);
+        if (c0 + 8 < ce) chunk(c0 + 8, rb, ghc[1], tcur[1]);
       }
       fit_signal(&epid);
     }
@@ -1678,7 +1790,7 @@ __global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, FitTiles
     const int npass = (K0 + kFitDgN - 1) / kFitDgN;
     const float usc0 = 1.f / (M.fit_wsc[ti][0] * M.fit_gsc[ti][0]);
     for (int pp = 0; pp < npass && ok; ++pp) {
-      ok = __all_sync(0xffffffffu, fit_wait(&accfD[pp & 1], (pp >> 1) & 1, abort));
+      ok = fit_wait_warp(&accfD[pp & 1], (pp >> 1) & 1, abort);
       if (!ok) break;
       tc::fence_after_sync();
       const int n0 = kFitDgN * pp, nv = min(kFitDgN, K0 - n0);
@@ -1726,7 +1838,7 @@ __global__ void __launch_bounds__(kFitThreads, 2) k_mix_fit(DevModel M, FitTiles
         }
       }
       tc::fence_before_sync();
-      tc::mbar_arrive(&accfree[pp & 1]);
+      fit_arrive_warp(&accfree[pp & 1]);
     }
 #undef FIT_SCR
   }
@@ -1743,7 +1855,7 @@ int launch_mix_fit(const DevModel &M, const SysDesc &D, const __half *Gb, DGT *d
   using C = FitCfg<FW, DEEP>;
   if (!M.fit_bt[0][kFitBtDg]) return DPB_ERR_UNSUPPORTED;
   DPB_CUDA_TRY(
-      cudaFuncSetAttribute(k_mix_fit<FW, DGT, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM));
+      cudaFuncSetAttribute(k_mix_fit<FW, DGT, DEEP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem(M.nfit)));
   FitTiles ft{};  // scratch tiles of 128 rows are numbered as the launch's tiles
   for (int ti = 0; ti < M.ntypes; ++ti) {
     const int cnt = D.offs[ti + 1] - D.offs[ti];
@@ -1755,7 +1867,7 @@ int launch_mix_fit(const DevModel &M, const SysDesc &D, const __half *Gb, DGT *d
     ++ft.n;
   }
   if (ft.n == 0) return DPB_OK;
-  k_mix_fit<FW, DGT, DEEP><<<ft.t0[ft.n], kFitThreads, C::SMEM, st>>>(M, ft, Gb, dG, scratch, Eatom, energy, D.N, err,
+  k_mix_fit<FW, DGT, DEEP><<<ft.t0[ft.n], kFitThreads, C::smem(M.nfit), st>>>(M, ft, Gb, dG, scratch, Eatom, energy, D.N, err,
                                                                       D.seg);
   count_launch();
   DPB_LAUNCH_CHECK();
@@ -1766,6 +1878,13 @@ int launch_mix_fit(const DevModel &M, const SysDesc &D, const __half *Gb, DGT *d
 template <int FW, typename DGT>
 static int launch_mix_fit_d(const DevModel &M, const SysDesc &D, const __half *Gb, DGT *dG, float *scratch,
                             float *Eatom, double *energy, int *err, bool deep, cudaStream_t st) {
+  // two tiles that share an SM take 5/3 of one that has it to itself (138 us and
+  // 83 us at width 240, K0 = 1600), so the shape with fewer such units in its
+  // whole waves is taken
+  int tiles = 0;
+  for (int ti = 0; ti < M.ntypes; ++ti) tiles += ((D.offs[ti + 1] - D.offs[ti]) * D.F + 127) / 128;
+  const int sms = num_sms();
+  deep = deep || 3 * ((tiles + sms - 1) / sms) < 5 * ((tiles + 2 * sms - 1) / (2 * sms));
   return deep ? launch_mix_fit<FW, DGT, true>(M, D, Gb, dG, scratch, Eatom, energy, err, st)
               : launch_mix_fit<FW, DGT, false>(M, D, Gb, dG, scratch, Eatom, energy, err, st);
 }
