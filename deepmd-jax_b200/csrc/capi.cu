@@ -75,6 +75,7 @@ int launch_embed_bwd_cmp(const DevModel &, const SysDesc &, int, const float *, 
                          const int32_t *, const float *, const float *, float4 *, double *, cudaStream_t);
 // fitting GEMMs on the tensor cores (gemm_split.cu)
 size_t gemm_tiles_halves(int N, int K);
+size_t gemm_operand_halves(int mt, int K);
 int launch_gemm_tiles(const float *w, int N, int K, int sn, int sk, float scale, __half *out);
 int launch_gemm_split(const GemmArgs &g, cudaStream_t st);
 // any embedding shape (eval_general.cu)
@@ -82,7 +83,7 @@ int launch_embed_fwd_gen(const DevModel &, const SysDesc &, int, const float *, 
                          const int32_t *, float *, float *, float *, cudaStream_t);
 int launch_embed_bwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
                          const int32_t *, const float *, const float *, float4 *, double *, cudaStream_t);
-int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, float *gZ, double *energy,
+int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, __half *gZ, double *energy,
                       const int32_t *seg, cudaStream_t st);
 int launch_finalize(int, int, const float4 *, float *, const float *, const int32_t *, float *, double *, int,
                     const float *, const int32_t *, uint32_t *, cudaStream_t);
@@ -398,15 +399,17 @@ static int fit_width_max(const DevModel &M) {
   return w;
 }
 
-static size_t fp32_ws_per_atom(const DevModel &M) {
+static size_t fp32_ws_bytes(const DevModel &M, size_t NF) {
   int hid = 0;
   for (int l = 0; l < M.nfit; ++l) hid += M.FW[l];
-  return (size_t)(10 * M.E2 + M.A * M.E2 + 2 * hid + 4 * fit_width_max(M) + 1) * 4 + 16;
+  const size_t fw = fit_width_max(M), fwp = (fw + 31) / 32 * 32;  // operand tiles are 128 rows x 32 columns
+  return al(NF * ((10 * M.E2 + M.A * M.E2 + 2 * hid + 2 * fw + 2 * fwp + 1) * 4 + 16)) +
+         al((size_t)128 * M.ntypes * 2 * fwp * 4);
 }
 
 // Workspace of NF atoms with nE energy / virial rows.
 static size_t eval_ws_bytes(const DevModel &M, size_t NF, size_t nE) {
-  size_t a = al(NF * fp32_ws_per_atom(M)) + 16 * 256 + al(nE * 9 * 8);
+  size_t a = fp32_ws_bytes(M, NF) + 16 * 256 + al(nE * 9 * 8);
   size_t b = al(NF * mixed_workspace_per_atom(M)) + mixed_workspace_fixed(M) + al(NF * 16) + al(NF * 4) +
              al(nE * 9 * 8) + 16 * 256;
   return std::max(a, b);
@@ -456,11 +459,10 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
   float *tb[kMaxFitLayers], *hb[kMaxFitLayers];
   for (int l = 0; l < L; ++l) { tb[l] = (float *)w; w += al(NF * M.FW[l] * 4); }
   for (int l = 0; l < L; ++l) { hb[l] = (float *)w; w += al(NF * M.FW[l] * 4); }
-  float *gz[2], *gh[2];
-  gz[0] = (float *)w; w += al(NF * FWM * 4);
-  gz[1] = (float *)w; w += al(NF * FWM * 4);
+  float *gh[2];
   gh[0] = (float *)w; w += al(NF * FWM * 4);
   gh[1] = (float *)w; w += al(NF * FWM * 4);
+  __half *op[2];  // operand tiles of the running and of the next GEMM
   GemmArgs g{};
   EnergyArgs en{};
   int ty[kMaxTypes], n = 0;  // the types present
@@ -475,11 +477,21 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
     ++n;
   }
   g.ntypes = en.ntypes = n;
-  int rc;
+  for (int i = 0; i < 2; ++i) { op[i] = (__half *)w; w += al(gemm_operand_halves(g.mt0[n], FWM) * 2); }
+  int rc, cur = 0;
   for (int l = 0; l < L; ++l) {
-    g.A = l == 0 ? G : hb[l - 1];
+    g.A = l == 0 ? G : nullptr;
+    g.At = l == 0 ? nullptr : op[cur ^ 1];
     g.lda = g.K = l == 0 ? K0 : M.FW[l - 1];
     g.N = M.FW[l];
+    // outputs in FP32: for the energy and the next layer's residual; without a
+    // residual of its own a layer's output is its tanh value
+    bool res = false, need_h = l == L - 1;
+    for (int k = 0; k < n; ++k) {
+      res = res || (l > 0 && M.fdt[ty[k]][l]);
+      need_h = need_h || M.fdt[ty[k]][l + 1 < L ? l + 1 : l];
+    }
+    if (!res) hb[l] = tb[l];
     for (int k = 0; k < n; ++k) {
       const int ti = ty[k];
       GemmType &t = g.t[k];
@@ -490,8 +502,10 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
       t.ep = Epi{};
       t.ep.bias = M.fb[ti][l];
       t.ep.out1 = tb[l];
-      t.ep.out2 = hb[l];
+      t.ep.out2 = res && need_h ? hb[l] : nullptr;
       t.ep.ld = g.N;
+      t.ep.tile = l < L - 1 ? op[cur] : nullptr;
+      t.ep.tscale = M.fit_hsc[ti][l];
       t.ep.mode = EPI_TANH;
       if (l > 0 && M.fdt[ti][l]) {
         t.ep.mode = EPI_TANH_RES;
@@ -500,19 +514,22 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
       }
     }
     if ((rc = launch_gemm_split(g, st))) return rc;
+    cur ^= 1;
   }
-  int cur = 0;
   en.FWl = M.FW[L - 1];
   en.N = D.N;
   for (int k = 0; k < n; ++k) {
     en.t[k].wfin = M.fw[ty[k]][L];
     en.t[k].bfin = M.fb[ty[k]][L];
     en.t[k].dtl = M.fdt[ty[k]][L - 1];
+    en.t[k].gscale = M.fit_gsc[ty[k]][L - 1];
   }
-  if ((rc = launch_fit_energy(en, hb[L - 1], tb[L - 1], Eatom, gz[cur], energy, D.seg, st))) return rc;
+  for (int k = 0; k <= n; ++k) en.mt0[k] = g.mt0[k];
+  if ((rc = launch_fit_energy(en, hb[L - 1], tb[L - 1], Eatom, op[cur], energy, D.seg, st))) return rc;
   for (int l = L - 1; l >= 0; --l) {
     // l >= 1: gH_{l-1} = gZ_l W_l^T (+ gH_l through layer l's residual); l = 0: dE/dG
-    g.A = gz[cur];
+    g.A = nullptr;
+    g.At = op[cur];
     g.lda = g.K = M.FW[l];
     g.N = l == 0 ? K0 : M.FW[l - 1];
     for (int k = 0; k < n; ++k) {
@@ -534,7 +551,8 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
         if (l == L - 1) t.ep.gvec = M.fw[ti][L];
         else t.ep.gmat = gh[cur];
       }
-      t.ep.out1 = gz[cur ^ 1];
+      t.ep.tile = op[cur ^ 1];
+      t.ep.tscale = M.fit_gsc[ti][l - 1];
       t.ep.mode = EPI_GRAD;
       if (l - 1 > 0 && M.fdt[ti][l - 1]) {
         t.ep.mode = EPI_GRAD_RES;
@@ -558,7 +576,7 @@ struct SplitWs {
   int *rcnt;
 };
 static SplitWs split_ws(const DevModel &M, size_t NF, size_t nE, char *base, char *fit_scratch) {
-  const size_t a = al(NF * fp32_ws_per_atom(M)) + 16 * 256 + al(nE * 9 * 8);
+  const size_t a = fp32_ws_bytes(M, NF) + 16 * 256 + al(nE * 9 * 8);
   const size_t need = al(NF * 16) + al(NF * kRowStoreCap * 16) + al(NF * M.ntypes * 4);
   SplitWs s{reinterpret_cast<float4 *>(fit_scratch), nullptr, nullptr};
   if (eval_ws_bytes(M, NF, nE) >= a + need) {

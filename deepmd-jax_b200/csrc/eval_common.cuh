@@ -137,9 +137,21 @@ struct Epi {
   const float *tin;     // per atom tanh values of the layer below, ld
   const float *gvec;    // [Nc] broadcast addend (or NULL)
   const float *gmat;    // per atom addend (or NULL)
-  float *out1, *out2;   // per atom, ld
+  float *out1, *out2;   // per atom, ld (or NULL)
   int ld;
+  __half *tile;         // the next GEMM's operand (GemmArgs::At) times tscale, or NULL
+  float tscale;
 };
+
+// Place of a value (atom row lr of row tile mt, column n) in the operand that one
+// fitting GEMM's epilogue leaves for the next: FP16 tiles of 128 rows x 32
+// columns, [row tile][chunk][hi, lo][column / 8][row][8], nc chunks per row
+// tile; the lo part lies kGemmPart halves after the hi part.
+constexpr int kGemmK = 32;
+constexpr int kGemmPart = 128 * kGemmK;
+__host__ __device__ __forceinline__ size_t gemm_operand_at(int nc, int mt, int lr, int n) {
+  return ((size_t)mt * nc + n / kGemmK) * (2 * kGemmPart) + ((n >> 3) & 3) * 1024 + lr * 8 + (n & 7);
+}
 
 // One centre type's part of a fitting GEMM over the atoms of every type
 // (gemm_split.cu): rows, weights, operand scales and epilogue.
@@ -152,7 +164,8 @@ struct GemmType {
   Epi ep;
 };
 struct GemmArgs {
-  const float *A;       // per atom, lda
+  const float *A;       // per atom, lda; or, where At is set,
+  const __half *At;     // hi and lo parts in tiles of 128 rows x 32 of K (gemm_tile_at)
   int lda, K, N, ntypes;
   int mt0[kMaxTypes + 1];  // first 128-row tile of each type
   GemmType t[kMaxTypes];
@@ -163,10 +176,12 @@ struct EnergyType {
   int Mrows;
   RowMap rm;
   const float *wfin, *bfin, *dtl;
+  float gscale;  // of the gate written as the adjoint GEMM's operand
 };
 struct EnergyArgs {
   int ntypes, FWl, N;
-  int b0[kMaxTypes + 1];  // first block of each type
+  int b0[kMaxTypes + 1];   // first block of each type
+  int mt0[kMaxTypes + 1];  // first 128-row tile of each type
   EnergyType t[kMaxTypes];
 };
 

@@ -446,7 +446,7 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
 // reduced in FP64, one atomic per run of one energy row.
 __global__ void __launch_bounds__(256) k_fit_energy(EnergyArgs g, const float *__restrict__ H,
                                                     const float *__restrict__ tl, float *__restrict__ Eatom,
-                                                    float *__restrict__ gZ, double *__restrict__ energy,
+                                                    __half *__restrict__ gZ, double *__restrict__ energy,
                                                     const int32_t *__restrict__ seg) {
   __shared__ double es[8];
   __shared__ int fs[8];
@@ -460,10 +460,33 @@ __global__ void __launch_bounds__(256) k_fit_energy(EnergyArgs g, const float *_
   if (r < et.Mrows) {
     const size_t at = et.rm.atom(r);
     float s = 0.f;
-    for (int n = lane; n < g.FWl; n += 32) {
-      const float w = et.wfin[n], t = tl[at * g.FWl + n];
-      s = fmaf(H[at * g.FWl + n], w, s);
-      gZ[at * g.FWl + n] = w * (et.dtl ? et.dtl[n] : 1.f) * (1.f - t * t);
+    const int nc = (g.FWl + kGemmK - 1) / kGemmK, mt = g.mt0[ti] + r / 128, lr = r & 127;
+    const float *h_ = H + at * g.FWl, *t_ = tl + at * g.FWl;
+    for (int n = 4 * lane; n < (g.FWl + 15) / 16 * 16; n += 128) {  // whole K = 16 steps
+      __align__(16) float h[4] = {0.f, 0.f, 0.f, 0.f}, t[4] = {1.f, 1.f, 1.f, 1.f}, w[4] = {0.f, 0.f, 0.f, 0.f};
+      if ((g.FWl & 3) == 0 && n < g.FWl) {
+        *reinterpret_cast<float4 *>(h) = *reinterpret_cast<const float4 *>(h_ + n);
+        *reinterpret_cast<float4 *>(t) = *reinterpret_cast<const float4 *>(t_ + n);
+      }
+      __align__(8) __half hi[4], lo[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        float gz = 0.f;
+        if (n + e < g.FWl) {
+          if ((g.FWl & 3) != 0) {
+            h[e] = h_[n + e];
+            t[e] = t_[n + e];
+          }
+          w[e] = et.wfin[n + e];
+          s = fmaf(h[e], w[e], s);
+          gz = w[e] * (et.dtl ? et.dtl[n + e] : 1.f) * (1.f - t[e] * t[e]) * et.gscale;
+        }
+        hi[e] = __float2half_rn(gz);
+        lo[e] = __float2half_rn(gz - __half2float(hi[e]));
+      }
+      __half *o = gZ + gemm_operand_at(nc, mt, lr, n);
+      *reinterpret_cast<uint2 *>(o) = *reinterpret_cast<const uint2 *>(hi);
+      *reinterpret_cast<uint2 *>(o + kGemmPart) = *reinterpret_cast<const uint2 *>(lo);
     }
     s = warp_sum(s) + et.bfin[0];
     if (lane == 0) {
@@ -558,7 +581,7 @@ template int launch_embed_bwd_cmp<64>(const DevModel &, const SysDesc &, int, co
                                       const float *, const int32_t *, const float *, const float *, float4 *, double *,
                                       cudaStream_t);
 
-int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, float *gZ, double *energy,
+int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, __half *gZ, double *energy,
                       const int32_t *seg, cudaStream_t st) {
   const int nb = g.b0[g.ntypes];
   if (nb == 0) return DPB_OK;

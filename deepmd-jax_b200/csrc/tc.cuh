@@ -203,6 +203,9 @@ __device__ __forceinline__ void ldmatrix_x2_trans(uint32_t &r0, uint32_t &r1, co
 }
 
 // Asynchronous 16-byte global -> shared copies (no register round trip).
+__device__ __forceinline__ void cp_async4(void *smem, const void *gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem)), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_async16(void *dst_smem, const void *src_gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst_smem)), "l"(src_gmem) : "memory");
 }
