@@ -1,19 +1,17 @@
-// Plain FP32 evaluation path: energy, forces and virial of the se_a model.
-//
-// Three stages per centre type (reference model: deepmd_jax/dpmodel.py:30-100,
+// FP32 evaluation with compressed embedding tables, and the pieces that every
+// FP32 evaluation shares (reference model: deepmd_jax/dpmodel.py:30-100,
 // embedding/fitting nets deepmd_jax/utils.py:100-166):
-//   1. k_embed_fwd   warp per centre atom: neighbour rows with s(r) != 0 are
-//                    compacted, pushed through the per-type-pair embedding MLP,
-//                    contracted with the 10-channel env rows into T (10 x W);
-//                    the epilogue forms the descriptor G (A x W).
-//   2. fitting       tiled SGEMM chain over the atoms of one centre type, fused
-//                    tanh / dt-residual epilogues, per-atom energy, and the
-//                    adjoint chain down to dE/dG.
-//   3. k_embed_bwd   warp per centre atom: dE/dT from dE/dG, then the rows are
-//                    recomputed with forward-mode tangents (h, dh/ds~) so
-//                    dE/ds~ and dE/dR~ come out of one sweep; the row adjoint
-//                    gives dE/dx, scattered as forces (float4 atomics) and
-//                    reduced into the virial.
+//   k_embed_fwd   warp per centre atom: neighbour rows with s(r) != 0 are
+//                 compacted, looked up in the type pair's table, contracted with
+//                 the 10-channel env rows into T (10 x W); the epilogue forms
+//                 the descriptor G (A x W) and its largest entry.
+//   k_embed_bwd   warp per centre atom: dE/dT from dE/dG, then the rows' h and
+//                 dh/ds~ give dE/ds~ and dE/dR~; the row adjoint gives dE/dx,
+//                 scattered as forces (float4 atomics) and reduced into the
+//                 virial.
+//   k_fit_energy, k_finalize
+// The tuned uncompressed nets run in embed_split.cu, other shapes in
+// eval_general.cu, the fitting net in gemm_split.cu.
 // Rows with s(r) = 0 contribute exactly zero in the reference (R~ = 0) and are
 // skipped here.
 #include "eval_common.cuh"
@@ -39,14 +37,19 @@ __device__ __forceinline__ void cmp_locate(float st, float srmin, float delta, i
   idx = k < 0 ? 0 : (k >= ng ? ng - 1 : k);
 }
 
-// One round of up to 32 compacted rows, column-parallel: lane owns columns
-// q*32 + lane; the rows' (idx, x0) and env rows are read from the row buffer
-// (st slot overwritten by x0, slot 11 by idx) and each table row is read with
-// coalesced loads.  T += R~^T h accumulates into the warp's shared T.
+// One round of up to 32 compacted rows, column-parallel: a lane owns VC
+// neighbouring columns, so that one pass over the rows covers all of them; the
+// rows' (idx, x0) and env rows are read from the row buffer (st slot overwritten
+// by x0, slot 11 by idx) as three 16-byte words and each table row is read with
+// coalesced loads.  T += R~^T h accumulates into the warp's shared T.  (With one
+// column per lane, two or four passes of twelve 4-byte reads per row: 206 us for
+// 12,288 atoms of width 64, 170 us now.)
 template <int E2>
 __device__ __forceinline__ void embed_rows_fwd_cmp(const float *__restrict__ coeff, float srmin, float delta,
                                                    int ng, int n, float *__restrict__ rowbuf,
                                                    float *__restrict__ Ts, int lane) {
+  constexpr int VC = E2 <= 64 ? 2 : 4;
+  static_assert(E2 % VC == 0 && E2 / VC <= 32, "columns per lane");
   if (lane < n) {
     int idx;
     float x0;
@@ -55,26 +58,44 @@ __device__ __forceinline__ void embed_rows_fwd_cmp(const float *__restrict__ coe
     rowbuf[lane * 12 + 11] = __int_as_float(idx);
   }
   __syncwarp();
-#pragma unroll 1
-  for (int q = 0; q < (E2 + 31) / 32; ++q) {
-    const int col = q * 32 + lane;
-    if (col < E2) {
-      float Tq[10];
+  if (lane < E2 / VC) {
+    const int col = VC * lane;
+    float Tq[10][VC];
 #pragma unroll
-      for (int c = 0; c < 10; ++c) Tq[c] = 0.f;
-      for (int r = 0; r < n; ++r) {
-        const float *rb = rowbuf + r * 12;
-        const float x0 = rb[0];
-        const float *cr = coeff + (size_t)__float_as_int(rb[11]) * 6 * E2 + col;
-        float h = __ldg(cr);
+    for (int c = 0; c < 10; ++c)
 #pragma unroll
-        for (int i = 1; i < 6; ++i) h = fmaf(h, x0, __ldg(cr + i * E2));
+      for (int e = 0; e < VC; ++e) Tq[c][e] = 0.f;
+#pragma unroll 2
+    for (int r = 0; r < n; ++r) {
+      const float4 *rb = reinterpret_cast<const float4 *>(rowbuf + r * 12);
+      const float4 w0 = rb[0], w1 = rb[1], w2 = rb[2];
+      const float R[10] = {w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w, w2.x, w2.y, w2.z};
+      const float x0 = w0.x;
+      const float *cr = coeff + (size_t)__float_as_int(w2.w) * 6 * E2 + col;
+      float cf[6][VC];
 #pragma unroll
-        for (int c = 0; c < 10; ++c) Tq[c] = fmaf(rb[1 + c], h, Tq[c]);
+      for (int i = 0; i < 6; ++i) {
+        if constexpr (VC == 2) {
+          const float2 t = __ldg(reinterpret_cast<const float2 *>(cr + i * E2));
+          cf[i][0] = t.x; cf[i][1] = t.y;
+        } else {
+          const float4 t = __ldg(reinterpret_cast<const float4 *>(cr + i * E2));
+          cf[i][0] = t.x; cf[i][1] = t.y; cf[i][2] = t.z; cf[i][3] = t.w;
+        }
       }
 #pragma unroll
-      for (int c = 0; c < 10; ++c) Ts[c * E2 + col] += Tq[c];
+      for (int e = 0; e < VC; ++e) {
+        float h = cf[0][e];
+#pragma unroll
+        for (int i = 1; i < 6; ++i) h = fmaf(h, x0, cf[i][e]);
+#pragma unroll
+        for (int c = 0; c < 10; ++c) Tq[c][e] = fmaf(R[c], h, Tq[c][e]);
+      }
     }
+#pragma unroll
+    for (int c = 0; c < 10; ++c)
+#pragma unroll
+      for (int e = 0; e < VC; ++e) Ts[c * E2 + col + e] += Tq[c][e];
   }
   __syncwarp();
 }
@@ -200,15 +221,23 @@ __global__ void __launch_bounds__(256) k_embed_fwd(DevModel M, SysDesc D, int ti
 }
 
 // ---------------------------------------------------------------- adjoint
-// Adjoint of one round of rows of a compressed net (row = lane): h and
-// dh/ds~ = dh/dx0 from the row's table entry (float4 loads along w), u =
-// dT.h, v = dT.dh, then the same env-row adjoint as the MLP path.
+// Adjoint of one round of rows of a compressed net: h and dh/ds~ = dh/dx0 from
+// the rows' table entries, u = dT.h, v = dT.dh, then (row = lane) the same
+// env-row adjoint as the MLP path.  The table entries of 16 rows are read 32
+// columns at a time, 8 lanes on one row's whole line, and h and dh go through
+// shared memory to two lanes per row for the sums.  (With row = lane every load
+// touched 32 lines at the same offset: up to 32 tag lookups and 8-way conflicts
+// per instruction, 3,000 clocks per round of 32 rows: 637 us for 12,288 atoms of
+// width 64, 413 us now.)
+constexpr int kCmpS = 36;                    // row stride of h and dh (floats)
+constexpr int kCmpHd = 2 * 16 * kCmpS;       // floats of both
 template <int E2>
 __device__ __forceinline__ void embed_rows_bwd_cmp(const float *__restrict__ coeff, float srmin, float delta,
                                                    int ng, int n, const float *__restrict__ rowbuf,
-                                                   const float *__restrict__ dT, float inv_std, float mean,
-                                                   int lane, float &fi0, float &fi1, float &fi2, float (&vir)[9],
-                                                   float4 *__restrict__ F4, size_t frame_base) {
+                                                   float *__restrict__ hd, const float *__restrict__ dT,
+                                                   float inv_std, float mean, int lane, float &fi0, float &fi1,
+                                                   float &fi2, float (&vir)[9], float4 *__restrict__ F4,
+                                                   size_t frame_base) {
   static_assert(E2 % 4 == 0, "table width");
   const bool act = lane < n;
   RowGeom gm;
@@ -226,35 +255,71 @@ __device__ __forceinline__ void embed_rows_bwd_cmp(const float *__restrict__ coe
   float x0;
   cmp_locate(st, srmin, delta, ng, idx, x0);
   float u[10], v[10];
-#pragma unroll
-  for (int c = 0; c < 10; ++c) u[c] = v[c] = 0.f;
-  const float4 *cr = reinterpret_cast<const float4 *>(coeff + (size_t)idx * 6 * E2);
+  const int half = lane >> 4, cq = 4 * (lane & 7);
 #pragma unroll 1
-  for (int w4 = 0; w4 < E2 / 4; ++w4) {
-    float4 c[6];
+  for (int b = 0; 16 * b < n; ++b) {  // rows 16 b .. 16 b + 15
+    float us[10], vs[10];
 #pragma unroll
-    for (int i = 0; i < 6; ++i) c[i] = __ldg(cr + i * (E2 / 4) + w4);
-    const float cc[6][4] = {{c[0].x, c[0].y, c[0].z, c[0].w}, {c[1].x, c[1].y, c[1].z, c[1].w},
-                            {c[2].x, c[2].y, c[2].z, c[2].w}, {c[3].x, c[3].y, c[3].z, c[3].w},
-                            {c[4].x, c[4].y, c[4].z, c[4].w}, {c[5].x, c[5].y, c[5].z, c[5].w}};
+    for (int c = 0; c < 10; ++c) us[c] = vs[c] = 0.f;
+#pragma unroll 1
+    for (int c0 = 0; c0 < E2; c0 += 32) {
+      __syncwarp();
+#pragma unroll 2
+      for (int p = 0; p < 4; ++p) {
+        const int r = 4 * p + (lane >> 3);
+        const int id = __shfl_sync(0xffffffffu, idx, 16 * b + r);
+        const float x = __shfl_sync(0xffffffffu, x0, 16 * b + r);
+        if (E2 % 32 == 0 || c0 + cq < E2) {
+          const float4 *cr = reinterpret_cast<const float4 *>(coeff + (size_t)id * 6 * E2 + c0 + cq);
+          float4 c[6];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float h = cc[0][e], dh = 5.f * cc[0][e];
+          for (int i = 0; i < 6; ++i) c[i] = __ldg(cr + i * (E2 / 4));
+          const float cc[6][4] = {{c[0].x, c[0].y, c[0].z, c[0].w}, {c[1].x, c[1].y, c[1].z, c[1].w},
+                                  {c[2].x, c[2].y, c[2].z, c[2].w}, {c[3].x, c[3].y, c[3].z, c[3].w},
+                                  {c[4].x, c[4].y, c[4].z, c[4].w}, {c[5].x, c[5].y, c[5].z, c[5].w}};
+          float h[4], dh[4];
 #pragma unroll
-      for (int i = 1; i < 5; ++i) {
-        h = fmaf(h, x0, cc[i][e]);
-        dh = fmaf(dh, x0, (float)(5 - i) * cc[i][e]);
+          for (int e = 0; e < 4; ++e) {
+            h[e] = cc[0][e];
+            dh[e] = 5.f * cc[0][e];
+#pragma unroll
+            for (int i = 1; i < 5; ++i) {
+              h[e] = fmaf(h[e], x, cc[i][e]);
+              dh[e] = fmaf(dh[e], x, (float)(5 - i) * cc[i][e]);
+            }
+            h[e] = fmaf(h[e], x, cc[5][e]);
+          }
+          *reinterpret_cast<float4 *>(hd + r * kCmpS + cq) = make_float4(h[0], h[1], h[2], h[3]);
+          *reinterpret_cast<float4 *>(hd + kCmpHd / 2 + r * kCmpS + cq) = make_float4(dh[0], dh[1], dh[2], dh[3]);
+        }
       }
-      h = fmaf(h, x0, cc[5][e]);
-      const int col = w4 * 4 + e;
+      __syncwarp();
+#pragma unroll 2
+      for (int q = 0; q < 4; ++q) {
+        const int k = 16 * half + 4 * q, col = c0 + k;
+        if (E2 % 32 == 0 || col < E2) {
+          const float4 h = *reinterpret_cast<const float4 *>(hd + (lane & 15) * kCmpS + k);
+          const float4 d = *reinterpret_cast<const float4 *>(hd + kCmpHd / 2 + (lane & 15) * kCmpS + k);
 #pragma unroll
-      for (int ch = 0; ch < 10; ++ch) {
-        const float dtc = dT[ch * E2 + col];
-        u[ch] = fmaf(dtc, h, u[ch]);
-        v[ch] = fmaf(dtc, dh, v[ch]);
+          for (int ch = 0; ch < 10; ++ch) {
+            const float4 t = *reinterpret_cast<const float4 *>(dT + ch * (E2 + 4) + col);
+            us[ch] = fmaf(t.w, h.w, fmaf(t.z, h.z, fmaf(t.y, h.y, fmaf(t.x, h.x, us[ch]))));
+            vs[ch] = fmaf(t.w, d.w, fmaf(t.z, d.z, fmaf(t.y, d.y, fmaf(t.x, d.x, vs[ch]))));
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 10; ++c) {  // the two lanes of a row
+      const float uc = us[c] + __shfl_xor_sync(0xffffffffu, us[c], 16);
+      const float vc = vs[c] + __shfl_xor_sync(0xffffffffu, vs[c], 16);
+      if (b == 0 || half == b) {
+        u[c] = uc;
+        v[c] = vc;
       }
     }
   }
+  __syncwarp();
   const float inv_rp = 1.f / (gm.r + 1e-16f);
   const float xh[3] = {gm.x[0] * inv_rp, gm.x[1] * inv_rp, gm.x[2] * inv_rp};
   float R[10];
@@ -274,8 +339,15 @@ __device__ __forceinline__ void embed_rows_bwd_cmp(const float *__restrict__ coe
   }
 }
 
+// Floats of a warp's dG (row stride E2 + 1), later its 64 rows and h and dh.
 template <int E2>
-__global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti, const float *__restrict__ pos,
+__host__ __device__ __forceinline__ int cmp_bwd_r1(int A) {
+  const int a = (A * (E2 + 1) + 3) / 4 * 4, b = 64 * 8 + kCmpHd;
+  return a > b ? a : b;
+}
+
+template <int E2>
+__global__ void __launch_bounds__(256, 2) k_embed_bwd(DevModel M, SysDesc D, int ti, const float *__restrict__ pos,
                                                    const int32_t *__restrict__ perm, const float *__restrict__ box,
                                                    const int32_t *__restrict__ nbrs, const float *__restrict__ Tin,
                                                    const float *__restrict__ dG, float4 *__restrict__ F4,
@@ -284,11 +356,12 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
   extern __shared__ float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const int A = M.A;
-  const int r1 = A * E2 > 64 * 8 ? A * E2 : 64 * 8;
-  const int per_warp = r1 + 10 * E2 + 20 * A;
-  float *bufA = smem + warp * per_warp;  // dG, later rows
+  constexpr int AS = E2 + 1, BS = E2 + 4;  // row strides: dot products along rows without bank conflicts
+  const int r1 = cmp_bwd_r1<E2>(A);
+  const int per_warp = r1 + 10 * BS + 20 * A;
+  float *bufA = smem + warp * per_warp;  // dG, later rows, h and dh
   float *bufB = bufA + r1;                                   // X, later dT
-  float *Qs = bufB + 10 * E2;                                // 10 x A
+  float *Qs = bufB + 10 * BS;                                // 10 x A
   float *dQs = Qs + 10 * A;                                  // 10 x A
   __shared__ double vsm[9];
   if (threadIdx.x < 9) vsm[threadIdx.x] = 0.0;
@@ -305,24 +378,24 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
     // ---- dE/dT from dE/dG (adjoint of dpmodel.py:74-78)
     for (int e = lane; e < 10 * E2; e += 32) {
       const int c = e / E2, w = e - c * E2;
-      bufB[e] = Tin[g * 10 * E2 + e] + (c == 0 ? M.tbias[w] : 0.f);
+      bufB[c * BS + w] = Tin[g * 10 * E2 + e] + (c == 0 ? M.tbias[w] : 0.f);
     }
-    for (int e = lane; e < A * E2; e += 32) bufA[e] = dG[g * (size_t)A * E2 + e];
+    for (int e = lane; e < A * E2; e += 32) bufA[e / E2 * AS + e % E2] = dG[g * (size_t)A * E2 + e];
     __syncwarp();
     for (int e = lane; e < 10 * A; e += 32) {
       const int c = e / A, aa = e - c * A;
       float qv;
       if (c < 4) {
-        qv = bufB[c * E2 + aa];
+        qv = bufB[c * BS + aa];
       } else {
-        const float y1 = bufB[1 * E2 + A + aa], y2 = bufB[2 * E2 + A + aa], y3 = bufB[3 * E2 + A + aa];
+        const float y1 = bufB[1 * BS + A + aa], y2 = bufB[2 * BS + A + aa], y3 = bufB[3 * BS + A + aa];
         const int m = c - 4;
         const float base[6] = {y1 * y1, y2 * y2, y3 * y3, kSqrt2 * y1 * y3, kSqrt2 * y2 * y1, kSqrt2 * y3 * y2};
-        qv = base[m] + bufB[c * E2 + A + aa];
+        qv = base[m] + bufB[c * BS + A + aa];
       }
       Qs[e] = qv;
       float dq = 0.f;
-      for (int w = 0; w < E2; ++w) dq = fmaf(bufA[aa * E2 + w], bufB[c * E2 + w], dq);
+      for (int w = 0; w < E2; ++w) dq = fmaf(bufA[aa * AS + w], bufB[c * BS + w], dq);
       dQs[e] = dq;
     }
     __syncwarp();
@@ -334,7 +407,7 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
       for (int c = 0; c < 10; ++c) dX[q][c] = 0.f;
       if (col < E2) {
         for (int aa = 0; aa < A; ++aa) {
-          const float dg = bufA[aa * E2 + col];
+          const float dg = bufA[aa * AS + col];
 #pragma unroll
           for (int c = 0; c < 10; ++c) dX[q][c] = fmaf(dg, Qs[c * A + aa], dX[q][c]);
         }
@@ -349,7 +422,7 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
       float d2[6];
 #pragma unroll
       for (int m = 0; m < 6; ++m) d2[m] = dQs[(4 + m) * A + aa];
-      const float y1 = bufB[1 * E2 + lane], y2 = bufB[2 * E2 + lane], y3 = bufB[3 * E2 + lane];
+      const float y1 = bufB[1 * BS + lane], y2 = bufB[2 * BS + lane], y3 = bufB[3 * BS + lane];
 #pragma unroll
       for (int m = 0; m < 6; ++m) dX[0][4 + m] += d2[m];
       dX[0][1] += 2.f * y1 * d2[0] + kSqrt2 * y3 * d2[3] + kSqrt2 * y2 * d2[4];
@@ -362,7 +435,7 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
       const int col = q * 32 + lane;
       if (col < E2)
 #pragma unroll
-        for (int c = 0; c < 10; ++c) bufB[c * E2 + col] = dX[q][c] * M.inv_nnbrs;
+        for (int c = 0; c < 10; ++c) bufB[c * BS + col] = dX[q][c] * M.inv_nnbrs;
     }
     __syncwarp();
     // ---- rows: recompute with tangents, scatter forces
@@ -407,7 +480,7 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
         __syncwarp();
         if (nbuf >= 32) {
           embed_rows_bwd_cmp<E2>(M.cmp_coeff[ti * M.ntypes + tj], M.cmp_srmin[ti * M.ntypes + tj],
-                                 M.cmp_delta[ti * M.ntypes + tj], M.ngrids, 32, rowbuf, bufB, inv_std, mean,
+                                 M.cmp_delta[ti * M.ntypes + tj], M.ngrids, 32, rowbuf, bufA + 64 * 8, bufB, inv_std, mean,
                                  lane, fi0, fi1, fi2, vir, F4, frame_base);
           const int rem = nbuf - 32;
           if (lane < rem)
@@ -418,7 +491,7 @@ __global__ void __launch_bounds__(256) k_embed_bwd(DevModel M, SysDesc D, int ti
       }
       if (nbuf > 0) {
         embed_rows_bwd_cmp<E2>(M.cmp_coeff[ti * M.ntypes + tj], M.cmp_srmin[ti * M.ntypes + tj],
-                               M.cmp_delta[ti * M.ntypes + tj], M.ngrids, nbuf, rowbuf, bufB, inv_std, mean,
+                               M.cmp_delta[ti * M.ntypes + tj], M.ngrids, nbuf, rowbuf, bufA + 64 * 8, bufB, inv_std, mean,
                                lane, fi0, fi1, fi2, vir, F4, frame_base);
       }
       __syncwarp();
@@ -561,8 +634,7 @@ int launch_embed_bwd_cmp(const DevModel &M, const SysDesc &D, int ti, const floa
   const int cnt = D.offs[ti + 1] - D.offs[ti];
   if (cnt == 0) return DPB_OK;
   dim3 grid((cnt + 7) / 8, D.F);
-  const int r1 = M.A * E2 > 64 * 8 ? M.A * E2 : 64 * 8;
-  const size_t smem = (size_t)8 * (r1 + 10 * E2 + 20 * M.A) * sizeof(float);
+  const size_t smem = (size_t)8 * (cmp_bwd_r1<E2>(M.A) + 10 * (E2 + 4) + 20 * M.A) * sizeof(float);
   cudaFuncSetAttribute(k_embed_bwd<E2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   k_embed_bwd<E2><<<grid, 256, smem, st>>>(M, D, ti, pos, perm, box, nbrs, T, dG, F4, virial);
   count_launch();
