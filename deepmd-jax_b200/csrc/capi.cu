@@ -85,6 +85,8 @@ int launch_embed_bwd_gen(const DevModel &, const SysDesc &, int, const float *, 
                          const int32_t *, const float *, const float *, float4 *, double *, cudaStream_t);
 int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, __half *gZ, double *energy,
                       const int32_t *seg, cudaStream_t st);
+int launch_eval_begin(size_t NF, float4 *F4, size_t nE, double *energy, double *virial, int *err, cudaStream_t st);
+int *mixed_err(const DevModel &M, size_t NF, void *ws);
 int launch_finalize(int, int, const float4 *, float *, const float *, const int32_t *, float *, double *, int,
                     const float *, const int32_t *, uint32_t *, cudaStream_t);
 // mixed path (mixed.cu)
@@ -666,13 +668,12 @@ int dpb::eval_impl(const dpb_model *m, int precision, const float *pos, const in
   double *vir = virial;
   double *vscratch = (double *)w; w += al(nE * 9 * 8);
   if (!vir) vir = vscratch;
-  DPB_CUDA_TRY(cudaMemsetAsync(F4, 0, NF * 16, st));
-  DPB_CUDA_TRY(cudaMemsetAsync(energy, 0, nE * 8, st));
-  DPB_CUDA_TRY(cudaMemsetAsync(vir, 0, nE * 72, st));
+  if (precision == DPB_PREC_MIXED && !mixed_supported(M)) return DPB_ERR_UNSUPPORTED;
+  rc = launch_eval_begin(NF, F4, nE, energy, vir, precision == DPB_PREC_MIXED ? mixed_err(M, NF, w) : nullptr, st);
+  if (rc) return rc;
   if (precision == DPB_PREC_FP32) {
     rc = eval_fp32(M, D, pos, perm, box, nbrs, energy, F4, Eatom, vir, (char *)workspace, w, nE, st);
   } else {
-    if (!mixed_supported(M)) return DPB_ERR_UNSUPPORTED;
     rc = mixed_eval(M, D, pos, perm, box, nbrs, energy, Eatom, F4, vir, w, st, m->dT_warps, m->fit_deep != 0);
   }
   if (rc) return rc;

@@ -2128,6 +2128,9 @@ int mixed_tune_dT(const DevModel &M, size_t NF, void *ws, cudaStream_t st, int *
   return rc;
 }
 
+// The error word of mixed_eval's workspace, zero on its entry.
+int *mixed_err(const DevModel &M, size_t NF, void *ws) { return mixed_ws(M, NF, ws).err; }
+
 int mixed_eval(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm, const float *box,
                const int32_t *nbrs, double *energy, float *Eatom, float4 *F4, double *virial, void *ws,
                cudaStream_t st, int dT_warps, bool fit_deep) {
@@ -2137,7 +2140,6 @@ int mixed_eval(const DevModel &M, const SysDesc &D, const float *pos, const int3
   float *T = mw.T, *dG = mw.dG, *scratch = mw.scratch;
   __half *Gb = mw.Gb;
   float4 *posS = mw.posS;
-  DPB_CUDA_TRY(cudaMemsetAsync(err, 0, 4, st));
   if (M.ngrids > 0 || !M.emb_tuned)
     return mixed_eval_compressed(M, D, pos, perm, box, nbrs, energy, Eatom, F4, virial, T, Gb, dG, scratch, err,
                                  fit_deep, st);
