@@ -401,12 +401,18 @@ static int fit_width_max(const DevModel &M) {
   return w;
 }
 
+// A dt residual needs equal widths (utils.py:158-163).
+static bool fit_res_width(const DevModel &M, int l) { return l > 0 && M.FW[l] == M.FW[l - 1]; }
+
 static size_t fp32_ws_bytes(const DevModel &M, size_t NF) {
-  int hid = 0;
-  for (int l = 0; l < M.nfit; ++l) hid += M.FW[l];
-  const size_t fw = fit_width_max(M), fwp = (fw + 31) / 32 * 32;  // operand tiles are 128 rows x 32 columns
-  return al(NF * ((10 * M.E2 + M.A * M.E2 + 2 * hid + 2 * fw + 2 * fwp + 1) * 4 + 16)) +
-         al((size_t)128 * M.ntypes * 2 * fwp * 4);
+  // per layer the tanh values and, where a residual is possible, the outputs
+  size_t hid = 0;
+  for (int l = 0; l < M.nfit; ++l) hid += M.FW[l] * (fit_res_width(M, l) ? 2 : 1);
+  // operand tiles of 128 rows x 32 columns: one set beside, one in G where it fits
+  const size_t fw = fit_width_max(M), op = al((NF + (size_t)127 * M.ntypes) * ((fw + 31) / 32 * 32) * 4);
+  const size_t gh = M.nfit > 2 ? 2 * fw : 0;
+  return al(NF * ((10 * M.E2 + M.A * M.E2 + hid + gh + 1) * 4 + 16)) + op +
+         (M.nfit == 1 || op <= NF * (size_t)(M.A * M.E2) * 4 ? 0 : op);
 }
 
 // Workspace of NF atoms with nE energy / virial rows.
@@ -460,11 +466,15 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
   const int E2 = M.E2, A = M.A, K0 = A * E2, L = M.nfit, FWM = fit_width_max(M);
   float *tb[kMaxFitLayers], *hb[kMaxFitLayers];
   for (int l = 0; l < L; ++l) { tb[l] = (float *)w; w += al(NF * M.FW[l] * 4); }
-  for (int l = 0; l < L; ++l) { hb[l] = (float *)w; w += al(NF * M.FW[l] * 4); }
-  float *gh[2];
-  gh[0] = (float *)w; w += al(NF * FWM * 4);
-  gh[1] = (float *)w; w += al(NF * FWM * 4);
-  __half *op[2];  // operand tiles of the running and of the next GEMM
+  for (int l = 0; l < L; ++l) {
+    hb[l] = tb[l];  // without a residual a layer's output is its tanh value
+    if (fit_res_width(M, l)) { hb[l] = (float *)w; w += al(NF * M.FW[l] * 4); }
+  }
+  float *gh[2] = {nullptr, nullptr};  // residual adjoints of the layers between the first and the last
+  for (int i = 0; i < 2 && L > 2; ++i) { gh[i] = (float *)w; w += al(NF * FWM * 4); }
+  // operand tiles: layer l's output, later its gate, in op[l & 1].  op[1] is G's
+  // space, which is free between layer 0 (writes op[0]) and dE/dG (reads op[0])
+  __half *op[2];
   GemmArgs g{};
   EnergyArgs en{};
   int ty[kMaxTypes], n = 0;  // the types present
@@ -479,18 +489,19 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
     ++n;
   }
   g.ntypes = en.ntypes = n;
-  for (int i = 0; i < 2; ++i) { op[i] = (__half *)w; w += al(gemm_operand_halves(g.mt0[n], FWM) * 2); }
+  const size_t opb = al(gemm_operand_halves(g.mt0[n], FWM) * 2);
+  op[0] = (__half *)w; w += opb;
+  op[1] = opb <= NF * (size_t)K0 * 4 ? (__half *)G : (__half *)w;
   int rc, cur = 0;
   for (int l = 0; l < L; ++l) {
     g.A = l == 0 ? G : nullptr;
-    g.At = l == 0 ? nullptr : op[cur ^ 1];
+    g.At = l == 0 ? nullptr : op[(l - 1) & 1];
     g.lda = g.K = l == 0 ? K0 : M.FW[l - 1];
     g.N = M.FW[l];
-    // outputs in FP32: for the energy and the next layer's residual; without a
-    // residual of its own a layer's output is its tanh value
+    // outputs in FP32: for the energy and the next layer's residual
     bool res = false, need_h = l == L - 1;
     for (int k = 0; k < n; ++k) {
-      res = res || (l > 0 && M.fdt[ty[k]][l]);
+      res = res || (fit_res_width(M, l) && M.fdt[ty[k]][l]);
       need_h = need_h || M.fdt[ty[k]][l + 1 < L ? l + 1 : l];
     }
     if (!res) hb[l] = tb[l];
@@ -506,17 +517,16 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
       t.ep.out1 = tb[l];
       t.ep.out2 = res && need_h ? hb[l] : nullptr;
       t.ep.ld = g.N;
-      t.ep.tile = l < L - 1 ? op[cur] : nullptr;
+      t.ep.tile = l < L - 1 ? op[l & 1] : nullptr;
       t.ep.tscale = M.fit_hsc[ti][l];
       t.ep.mode = EPI_TANH;
-      if (l > 0 && M.fdt[ti][l]) {
+      if (fit_res_width(M, l) && M.fdt[ti][l]) {
         t.ep.mode = EPI_TANH_RES;
         t.ep.dt = M.fdt[ti][l];
         t.ep.hprev = hb[l - 1];
       }
     }
     if ((rc = launch_gemm_split(g, st))) return rc;
-    cur ^= 1;
   }
   en.FWl = M.FW[L - 1];
   en.N = D.N;
@@ -527,11 +537,11 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
     en.t[k].gscale = M.fit_gsc[ty[k]][L - 1];
   }
   for (int k = 0; k <= n; ++k) en.mt0[k] = g.mt0[k];
-  if ((rc = launch_fit_energy(en, hb[L - 1], tb[L - 1], Eatom, op[cur], energy, D.seg, st))) return rc;
+  if ((rc = launch_fit_energy(en, hb[L - 1], tb[L - 1], Eatom, op[(L - 1) & 1], energy, D.seg, st))) return rc;
   for (int l = L - 1; l >= 0; --l) {
     // l >= 1: gH_{l-1} = gZ_l W_l^T (+ gH_l through layer l's residual); l = 0: dE/dG
     g.A = nullptr;
-    g.At = op[cur];
+    g.At = op[l & 1];
     g.lda = g.K = M.FW[l];
     g.N = l == 0 ? K0 : M.FW[l - 1];
     for (int k = 0; k < n; ++k) {
@@ -549,14 +559,14 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
         continue;
       }
       t.ep.tin = tb[l - 1];
-      if (M.fdt[ti][l]) {
+      if (fit_res_width(M, l) && M.fdt[ti][l]) {
         if (l == L - 1) t.ep.gvec = M.fw[ti][L];
         else t.ep.gmat = gh[cur];
       }
-      t.ep.tile = op[cur ^ 1];
+      t.ep.tile = op[(l - 1) & 1];
       t.ep.tscale = M.fit_gsc[ti][l - 1];
       t.ep.mode = EPI_GRAD;
-      if (l - 1 > 0 && M.fdt[ti][l - 1]) {
+      if (fit_res_width(M, l - 1) && M.fdt[ti][l - 1]) {
         t.ep.mode = EPI_GRAD_RES;
         t.ep.dt = M.fdt[ti][l - 1];
         t.ep.out2 = gh[cur ^ 1];

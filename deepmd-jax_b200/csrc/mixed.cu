@@ -1,4 +1,4 @@
-// Mixed-precision (BF16 tensor-core) evaluation path.
+// Mixed-precision (FP16 tensor-core) evaluation path.
 #include "rows.cuh"
 
 namespace dpb {
@@ -110,7 +110,7 @@ struct HalfSplit {
   static_assert(S1 % 8 == 0 && S2 % 8 == 0 && H0LO1 % 2 == 0 && A0C % 8 == 0, "pair-aligned split");
 };
 
-// Asynchronous copy of one net's shared-memory image (BF16 B tiles and the
+// Asynchronous copy of one net's shared-memory image (FP16 B tiles and the
 // FP32 first layer / biases); completes at the caller's cp_async_wait.
 template <int E0, int E1, int E2>
 __device__ __forceinline__ void mix_load_net(const DevModel &M, int k, char *netb, float *small) {
@@ -123,7 +123,7 @@ __device__ __forceinline__ void mix_load_net(const DevModel &M, int k, char *net
 }
 
 // Row geometry of the mixed form: the guarded norm, s(r) of utils.py:29-32
-// and ds/dr as in row_geom, with fast reciprocals (a few ulp; the BF16 GEMMs
+// and ds/dr as in row_geom, with fast reciprocals (a few ulp; the FP16 GEMMs
 // downstream round far more).
 __device__ __forceinline__ void row_geom_mixed(float3 x, float rcut, RowGeom &g) {
   g.x[0] = x.x; g.x[1] = x.y; g.x[2] = x.z;
@@ -182,11 +182,6 @@ __device__ __forceinline__ void mix_row_env(float4 rb, float rcut, float inv_std
 __device__ __forceinline__ uint4 pack8h(const float *v, float s) {
   return make_uint4(tc::as_u32(tc::f2_to_h2(v[0] * s, v[1] * s)), tc::as_u32(tc::f2_to_h2(v[2] * s, v[3] * s)),
                     tc::as_u32(tc::f2_to_h2(v[4] * s, v[5] * s)), tc::as_u32(tc::f2_to_h2(v[6] * s, v[7] * s)));
-}
-
-__device__ __forceinline__ uint4 pack8(const float *v) {
-  return make_uint4(tc::pack_bf16(v[0], v[1]), tc::pack_bf16(v[2], v[3]), tc::pack_bf16(v[4], v[5]),
-                    tc::pack_bf16(v[6], v[7]));
 }
 
 // ---------------------------------------------------------------- embedding rows in packed FP16
@@ -362,7 +357,7 @@ __device__ __forceinline__ float row_stilde(float4 rb, float rcut, float inv_std
 // where Rblk holds each row's env row R~ in its atom's 16-lane slot (zero
 // elsewhere), so D3 accumulates T_a = sum_rows R~^T h2 for the 8 atoms in
 // TMEM across all tiles of both neighbour types.  The block epilogue writes
-// T / Nnbrs (FP32) and the descriptor G (BF16, dpmodel.py:74-78).  Only the
+// T / Nnbrs (FP32) and the descriptor G (FP16, dpmodel.py:74-78).  Only the
 // current neighbour type's net is resident (2 CTAs per SM).
 constexpr int kRblkBytes = 128 * 128 * 2;
 constexpr int kFwdThreads = 256;
@@ -560,7 +555,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_mix_embed_fwd(DevModel M, Sy
         *reinterpret_cast<uint4 *>(rblk + o + 128) = make_uint4(0, 0, 0, 0);
       }
     }
-    // ---- block epilogue: T (FP32) and G (BF16) from the TMEM accumulators
+    // ---- block epilogue: T (FP32) and G (FP16) from the TMEM accumulators
     __syncthreads();
     float *Xs = reinterpret_cast<float *>(rblk);  // T staging [slot][c][w], 8 x 10 x E2 floats
     {
@@ -1285,7 +1280,7 @@ int launch_mix_embed_bwd(const DevModel &M, const SysDesc &D, const float4 *posS
   return DPB_OK;
 }
 
-// ---------------------------------------------------------------- fitting chain (BF16 tcgen05, TMA weights)
+// ---------------------------------------------------------------- fitting chain (FP16 tcgen05, TMA weights)
 // One CTA per 128 atoms of one centre type (thread = atom = TMEM lane).  The
 // forward layers, the adjoint down to the first hidden layer and dE/dG are a
 // fixed sequence of M = 128 GEMMs on the tensor cores, with L hidden layers:
@@ -2018,7 +2013,7 @@ int launch_embed_bwd_gen(const DevModel &, const SysDesc &, int, const float *, 
 // Embedding nets without tensor-core kernels in the mixed form - compressed
 // tables (a lookup, no GEMM) and shapes other than the tuned ones: the FP32
 // kernels produce T and G (FP32) and take the adjoint; the fitting chain runs
-// on the tensor cores from a BF16 copy of G.
+// on the tensor cores from an FP16 copy of G.
 static int mixed_eval_compressed(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm,
                                  const float *box, const int32_t *nbrs, double *energy, float *Eatom, float4 *F4,
                                  double *virial, float *T, __half *Gb, float *dG, float *scratch, int *err,
@@ -2053,7 +2048,7 @@ static int mixed_eval_compressed(const DevModel &M, const SysDesc &D, const floa
   return DPB_OK;
 }
 
-// Descriptor stage alone (diagnostics): T and G as FP32; the BF16 G of the
+// Descriptor stage alone (diagnostics): T and G as FP32; the FP16 G of the
 // tensor-core kernel is staged in the caller's workspace.
 int mixed_descriptors_f32(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm,
                           const float *box, const int32_t *nbrs, float *T, float *G, int *err, void *ws,

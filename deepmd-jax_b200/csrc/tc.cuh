@@ -153,11 +153,6 @@ __device__ __forceinline__ float tanh_fast(float x) {
   return y;
 }
 
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-  __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-  return *reinterpret_cast<uint32_t *>(&h);
-}
-
 // ---- packed FP16 pairs (element k in the low half, k + 1 in the high half,
 // the order of consecutive elements in the operand tiles)
 __device__ __forceinline__ __half2 as_h2(uint32_t u) { return *reinterpret_cast<__half2 *>(&u); }
