@@ -59,7 +59,7 @@ class DPModel:
     """se_a energy model with the reference DPModel's methods.
 
     ``precision`` selects 'fp32' (default; the reference's float32) or
-    'mixed' (BF16 tensor-core contractions with FP32 accumulation)."""
+    'mixed' (FP16 tensor-core contractions with FP32 accumulation)."""
 
     def __init__(self, params, precision="fp32"):
         self.params = params

@@ -128,7 +128,7 @@ def parse_couple_axes(couple_axes):
 class Simulation:
     """Two-step usage, as in the reference: ``sim = Simulation(...)`` then
     ``traj = sim.run(steps)``.  Extra keyword ``precision`` selects 'fp32'
-    (default, the reference's float32) or 'mixed' (BF16 tensor-core GEMMs);
+    (default, the reference's float32) or 'mixed' (FP16 tensor-core GEMMs);
     ``autotune`` (default: on from 10,000 atom-beads) lets the library time
     its launch-shape candidates on this system once, before any graph is
     captured (``launch_shapes`` holds the choice).  Besides a model.pkl path

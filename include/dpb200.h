@@ -50,7 +50,7 @@ extern "C" {
 /* Precision of the evaluation.
  * DPB_PREC_FP32:  all arithmetic in FP32 (the reference's float32 with
  *                 jax_default_matmul_precision='float32', deepmd_jax/__init__.py:10).
- * DPB_PREC_MIXED: embedding/fitting contractions in BF16 on the tensor cores
+ * DPB_PREC_MIXED: embedding/fitting contractions in FP16 on the tensor cores
  *                 with FP32 accumulation; s(r), env matrix, first embedding
  *                 layer, per-atom energies and forces in FP32. */
 #define DPB_PREC_FP32 0
@@ -98,7 +98,7 @@ typedef struct {
   const double *cmp_srmax;          /* [ntypes*ntypes] or NULL */
 } dpb_model_desc;
 
-/* Upload the weights (FP32 and BF16 copies) to the current device.
+/* Upload the weights (FP32, and the tensor-core images) to the current device.
  * Replaces: model loading + replication, deepmd_jax/utils.py:230-237. */
 DPB_API int dpb_model_create(const dpb_model_desc *desc, dpb_model **out);
 DPB_API int dpb_model_destroy(dpb_model *model);
