@@ -110,11 +110,29 @@ using namespace dpb;
 
 static size_t al(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// Device memory of a model, 256-byte aligned, freed with it.  Parts below 4 MB
+// share blocks of that size: a cudaMalloc for each of a model's hundred-odd parts
+// took 3 of the 24 ms of its creation.
+static int model_alloc(dpb_model *m, size_t bytes, void **p) {
+  constexpr size_t kBlock = (size_t)8 << 20;
+  bytes = al(bytes);
+  if (bytes >= kBlock / 2 || bytes > m->block_left) {
+    if (cudaMalloc(p, bytes >= kBlock / 2 ? bytes : kBlock) != cudaSuccess) return DPB_ERR_CUDA;
+    m->allocs.push_back(*p);
+    if (bytes >= kBlock / 2) return DPB_OK;
+    m->block = (char *)*p;
+    m->block_left = kBlock;
+  }
+  *p = m->block;
+  m->block += bytes;
+  m->block_left -= bytes;
+  return DPB_OK;
+}
+
 template <class T>
 static int upload(dpb_model *m, const T *host, size_t n, const T **dev) {
   void *p = nullptr;
-  if (cudaMalloc(&p, n * sizeof(T)) != cudaSuccess) return DPB_ERR_CUDA;
-  m->allocs.push_back(p);
+  if (int rc = model_alloc(m, n * sizeof(T), &p)) return rc;
   if (cudaMemcpy(p, host, n * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) return DPB_ERR_CUDA;
   *dev = (const T *)p;
   return DPB_OK;
@@ -124,8 +142,7 @@ static int upload(dpb_model *m, const T *host, size_t n, const T **dev) {
 // uploaded matrix: B[n][k] = w[n sn + k sk].
 static int fit_tiles(dpb_model *m, const float *w, int N, int K, int sn, int sk, float scale, const __half **dev) {
   void *p = nullptr;
-  if (cudaMalloc(&p, gemm_tiles_halves(N, K) * sizeof(__half)) != cudaSuccess) return DPB_ERR_CUDA;
-  m->allocs.push_back(p);
+  if (int rc = model_alloc(m, gemm_tiles_halves(N, K) * sizeof(__half), &p)) return rc;
   *dev = (const __half *)p;
   return launch_gemm_tiles(w, N, K, sn, sk, scale, (__half *)p);
 }

@@ -8,6 +8,9 @@
 struct dpb_model {
   dpb::DevModel dm;
   std::vector<void *> allocs;
+  // the rest of the newest 8 MB block that small parts of the model are placed in
+  char *block = nullptr;
+  size_t block_left = 0;
   int device;
   // launch shapes chosen by dpb_md_autotune (they never change results):
   // atoms (warps) per block of the mixed dE/dT kernel, and the mixed fitting
