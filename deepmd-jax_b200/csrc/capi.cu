@@ -62,11 +62,11 @@ void split_net_image(int E2, const float *w0, const float *b0, const float *w1, 
                      const float *b2, double s_lo, double s_hi, std::vector<char> &img, std::vector<float> &small);
 int split_block_atoms(const SysDesc &D);
 int split_embed_fwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
-                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, float *gmax,
+                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, float *gmax, int *err,
                     cudaStream_t st);
 int split_embed_bwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
                     const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, const float *dG, float4 *F4,
-                    double *virial, cudaStream_t st);
+                    double *virial, int *err, cudaStream_t st);
 template <int E2>
 int launch_embed_fwd_cmp(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
                          const int32_t *, float *, float *, float *, cudaStream_t);
@@ -88,7 +88,7 @@ int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, floa
 int launch_eval_begin(size_t NF, float4 *F4, size_t nE, double *energy, double *virial, int *err, cudaStream_t st);
 int *mixed_err(const DevModel &M, size_t NF, void *ws);
 int launch_finalize(int, int, const float4 *, float *, const float *, const int32_t *, float *, double *, int,
-                    const float *, const int32_t *, uint32_t *, cudaStream_t);
+                    const float *, const int32_t *, const int *, uint32_t *, cudaStream_t);
 // mixed path (mixed.cu)
 int mixed_supported(const DevModel &M);
 int mixed_fit_width(const DevModel &M);
@@ -621,12 +621,12 @@ static SplitWs split_ws(const DevModel &M, size_t NF, size_t nE, char *base, cha
 // tables and other shapes in the FP32 kernels.
 static int embed_fwd_fp32(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm,
                           const float *box, const int32_t *nbrs, const SplitWs &sw, int ba, float *T, float *G,
-                          float *gmax, cudaStream_t st) {
+                          float *gmax, int *err, cudaStream_t st) {
   int rc = DPB_OK;
   if (M.ngrids == 0 && M.emb_tuned) {
     rc = launch_pos_sorted(D, pos, perm, sw.posS, st);
     if (!rc && sw.rows && D.S <= kRowStoreCap) rc = launch_rows(M, D, ba, sw.posS, box, nbrs, sw.rows, sw.rcnt, st);
-    if (!rc) rc = split_embed_fwd(M, D, ba, sw.posS, box, nbrs, sw.rows, sw.rcnt, T, G, gmax, st);
+    if (!rc) rc = split_embed_fwd(M, D, ba, sw.posS, box, nbrs, sw.rows, sw.rcnt, T, G, gmax, err, st);
     return rc;
   }
   for (int ti = 0; ti < M.ntypes && !rc; ++ti)
@@ -638,7 +638,7 @@ static int embed_fwd_fp32(const DevModel &M, const SysDesc &D, const float *pos,
 
 static int eval_fp32(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm,
                      const float *box, const int32_t *nbrs, double *energy, float4 *F4, float *Eatom,
-                     double *virial, char *base, char *w, size_t nE, cudaStream_t st) {
+                     double *virial, char *base, char *w, size_t nE, int *err, cudaStream_t st) {
   const size_t NF = (size_t)D.N * D.F;
   const int E2 = M.E2, A = M.A, K0 = A * E2;
   float *T = (float *)w; w += al(NF * 10 * E2 * 4);
@@ -647,7 +647,7 @@ static int eval_fp32(const DevModel &M, const SysDesc &D, const float *pos, cons
   const int ba = split_block_atoms(D);
   int rc;
   prof_begin(PROF_EMBED_FWD, st);
-  rc = embed_fwd_fp32(M, D, pos, perm, box, nbrs, sw, ba, T, G, Eatom, st);
+  rc = embed_fwd_fp32(M, D, pos, perm, box, nbrs, sw, ba, T, G, Eatom, err, st);
   if (rc) return rc;
   prof_end(PROF_EMBED_FWD, st);
   prof_begin(PROF_FIT, st);
@@ -657,7 +657,7 @@ static int eval_fp32(const DevModel &M, const SysDesc &D, const float *pos, cons
   prof_begin(PROF_EMBED_BWD, st);
   if (M.ngrids == 0 && M.emb_tuned) {
     if (!sw.rows) rc = launch_pos_sorted(D, pos, perm, sw.posS, st);  // the fitting chain overwrote them
-    if (!rc) rc = split_embed_bwd(M, D, ba, sw.posS, box, nbrs, sw.rows, sw.rcnt, T, G, F4, virial, st);
+    if (!rc) rc = split_embed_bwd(M, D, ba, sw.posS, box, nbrs, sw.rows, sw.rcnt, T, G, F4, virial, err, st);
     if (rc) return rc;
   } else {
     for (int ti = 0; ti < M.ntypes; ++ti) {
@@ -696,16 +696,18 @@ int dpb::eval_impl(const dpb_model *m, int precision, const float *pos, const in
   double *vscratch = (double *)w; w += al(nE * 9 * 8);
   if (!vir) vir = vscratch;
   if (precision == DPB_PREC_MIXED && !mixed_supported(M)) return DPB_ERR_UNSUPPORTED;
-  rc = launch_eval_begin(NF, F4, nE, energy, vir, precision == DPB_PREC_MIXED ? mixed_err(M, NF, w) : nullptr, st);
+  int *err = precision == DPB_PREC_MIXED ? mixed_err(M, NF, w) : (int *)w;  // a tensor-core wait gave up
+  rc = launch_eval_begin(NF, F4, nE, energy, vir, err, st);
   if (rc) return rc;
   if (precision == DPB_PREC_FP32) {
-    rc = eval_fp32(M, D, pos, perm, box, nbrs, energy, F4, Eatom, vir, (char *)workspace, w, nE, st);
+    w += 256;
+    rc = eval_fp32(M, D, pos, perm, box, nbrs, energy, F4, Eatom, vir, (char *)workspace, w, nE, err, st);
   } else {
     rc = mixed_eval(M, D, pos, perm, box, nbrs, energy, Eatom, F4, vir, w, st, m->dT_warps, m->fit_deep != 0);
   }
   if (rc) return rc;
-  return launch_finalize((int)NF, natoms, F4, force, Eatom, perm, atom_energy, energy, (int)nE, pos, seg, status,
-                         st);
+  return launch_finalize((int)NF, natoms, F4, force, Eatom, perm, atom_energy, energy, (int)nE, pos, seg, err,
+                         status, st);
 }
 
 namespace dpb {
@@ -770,7 +772,7 @@ extern "C" int dpb_eval_descriptors(const dpb_model *m, int precision, const flo
   auto fp32 = [&]() {
     char *w = (char *)workspace;
     const SplitWs sw = split_ws(m->dm, (size_t)natoms * nframes, (size_t)nframes, w, w);
-    return embed_fwd_fp32(m->dm, D, pos, perm, box, nbrs, sw, split_block_atoms(D), T, G, nullptr, st);
+    return embed_fwd_fp32(m->dm, D, pos, perm, box, nbrs, sw, split_block_atoms(D), T, G, nullptr, err, st);
   };
   if (precision == DPB_PREC_FP32) return fp32();
   if (precision == DPB_PREC_MIXED) {

@@ -370,7 +370,8 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_fwd(DevModel M, SysD
                                                                const int32_t *__restrict__ nbrs,
                                                                const float4 *__restrict__ rows_g,
                                                                const int *__restrict__ rcnt, float *__restrict__ Tout,
-                                                               float *__restrict__ Gout, float *__restrict__ gmax) {
+                                                               float *__restrict__ Gout, float *__restrict__ gmax,
+                                                               int *__restrict__ err) {
   using SD = SplitDims<E0, E1, E2>;
   using SM = SplitFwdSmem<E0, E1, E2>;
   extern __shared__ __align__(1024) char smem[];
@@ -692,8 +693,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_fwd(DevModel M, SysD
     if (gmax && tid < nb) gmax[g0 + tid] = __int_as_float(gmax_s[tid]);
   }
   if (!ok) {
-    // a tensor-core wait gave up: NaN descriptors reach the energy and the status word
-    if (tid == 0) Gout[0] = __int_as_float(0x7fffffff);
+    if (tid == 0) atomicOr(err, 1);  // a tensor-core wait gave up (k_finalize)
     tc::mbar_wait(&mbar, ph);
   }
   tc::cp_async_wait<0>();
@@ -859,7 +859,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
                                                                const float4 *__restrict__ rows_g,
                                                                const int *__restrict__ rcnt,
                                                                const float *__restrict__ dT, float4 *__restrict__ F4,
-                                                               double *__restrict__ virial) {
+                                                               double *__restrict__ virial, int *__restrict__ err) {
   using SD = SplitDims<E0, E1, E2>;
   using SM = SplitBwdSmem<E0, E1, E2>;
   extern __shared__ __align__(1024) char smem[];
@@ -1125,8 +1125,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
     if (lane == 0 && s != 0.f) atomicAdd(&vir_s[k], (double)s);
   }
   if (!ok) {
-    // a tensor-core wait gave up: a NaN force raises the status word
-    if (tid == 0) F4[0].x = __int_as_float(0x7fffffff);
+    if (tid == 0) atomicOr(err, 1);  // a tensor-core wait gave up (k_finalize)
     tc::mbar_wait(&mbar, ph);
   }
   tc::cp_async_wait<0>();
@@ -1155,13 +1154,13 @@ int split_block_atoms(const SysDesc &D) {
 
 template <int E0, int E1, int E2>
 static int launch_fwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
-                      const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, float *gmax,
-                    cudaStream_t st) {
+                      const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, float *gmax, int *err,
+                      cudaStream_t st) {
   const int nblk = blocks_total(D, ba), smem = SplitFwdSmem<E0, E1, E2>::total;
   if (!nblk) return DPB_OK;
   DPB_CUDA_TRY(cudaFuncSetAttribute(k_split_fwd<E0, E1, E2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int grid = std::min(nblk, 2 * split_sms());
-  k_split_fwd<E0, E1, E2><<<grid, kSplitThreads, smem, st>>>(M, D, ba, posS, box, nbrs, rows, rcnt, T, G, gmax);
+  k_split_fwd<E0, E1, E2><<<grid, kSplitThreads, smem, st>>>(M, D, ba, posS, box, nbrs, rows, rcnt, T, G, gmax, err);
   count_launch();
   DPB_LAUNCH_CHECK();
   return DPB_OK;
@@ -1170,7 +1169,7 @@ static int launch_fwd(const DevModel &M, const SysDesc &D, int ba, const float4 
 template <int E0, int E1, int E2>
 static int launch_bwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
                       const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, const float *dG, float4 *F4,
-                      double *virial, cudaStream_t st) {
+                      double *virial, int *err, cudaStream_t st) {
   const int nblk = blocks_total(D, ba), smem = SplitBwdSmem<E0, E1, E2>::total;
   if (!nblk) return DPB_OK;
   const size_t NF = (size_t)D.N * D.F;
@@ -1182,24 +1181,24 @@ static int launch_bwd(const DevModel &M, const SysDesc &D, int ba, const float4 
   DPB_LAUNCH_CHECK();
   DPB_CUDA_TRY(cudaFuncSetAttribute(k_split_bwd<E0, E1, E2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int grid = std::min(nblk, 2 * split_sms());
-  k_split_bwd<E0, E1, E2><<<grid, kSplitThreads, smem, st>>>(M, D, ba, posS, box, nbrs, rows, rcnt, T, F4, virial);
+  k_split_bwd<E0, E1, E2><<<grid, kSplitThreads, smem, st>>>(M, D, ba, posS, box, nbrs, rows, rcnt, T, F4, virial, err);
   count_launch();
   DPB_LAUNCH_CHECK();
   return DPB_OK;
 }
 
 int split_embed_fwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
-                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, float *gmax,
+                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, float *gmax, int *err,
                     cudaStream_t st) {
-  return M.E2 == 100 ? launch_fwd<25, 50, 100>(M, D, ba, posS, box, nbrs, rows, rcnt, T, G, gmax, st)
-                     : launch_fwd<32, 32, 64>(M, D, ba, posS, box, nbrs, rows, rcnt, T, G, gmax, st);
+  return M.E2 == 100 ? launch_fwd<25, 50, 100>(M, D, ba, posS, box, nbrs, rows, rcnt, T, G, gmax, err, st)
+                     : launch_fwd<32, 32, 64>(M, D, ba, posS, box, nbrs, rows, rcnt, T, G, gmax, err, st);
 }
 
 int split_embed_bwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
                     const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, const float *dG, float4 *F4,
-                    double *virial, cudaStream_t st) {
-  return M.E2 == 100 ? launch_bwd<25, 50, 100>(M, D, ba, posS, box, nbrs, rows, rcnt, T, dG, F4, virial, st)
-                     : launch_bwd<32, 32, 64>(M, D, ba, posS, box, nbrs, rows, rcnt, T, dG, F4, virial, st);
+                    double *virial, int *err, cudaStream_t st) {
+  return M.E2 == 100 ? launch_bwd<25, 50, 100>(M, D, ba, posS, box, nbrs, rows, rcnt, T, dG, F4, virial, err, st)
+                     : launch_bwd<32, 32, 64>(M, D, ba, posS, box, nbrs, rows, rcnt, T, dG, F4, virial, err, st);
 }
 
 }  // namespace dpb

@@ -589,28 +589,35 @@ __global__ void __launch_bounds__(256) k_fit_energy(EnergyArgs g, const float *_
 
 // Forces (float4 accumulator) and per-atom energies to the caller's layout;
 // non-finite positions or results raise status bit 16 and, as NaN inputs do
-// in the reference's float arithmetic, make the frame's energy NaN.
+// in the reference's float arithmetic, make the frame's energy NaN.  *err != 0:
+// a tensor-core wait gave up, and what its CTA did not write is left from an
+// earlier call, so every result is NaN.
 __global__ void k_finalize(int NF, int N, const float4 *__restrict__ F4, float *__restrict__ force,
                            const float *__restrict__ Eatom_sorted, const int32_t *__restrict__ perm,
                            float *__restrict__ atom_energy, double *__restrict__ energy, int nE,
                            const float *__restrict__ pos, const int32_t *__restrict__ seg,
-                           uint32_t *__restrict__ status) {
+                           const int *__restrict__ err, uint32_t *__restrict__ status) {
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool gave_up = err && *err != 0;
+  const float nan = __int_as_float(0x7fffffff);
   if (g < NF) {
-    const float4 v = F4[g];
+    const float4 v = gave_up ? make_float4(nan, nan, nan, 0.f) : F4[g];
     force[(size_t)g * 3 + 0] = v.x;
     force[(size_t)g * 3 + 1] = v.y;
     force[(size_t)g * 3 + 2] = v.z;
     const int f = g / N, k = g - f * N;
     const int dst = perm ? perm[k] : k;
-    if (atom_energy) atom_energy[(size_t)f * N + dst] = Eatom_sorted[g];
+    if (atom_energy) atom_energy[(size_t)f * N + dst] = gave_up ? nan : Eatom_sorted[g];
     const float *p = pos + ((size_t)f * N + dst) * 3;  // position of sorted atom g
     const bool bad_in = !isfinite(p[0]) || !isfinite(p[1]) || !isfinite(p[2]);
     if (bad_in || !isfinite(v.x) || !isfinite(v.y) || !isfinite(v.z)) atomicOr(status, DPB_ST_NONFINITE);
     const int e = energy_slot(seg, g, N);
     if (bad_in && e >= 0) energy[e] = __longlong_as_double(0x7ff8000000000000LL);
   }
-  if (g < nE && !isfinite(energy[g])) atomicOr(status, DPB_ST_NONFINITE);
+  if (g < nE) {
+    if (gave_up) energy[g] = __longlong_as_double(0x7ff8000000000000LL);
+    if (gave_up || !isfinite(energy[g])) atomicOr(status, DPB_ST_NONFINITE);
+  }
 }
 
 template <int E2>
@@ -665,13 +672,24 @@ int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, floa
 
 int launch_finalize(int NF, int N, const float4 *F4, float *force, const float *Eatom, const int32_t *perm,
                     float *atom_energy, double *energy, int nE, const float *pos, const int32_t *seg,
-                    uint32_t *status, cudaStream_t st) {
+                    const int *err, uint32_t *status, cudaStream_t st) {
   int n = NF > nE ? NF : nE;
   k_finalize<<<(n + 255) / 256, 256, 0, st>>>(NF, N, F4, force, Eatom, perm, atom_energy, energy, nE, pos, seg,
-                                              status);
+                                              err, status);
   count_launch();
   DPB_LAUNCH_CHECK();
   return DPB_OK;
 }
 
 }  // namespace dpb
+
+extern "C" int dpb_selftest_finalize(int natoms, int nframes, const float *acc, const float *pos, const int *err,
+                                     double *energy, float *atom_energy, float *force, uint32_t *status,
+                                     void *stream) {
+  if (natoms <= 0 || nframes <= 0 || !acc || !pos || !energy || !atom_energy || !force || !status ||
+      (reinterpret_cast<uintptr_t>(acc) & 15) != 0)
+    return DPB_ERR_INVALID_ARG;
+  return dpb::launch_finalize(natoms * nframes, natoms, reinterpret_cast<const float4 *>(acc), force, atom_energy,
+                              nullptr, atom_energy, energy, nframes, pos, nullptr, err, status,
+                              (cudaStream_t)stream);
+}

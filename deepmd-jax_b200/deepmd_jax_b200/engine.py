@@ -196,7 +196,8 @@ class DeviceModel:
                                            _lib.int_array(type_count), _ptr(box), _ptr(nbrs), _lib.int_array(sel),
                                            _ptr(T), _ptr(G), _ptr(err), _ptr(ws), ws.numel(), _stream())
         _lib.check(rc, "dpb_eval_descriptors")
-        return T, G
+        gave_up = err != 0  # a tensor-core wait gave up: no part is to be trusted
+        return T.masked_fill_(gave_up, float("nan")), G.masked_fill_(gave_up, float("nan"))
 
 
 class NeighborBuilder:

@@ -150,7 +150,8 @@ DPB_API int dpb_eval_workspace_bytes(const dpb_model *model, int natoms, int nfr
  *   virial   (F,9) float64 device out or NULL: W_ab = -sum_pairs x_a dE/dx_b
  *            with x = r_j - r_i; trace(W) = -dU/deps of a uniform strain
  *            (deepmd_jax/md_utils.py:139-159)
- *   status   device word (DPB_ST_NONFINITE on NaN/Inf energies). */
+ *   status   device word (DPB_ST_NONFINITE on NaN/Inf energies, and with NaN
+ *            results where a tensor-core wait gave up). */
 DPB_API int dpb_eval(const dpb_model *model, int precision, const float *pos, const int32_t *perm,
              int natoms, int nframes, const int *type_count, const float *box,
              const int32_t *nbrs, const int *sel, double *energy, float *atom_energy,
@@ -369,11 +370,17 @@ DPB_API int dpb_profile_enable(int on);
  * 128x64x32 BF16 product into TMEM (variant 0: K-major operands, 1: MN-major);
  * out: 128*64 floats (device), err: device int set on a barrier timeout. */
 DPB_API int dpb_selftest_tcgen05(int variant, float *out, int *err, void *stream);
+/* Diagnostics: the last step of an evaluation alone, on sums given by the
+ * caller (acc: (F,N,4) float32, 16-byte aligned; energy (F), atom_energy (F,N)
+ * in place).  err: device int or NULL; where it is set, as by a tensor-core wait
+ * that gave up, every result becomes NaN and DPB_ST_NONFINITE is raised. */
+DPB_API int dpb_selftest_finalize(int natoms, int nframes, const float *acc, const float *pos, const int *err,
+                                  double *energy, float *atom_energy, float *force, uint32_t *status, void *stream);
 DPB_API int dpb_profile_read(int stage, double *ms, uint64_t *count);
 
 /* The descriptor stage alone: T (F,N,10,W) = sum_j R~^T h2 / Nnbrs and
  * G (F,N,A*W) float32, type-sorted atom order (deepmd_jax/dpmodel.py:50-78);
- * err: device int set when a tensor-core wait gave up (mixed path);
+ * err: device int set when a tensor-core wait gave up;
  * workspace as for dpb_eval. */
 DPB_API int dpb_eval_descriptors(const dpb_model *model, int precision, const float *pos, const int32_t *perm,
                                  int natoms, int nframes, const int *type_count, const float *box,
