@@ -871,6 +871,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
   __shared__ float3 ri_s[kBlkAtoms];
   __shared__ float fi_s[4 * 3];
   __shared__ double vir_s[9];
+  __shared__ float wvir_s[4][9];
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tbase_s;
   const int tid = threadIdx.x, warp = tc::warp_index(), lane = tid & 31;
@@ -887,24 +888,11 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
   bool ok = true;
   const uint32_t idesc1 = tc::idesc_f16(128, SD::N1, 0, 0), idesc2 = tc::idesc_f16(128, SD::NP, 0, 0);
   const uint32_t w1_u = tc::smem_u32(netb), w2_u = w1_u + 2 * SD::W1B;
+  // the virial of the rows of one block in FP32, from block to block in FP64
   float vir[9];
 #pragma unroll
   for (int k = 0; k < 9; ++k) vir[k] = 0.f;
   int vframe = -1;
-  auto flush_virial = [&]() {
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-      const float s = warp_sum(vir[k]);
-      if (lane == 0 && s != 0.f) atomicAdd(&vir_s[k], (double)s);
-      vir[k] = 0.f;
-    }
-    __syncthreads();
-    if (tid < 9) {
-      atomicAdd(&virial[vframe * 9 + tid], vir_s[tid]);
-      vir_s[tid] = 0.0;
-    }
-    __syncthreads();
-  };
   const int nblk = blocks_total(D, ba);
   int loaded_net = -1;
 
@@ -921,10 +909,13 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
       prefetch_range_l2(dT + bn.g0 * 10 * E2, (size_t)bn.nb * 10 * E2 * 4);
     }
     const int bs = box_slot(D, g0, f);
-    if (bs != vframe) {
-      if (vframe >= 0) flush_virial();
-      vframe = bs;
+    if (bs != vframe && tid < 9) {
+      if (vframe >= 0) {
+        atomicAdd(&virial[vframe * 9 + tid], vir_s[tid]);
+        vir_s[tid] = 0.0;
+      }
     }
+    vframe = bs;
     const float3 L = make_float3(box[bs * 3], box[bs * 3 + 1], box[bs * 3 + 2]);
     const int3 ni = image_range(L, M.rcut);
     const int nim = (2 * ni.x + 1) * (2 * ni.y + 1) * (2 * ni.z + 1);
@@ -1111,18 +1102,23 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
       }
     }
     if (!ok) break;
+    if (half == 0) {
+#pragma unroll
+      for (int k = 0; k < 9; ++k) {
+        const float s = warp_sum(vir[k]);
+        if (lane == 0) wvir_s[warp][k] = s;
+        vir[k] = 0.f;
+      }
+    }
     __syncthreads();
+    if (tid < 9)
+      vir_s[tid] += ((double)wvir_s[0][tid] + (double)wvir_s[1][tid]) + ((double)wvir_s[2][tid] + (double)wvir_s[3][tid]);
     if (tid < nb * 3) {
       const int a = tid / 3, k = tid - a * 3;
       const int src = __float_as_int(posS[g0 + a].w);
       atomicAdd(reinterpret_cast<float *>(&F4[frame_base + src]) + k, fi_s[tid]);
     }
     __syncthreads();
-  }
-#pragma unroll
-  for (int k = 0; k < 9; ++k) {
-    const float s = warp_sum(vir[k]);
-    if (lane == 0 && s != 0.f) atomicAdd(&vir_s[k], (double)s);
   }
   if (!ok) {
     if (tid == 0) atomicOr(err, 1);  // a tensor-core wait gave up (k_finalize)
