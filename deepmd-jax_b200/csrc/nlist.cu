@@ -47,6 +47,8 @@ static NlGrid cell_grid(const float box[3], float rc, int reach) {
   for (int d = 0; d < 3; ++d) {
     g.nc[d] = std::max(1, std::min((int)floorf(box[d] * (float)reach / rc), 512));
     while (g.nc[d] > 1 && (double)box[d] * reach < (double)rc * g.nc[d]) --g.nc[d];
+    // where cells beyond `reach` exist, cells wide enough that rounding brings no atom of theirs within rc
+    while (g.nc[d] > 2 * reach + 1 && (double)box[d] * reach < ((double)rc + box[d] * 0x1p-20) * g.nc[d]) --g.nc[d];
     n *= g.nc[d];
     if (box[d] < 2.f * rc) g.image_mode = 1;
   }
@@ -505,7 +507,9 @@ int nlist_build_impl(const float *pos, const int32_t *perm, int natoms, int nfra
   P.reach = g.reach;
   P.h = make_float3(rb[0] / g.nc[0], rb[1] / g.nc[1], rb[2] / g.nc[2]);
   P.inv_h = make_float3(1.f / P.h.x, 1.f / P.h.y, 1.f / P.h.z);
-  const float rcm = rc_eff * 1.0001f + 1e-3f;  // far above the rounding of coordinates and bins
+  // above the rounding of bins, gaps (3 x 2^-24 L) and displacements (2^-21 L), also in a box so long
+  // that a float's step in it is no longer small
+  const float rcm = rc_eff * 1.0001f + 1e-3f + 0x1p-20f * std::max(rb[0], std::max(rb[1], rb[2]));
   P.rcm2 = rcm * rcm;
 
   const size_t C = (size_t)g.ncell * nframes;
