@@ -595,21 +595,20 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
   return DPB_OK;
 }
 
-// The workspace past the FP32 layout (sized for the larger of the two forms)
-// that holds the type-sorted positions and the row store of the tensor-core
-// embedding; where it is too small (fitting widths beyond the mixed form's) the
-// positions go to the fitting chain's scratch, idle then, and the kernels
-// compact the neighbour lists themselves.
+// Where the type-sorted positions and the row store of the tensor-core embedding
+// lie: at w, if `bytes` hold them.  In an evaluation that is the workspace past
+// the FP32 layout (it is sized for the larger of the two forms); where it is too
+// small (fitting widths beyond the mixed form's) the positions go to `fallback`,
+// the fitting chain's scratch, idle then, and the kernels compact the neighbour
+// lists themselves.
 struct SplitWs {
   float4 *posS, *rows;
   int *rcnt;
 };
-static SplitWs split_ws(const DevModel &M, size_t NF, size_t nE, char *base, char *fit_scratch) {
-  const size_t a = fp32_ws_bytes(M, NF) + 16 * 256 + al(nE * 9 * 8);
+static SplitWs split_ws(const DevModel &M, size_t NF, char *w, size_t bytes, char *fallback) {
   const size_t need = al(NF * 16) + al(NF * kRowStoreCap * 16) + al(NF * M.ntypes * 4);
-  SplitWs s{reinterpret_cast<float4 *>(fit_scratch), nullptr, nullptr};
-  if (eval_ws_bytes(M, NF, nE) >= a + need) {
-    char *w = base + a;
+  SplitWs s{reinterpret_cast<float4 *>(fallback), nullptr, nullptr};
+  if (bytes >= need) {
     s.posS = (float4 *)w; w += al(NF * 16);
     s.rows = (float4 *)w; w += al(NF * kRowStoreCap * 16);
     s.rcnt = (int *)w;
@@ -643,7 +642,8 @@ static int eval_fp32(const DevModel &M, const SysDesc &D, const float *pos, cons
   const int E2 = M.E2, A = M.A, K0 = A * E2;
   float *T = (float *)w; w += al(NF * 10 * E2 * 4);
   float *G = (float *)w; w += al(NF * K0 * 4);  // G, later dE/dG
-  const SplitWs sw = split_ws(M, NF, nE, base, w);
+  const size_t used = fp32_ws_bytes(M, NF) + 16 * 256 + al(nE * 9 * 8);
+  const SplitWs sw = split_ws(M, NF, base + used, eval_ws_bytes(M, NF, nE) - used, w);
   const int ba = split_block_atoms(D);
   int rc;
   prof_begin(PROF_EMBED_FWD, st);
@@ -770,8 +770,9 @@ extern "C" int dpb_eval_descriptors(const dpb_model *m, int precision, const flo
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   auto fp32 = [&]() {
-    char *w = (char *)workspace;
-    const SplitWs sw = split_ws(m->dm, (size_t)natoms * nframes, (size_t)nframes, w, w);
+    // nothing else is in the workspace, whose address may be any
+    char *w = (char *)al((size_t)workspace);
+    const SplitWs sw = split_ws(m->dm, (size_t)natoms * nframes, w, need - (size_t)(w - (char *)workspace), w);
     return embed_fwd_fp32(m->dm, D, pos, perm, box, nbrs, sw, split_block_atoms(D), T, G, nullptr, err, st);
   };
   if (precision == DPB_PREC_FP32) return fp32();
