@@ -770,10 +770,24 @@ extern "C" int dpb_eval_descriptors(const dpb_model *m, int precision, const flo
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   auto fp32 = [&]() {
-    // nothing else is in the workspace, whose address may be any
-    char *w = (char *)al((size_t)workspace);
-    const SplitWs sw = split_ws(m->dm, (size_t)natoms * nframes, w, need - (size_t)(w - (char *)workspace), w);
-    return embed_fwd_fp32(m->dm, D, pos, perm, box, nbrs, sw, split_block_atoms(D), T, G, nullptr, err, st);
+    // nothing else is in the workspace, whose address may be any; the kernels store
+    // 16 bytes at a time, so results for other addresses pass through it (an
+    // evaluation keeps its T and G there, next to much else)
+    const size_t NF = (size_t)natoms * nframes;
+    const size_t nT = NF * 10 * m->dm.E2 * 4, nG = NF * m->dm.A * m->dm.E2 * 4;
+    char *w = (char *)al((size_t)workspace), *end = (char *)workspace + need;
+    float *Td = T, *Gd = G;
+    if (((size_t)T | (size_t)G) & 15) {
+      Td = (float *)w; w += al(nT);
+      Gd = (float *)w; w += al(nG);
+    }
+    const SplitWs sw = split_ws(m->dm, NF, w, (size_t)(end - w), w);
+    int rc = embed_fwd_fp32(m->dm, D, pos, perm, box, nbrs, sw, split_block_atoms(D), Td, Gd, nullptr, err, st);
+    if (!rc && Td != T) {
+      DPB_CUDA_TRY(cudaMemcpyAsync(T, Td, nT, cudaMemcpyDeviceToDevice, st));
+      DPB_CUDA_TRY(cudaMemcpyAsync(G, Gd, nG, cudaMemcpyDeviceToDevice, st));
+    }
+    return rc;
   };
   if (precision == DPB_PREC_FP32) return fp32();
   if (precision == DPB_PREC_MIXED) {

@@ -636,17 +636,14 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_fwd(DevModel M, SysD
       }
     }
     __syncthreads();
-    if ((reinterpret_cast<uintptr_t>(Tout) & 15) == 0) {
+    {
       const int n4 = nb * 10 * E2 / 4;
       float4 *dst = reinterpret_cast<float4 *>(Tout + g0 * 10 * E2);
       for (int e = tid; e < n4; e += kSplitThreads) dst[e] = reinterpret_cast<const float4 *>(Xs)[e];
-    } else {  // a caller's array (dpb_eval_descriptors) at any float
-      for (int e = tid; e < nb * 10 * E2; e += kSplitThreads) Tout[g0 * 10 * E2 + e] = Xs[e];
     }
     // G[a][w] = sum_c Q[c][a] X[c][w], X = T + Tbias on channel 0 (dpmodel.py:74-78);
     // Q[slot][a][12] staged behind X
     const int A = M.A;
-    const bool g8 = (reinterpret_cast<uintptr_t>(Gout) & 7) == 0;
     float *Qs = Xs + 4 * 10 * E2;
     if (tid < 4) gmax_s[tid] = 0;
     for (int e = tid; e < nb * 160; e += kSplitThreads) {
@@ -687,12 +684,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_fwd(DevModel M, SysD
         v = tc::fma2(x[7], tc::pk1(qb.w), v);
         v = tc::fma2(x[8], tc::pk1(qc.x), v);
         v = tc::fma2(x[9], tc::pk1(qc.y), v);
-        if (g8) {
-          *reinterpret_cast<f2 *>(Gs + (size_t)aa * E2) = v;
-        } else {
-          Gs[(size_t)aa * E2] = lo_of(v);
-          Gs[(size_t)aa * E2 + 1] = hi_of(v);
-        }
+        *reinterpret_cast<f2 *>(Gs + (size_t)aa * E2) = v;
         gm = fmaxf(gm, fmaxf(fabsf(lo_of(v)), fabsf(hi_of(v))));
       }
       atomicMax(&gmax_s[slot], __float_as_int(gm));  // gm >= 0: the bits order as the values
