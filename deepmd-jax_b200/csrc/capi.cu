@@ -76,6 +76,7 @@ int launch_embed_bwd_cmp(const DevModel &, const SysDesc &, int, const float *, 
 // fitting GEMMs on the tensor cores (gemm_split.cu)
 size_t gemm_tiles_halves(int N, int K);
 size_t gemm_operand_halves(int mt, int K);
+size_t gemm_exp_bytes(size_t rows, int K);
 int launch_gemm_tiles(const float *w, int N, int K, int sn, int sk, float scale, __half *out);
 int launch_gemm_split(const GemmArgs &g, cudaStream_t st);
 // any embedding shape (eval_general.cu)
@@ -83,8 +84,8 @@ int launch_embed_fwd_gen(const DevModel &, const SysDesc &, int, const float *, 
                          const int32_t *, float *, float *, float *, cudaStream_t);
 int launch_embed_bwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
                          const int32_t *, const float *, const float *, float4 *, double *, cudaStream_t);
-int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, __half *gZ, double *energy,
-                      const int32_t *seg, cudaStream_t st);
+int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, __half *gZ, int8_t *gexp,
+                      double *energy, const int32_t *seg, cudaStream_t st);
 int launch_eval_begin(size_t NF, float4 *F4, size_t nE, double *energy, double *virial, int *err, cudaStream_t st);
 int *mixed_err(const DevModel &M, size_t NF, void *ws);
 int launch_finalize(int, int, const float4 *, float *, const float *, const int32_t *, float *, double *, int,
@@ -428,7 +429,8 @@ static size_t fp32_ws_bytes(const DevModel &M, size_t NF) {
   // operand tiles of 128 rows x 32 columns: one set beside, one in G where it fits
   const size_t fw = fit_width_max(M), op = al((NF + (size_t)127 * M.ntypes) * ((fw + 31) / 32 * 32) * 4);
   const size_t gh = M.nfit > 2 ? 2 * fw : 0;
-  return al(NF * ((10 * M.E2 + M.A * M.E2 + hid + gh + 1) * 4 + 16)) + op +
+  const size_t ex = al(gemm_exp_bytes(NF + (size_t)127 * M.ntypes, (int)fw)) * (M.nfit == 1 ? 1 : 2);
+  return al(NF * ((10 * M.E2 + M.A * M.E2 + hid + gh + 1) * 4 + 16)) + ex + op +
          (M.nfit == 1 || op <= NF * (size_t)(M.A * M.E2) * 4 ? 0 : op);
 }
 
@@ -492,6 +494,7 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
   // operand tiles: layer l's output, later its gate, in op[l & 1].  op[1] is G's
   // space, which is free between layer 0 (writes op[0]) and dE/dG (reads op[0])
   __half *op[2];
+  int8_t *ex[2] = {nullptr, nullptr};  // scale exponents of the gates in op[]
   GemmArgs g{};
   EnergyArgs en{};
   int ty[kMaxTypes], n = 0;  // the types present
@@ -507,6 +510,10 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
   }
   g.ntypes = en.ntypes = n;
   const size_t opb = al(gemm_operand_halves(g.mt0[n], FWM) * 2);
+  for (int i = 0; i < 2 && i < L; ++i) {
+    ex[i] = (int8_t *)w;
+    w += al(gemm_exp_bytes((size_t)g.mt0[n] * 128, FWM));
+  }
   op[0] = (__half *)w; w += opb;
   op[1] = opb <= NF * (size_t)K0 * 4 ? (__half *)G : (__half *)w;
   int rc, cur = 0;
@@ -551,14 +558,15 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
     en.t[k].wfin = M.fw[ty[k]][L];
     en.t[k].bfin = M.fb[ty[k]][L];
     en.t[k].dtl = M.fdt[ty[k]][L - 1];
-    en.t[k].gscale = M.fit_gsc[ty[k]][L - 1];
   }
   for (int k = 0; k <= n; ++k) en.mt0[k] = g.mt0[k];
-  if ((rc = launch_fit_energy(en, hb[L - 1], tb[L - 1], Eatom, op[(L - 1) & 1], energy, D.seg, st))) return rc;
+  if ((rc = launch_fit_energy(en, hb[L - 1], tb[L - 1], Eatom, op[(L - 1) & 1], ex[(L - 1) & 1], energy, D.seg, st)))
+    return rc;
   for (int l = L - 1; l >= 0; --l) {
     // l >= 1: gH_{l-1} = gZ_l W_l^T (+ gH_l through layer l's residual); l = 0: dE/dG
     g.A = nullptr;
     g.At = op[l & 1];
+    g.Aexp = ex[l & 1];
     g.lda = g.K = M.FW[l];
     g.N = l == 0 ? K0 : M.FW[l - 1];
     for (int k = 0; k < n; ++k) {
@@ -566,7 +574,7 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
       GemmType &t = g.t[k];
       t.B = M.fs_adj[ti][l];
       t.gmax = nullptr;
-      t.ascale = M.fit_gsc[ti][l];
+      t.ascale = 1.f;
       t.wscale = M.fit_wsc[ti][l];
       t.ep = Epi{};
       t.ep.ld = g.N;
@@ -581,7 +589,7 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
         else t.ep.gmat = gh[cur];
       }
       t.ep.tile = op[(l - 1) & 1];
-      t.ep.tscale = M.fit_gsc[ti][l - 1];
+      t.ep.texp = ex[(l - 1) & 1];
       t.ep.mode = EPI_GRAD;
       if (fit_res_width(M, l - 1) && M.fdt[ti][l - 1]) {
         t.ep.mode = EPI_GRAD_RES;

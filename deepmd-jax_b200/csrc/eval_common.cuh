@@ -124,8 +124,8 @@ enum EpiMode : int {
   EPI_STORE = 0,      // out1 = acc
   EPI_TANH = 1,       // t = tanh(acc + b); out1 = t; out2 = t (H = t)
   EPI_TANH_RES = 2,   // t = tanh(acc + b); out1 = t; out2 = t * dt + Hprev
-  EPI_GRAD_RES = 3,   // gH = acc + gadd; out2 = gH; out1 = gZ = gH * dt * (1 - t^2)
-  EPI_GRAD = 4,       // gH = acc + gadd; out1 = gZ = gH * (1 - t^2)
+  EPI_GRAD_RES = 3,   // gH = acc + gadd; out2 = gH; tile = gZ = gH * dt * (1 - t^2)
+  EPI_GRAD = 4,       // gH = acc + gadd; tile = gZ = gH * (1 - t^2)
 };
 
 // Fused epilogue of one fitting-layer GEMM (forward or adjoint).
@@ -139,7 +139,8 @@ struct Epi {
   const float *gmat;    // per atom addend (or NULL)
   float *out1, *out2;   // per atom, ld (or NULL)
   int ld;
-  __half *tile;         // the next GEMM's operand (GemmArgs::At) times tscale, or NULL
+  __half *tile;         // the next GEMM's operand (GemmArgs::At), or NULL: times tscale, or
+  int8_t *texp;         // (gates) times 2^k per row and 32 columns, k kept here (gemm_exp_at)
   float tscale;
 };
 
@@ -153,6 +154,15 @@ __host__ __device__ __forceinline__ size_t gemm_operand_at(int nc, int mt, int l
   return ((size_t)mt * nc + n / kGemmK) * (2 * kGemmPart) + ((n >> 3) & 3) * 1024 + lr * 8 + (n & 7);
 }
 
+// Place of the scale exponent of row lr and the 32 columns of chunk c: a byte each,
+// eight chunks to a word.
+__host__ __device__ __forceinline__ size_t gemm_exp_at(int nc, int mt, int lr, int c) {
+  return ((size_t)mt * 128 + lr) * ((nc + 7) & ~7) + c;
+}
+// k of the power of two that brings x >= 0 into [2^13, 2^14), within +-60; 2^k.
+__device__ __forceinline__ int gate_exp(float x) { return max(-60, min(60, 140 - (__float_as_int(x) >> 23))); }
+__device__ __forceinline__ float pow2i(int k) { return __int_as_float((127 + k) << 23); }
+
 // One centre type's part of a fitting GEMM over the atoms of every type
 // (gemm_split.cu): rows, weights, operand scales and epilogue.
 struct GemmType {
@@ -165,7 +175,8 @@ struct GemmType {
 };
 struct GemmArgs {
   const float *A;       // per atom, lda; or, where At is set,
-  const __half *At;     // hi and lo parts in tiles of 128 rows x 32 of K (gemm_tile_at)
+  const __half *At;     // hi and lo parts in tiles of 128 rows x 32 of K (gemm_operand_at)
+  const int8_t *Aexp;   // with At: the tiles' scale exponents (gemm_exp_at), or NULL: 0
   int lda, K, N, ntypes;
   int mt0[kMaxTypes + 1];  // first 128-row tile of each type
   GemmType t[kMaxTypes];
@@ -176,7 +187,6 @@ struct EnergyType {
   int Mrows;
   RowMap rm;
   const float *wfin, *bfin, *dtl;
-  float gscale;  // of the gate written as the adjoint GEMM's operand
 };
 struct EnergyArgs {
   int ntypes, FWl, N;

@@ -519,8 +519,8 @@ __global__ void __launch_bounds__(256, 2) k_embed_bwd(DevModel M, SysDesc D, int
 // reduced in FP64, one atomic per run of one energy row.
 __global__ void __launch_bounds__(256) k_fit_energy(EnergyArgs g, const float *__restrict__ H,
                                                     const float *__restrict__ tl, float *__restrict__ Eatom,
-                                                    __half *__restrict__ gZ, double *__restrict__ energy,
-                                                    const int32_t *__restrict__ seg) {
+                                                    __half *__restrict__ gZ, int8_t *__restrict__ gexp,
+                                                    double *__restrict__ energy, const int32_t *__restrict__ seg) {
   __shared__ double es[8];
   __shared__ int fs[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -535,16 +535,16 @@ __global__ void __launch_bounds__(256) k_fit_energy(EnergyArgs g, const float *_
     float s = 0.f;
     const int nc = (g.FWl + kGemmK - 1) / kGemmK, mt = g.mt0[ti] + r / 128, lr = r & 127;
     const float *h_ = H + at * g.FWl, *t_ = tl + at * g.FWl;
-    for (int n = 4 * lane; n < (g.FWl + 15) / 16 * 16; n += 128) {  // whole K = 16 steps
+    const int n16 = (g.FWl + 15) / 16 * 16;  // whole K = 16 steps
+    for (int n = 4 * lane; n - 4 * lane < n16; n += 128) {
       __align__(16) float h[4] = {0.f, 0.f, 0.f, 0.f}, t[4] = {1.f, 1.f, 1.f, 1.f}, w[4] = {0.f, 0.f, 0.f, 0.f};
       if ((g.FWl & 3) == 0 && n < g.FWl) {
         *reinterpret_cast<float4 *>(h) = *reinterpret_cast<const float4 *>(h_ + n);
         *reinterpret_cast<float4 *>(t) = *reinterpret_cast<const float4 *>(t_ + n);
       }
-      __align__(8) __half hi[4], lo[4];
+      float gz[4] = {0.f, 0.f, 0.f, 0.f}, gm = 0.f;
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        float gz = 0.f;
         if (n + e < g.FWl) {
           if ((g.FWl & 3) != 0) {
             h[e] = h_[n + e];
@@ -552,10 +552,21 @@ __global__ void __launch_bounds__(256) k_fit_energy(EnergyArgs g, const float *_
           }
           w[e] = et.wfin[n + e];
           s = fmaf(h[e], w[e], s);
-          gz = w[e] * (et.dtl ? et.dtl[n + e] : 1.f) * (1.f - t[e] * t[e]) * et.gscale;
+          gz[e] = w[e] * (et.dtl ? et.dtl[n + e] : 1.f) * (1.f - t[e] * t[e]);
+          gm = fmaxf(gm, fabsf(gz[e]));
         }
-        hi[e] = __float2half_rn(gz);
-        lo[e] = __float2half_rn(gz - __half2float(hi[e]));
+      }
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) gm = fmaxf(gm, __shfl_xor_sync(0xffffffffu, gm, o));
+      if (n >= n16) continue;
+      const int k = gate_exp(gm);
+      const float sc = pow2i(k);
+      if ((lane & 7) == 0) gexp[gemm_exp_at(nc, mt, lr, n / kGemmK)] = (int8_t)k;
+      __align__(8) __half hi[4], lo[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        hi[e] = __float2half_rn(gz[e] * sc);
+        lo[e] = __float2half_rn(gz[e] * sc - __half2float(hi[e]));
       }
       __half *o = gZ + gemm_operand_at(nc, mt, lr, n);
       *reinterpret_cast<uint2 *>(o) = *reinterpret_cast<const uint2 *>(hi);
@@ -660,11 +671,11 @@ template int launch_embed_bwd_cmp<64>(const DevModel &, const SysDesc &, int, co
                                       const float *, const int32_t *, const float *, const float *, float4 *, double *,
                                       cudaStream_t);
 
-int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, __half *gZ, double *energy,
-                      const int32_t *seg, cudaStream_t st) {
+int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, __half *gZ, int8_t *gexp,
+                      double *energy, const int32_t *seg, cudaStream_t st) {
   const int nb = g.b0[g.ntypes];
   if (nb == 0) return DPB_OK;
-  k_fit_energy<<<nb, 256, 0, st>>>(g, H, tl, Eatom, gZ, energy, seg);
+  k_fit_energy<<<nb, 256, 0, st>>>(g, H, tl, Eatom, gZ, gexp, energy, seg);
   count_launch();
   DPB_LAUNCH_CHECK();
   return DPB_OK;

@@ -8,8 +8,10 @@
 // multiply-add chains that they replace.
 //
 // Operand scales are powers of two: the weights' per layer, hidden activations'
-// and gates' from bounds known at model creation, the descriptor's per atom from
-// its largest entry (gmax, written with G), all divided out of the sum exactly.
+// from bounds known at model creation, the descriptor's per atom from its largest
+// entry (gmax, written with G), the gates' per atom and 32 columns from their largest
+// entry (a bound down all layers left wide deep nets 11 bits: force error 3.2e-6 of
+// the rms force at 1024^4, 5e-7 now), all divided out of the sum exactly.
 #include <type_traits>
 
 #include "internal.cuh"
@@ -77,7 +79,8 @@ __device__ __forceinline__ float row_scale(float x) {
 // (about 850 clocks, against the 520 of the MMAs).  98,304 atoms, all six GEMMs:
 // 1,880 us with every A split by the warps of the tile that needs it (13 times for
 // dE/dG), one group of adders, a division per row for the epilogue's addresses and
-// 8-way bank conflicts in A's loads; 1,330 us now (layer 0 622 -> 567).
+// 8-way bank conflicts in A's loads; 1,330 us without (layer 0 622 -> 567); the
+// gates' scales per row and chunk cost 27 us of it.
 constexpr int kGemmStages = 3;
 constexpr int kGemmThreads = 18 * 32;
 
@@ -126,18 +129,18 @@ __device__ __forceinline__ GemmTilePos gemm_tile(const GemmArgs &g, int tile) {
 __device__ __forceinline__ __half *gemm_tile_at(const Epi &ep, int mt, int lr, int n) {
   return ep.tile + gemm_operand_at((ep.ld + kGemmK - 1) / kGemmK, mt, lr, n);
 }
-__device__ __forceinline__ void gemm_tile_store4(const Epi &ep, int mt, int lr, int n, float4 v) {
+__device__ __forceinline__ void gemm_tile_store4(const Epi &ep, int mt, int lr, int n, float4 v, float scale) {
   __half *o = gemm_tile_at(ep, mt, lr, n);
-  const tc::f2 sc = tc::pk1(ep.tscale);
+  const tc::f2 sc = tc::pk1(scale);
   uint2 h, l;
   tc::split_pair(tc::mul2(tc::pk(v.x, v.y), sc), h.x, l.x);
   tc::split_pair(tc::mul2(tc::pk(v.z, v.w), sc), h.y, l.y);
   *reinterpret_cast<uint2 *>(o) = h;
   *reinterpret_cast<uint2 *>(o + kGemmPart) = l;
 }
-__device__ __forceinline__ void gemm_tile_store1(const Epi &ep, int mt, int lr, int n, float v) {
+__device__ __forceinline__ void gemm_tile_store1(const Epi &ep, int mt, int lr, int n, float v, float scale) {
   __half *o = gemm_tile_at(ep, mt, lr, n);
-  const float x = v * ep.tscale;
+  const float x = v * scale;
   const __half h = __float2half_rn(x);
   o[0] = h;
   o[kGemmPart] = __float2half_rn(x - __half2float(h));
@@ -173,24 +176,33 @@ __device__ __forceinline__ void gemm_epilogue(const GemmType &gt, const GemmTile
   const int warp = (threadIdx.x >> 5) & 7, lane = threadIdx.x & 31;
   const Epi &ep = gt.ep;
   const int n16 = (ep.ld + 15) / 16 * 16;  // the next GEMM reads whole K = 16 steps
+  const int nc = (ep.ld + kGemmK - 1) / kGemmK;
   if ((ep.ld & 3) != 0) {
     for (int lr = warp; lr < 128 && p.m0 + lr < gt.Mrows; lr += 8) {
       const size_t at = gt.rm.atom(p.m0 + lr) * (size_t)ep.ld + p.n0;
-      for (int j = lane; j < NW && p.n0 + j < n16; j += 32) {
+      for (int j = lane; j - lane < NW && p.n0 + j - lane < n16; j += 32) {  // a warp takes 32 columns, one scale
         const int n = p.n0 + j;
-        if (j >= p.nv) {
-          if (ep.tile) gemm_tile_store1(ep, p.mt, lr, n, 0.f);
-          continue;
-        }
-        const float *am = MODE == EPI_TANH_RES ? ep.hprev : ep.gmat;
-        const float a = GRAD && ep.gvec ? ep.gvec[n] : (MODE == EPI_TANH_RES || GRAD) && am ? am[at + j] : 0.f;
         float o1 = 0.f, o2 = 0.f;
-        gemm_epi1<MODE>(zs[lr * ZS + j] + bad, TANH ? ep.bias[n] : 0.f,
-                        MODE == EPI_TANH_RES || MODE == EPI_GRAD_RES ? ep.dt[n] : 1.f, a, GRAD ? ep.tin[at + j] : 0.f,
-                        o1, o2);
-        if (ep.out1) ep.out1[at + j] = o1;
-        if (MODE != EPI_STORE && MODE != EPI_GRAD && ep.out2) ep.out2[at + j] = o2;
-        if (MODE != EPI_STORE && ep.tile) gemm_tile_store1(ep, p.mt, lr, n, GRAD ? o1 : o2);
+        if (j < p.nv) {
+          const float *am = MODE == EPI_TANH_RES ? ep.hprev : ep.gmat;
+          const float a = GRAD && ep.gvec ? ep.gvec[n] : (MODE == EPI_TANH_RES || GRAD) && am ? am[at + j] : 0.f;
+          gemm_epi1<MODE>(zs[lr * ZS + j] + bad, TANH ? ep.bias[n] : 0.f,
+                          MODE == EPI_TANH_RES || MODE == EPI_GRAD_RES ? ep.dt[n] : 1.f, a, GRAD ? ep.tin[at + j] : 0.f,
+                          o1, o2);
+          if (ep.out1) ep.out1[at + j] = o1;
+          if (MODE != EPI_STORE && MODE != EPI_GRAD && ep.out2) ep.out2[at + j] = o2;
+        }
+        if (MODE == EPI_STORE || !ep.tile) continue;
+        float sc = ep.tscale;
+        if (GRAD) {
+          float m = fabsf(o1);
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+          const int k = gate_exp(m);
+          sc = pow2i(k);
+          if (lane == 0) ep.texp[gemm_exp_at(nc, p.mt, lr, n / kGemmK)] = (int8_t)k;
+        }
+        if (n < n16) gemm_tile_store1(ep, p.mt, lr, n, GRAD ? o1 : o2, sc);
       }
     }
     return;
@@ -225,23 +237,32 @@ __device__ __forceinline__ void gemm_epilogue(const GemmType &gt, const GemmTile
     for (int b = 0; b < RB; ++b) {
       const int r = q + b * RPW + rl, lr = 16 * warp + r;
       const size_t at = __shfl_sync(0xffffffffu, at_l, r) + j;
-      if (r >= nrow) continue;
-      if (pad) gemm_tile_store4(ep, p.mt, lr, p.n0 + j, zero);
-      if (!on) continue;
-      const float4 x = *reinterpret_cast<const float4 *>(zs + lr * ZS + j);
       float4 o1 = zero, o2 = zero;
-      gemm_epi1<MODE>(x.x + bad, bias.x, dt.x, a[b].x, t[b].x, o1.x, o2.x);
-      gemm_epi1<MODE>(x.y + bad, bias.y, dt.y, a[b].y, t[b].y, o1.y, o2.y);
-      gemm_epi1<MODE>(x.z + bad, bias.z, dt.z, a[b].z, t[b].z, o1.z, o2.z);
-      gemm_epi1<MODE>(x.w + bad, bias.w, dt.w, a[b].w, t[b].w, o1.w, o2.w);
-      if (ep.out1) *reinterpret_cast<float4 *>(ep.out1 + at) = o1;
-      if (MODE != EPI_STORE && MODE != EPI_GRAD && ep.out2) *reinterpret_cast<float4 *>(ep.out2 + at) = o2;
-      if (MODE != EPI_STORE && ep.tile) gemm_tile_store4(ep, p.mt, lr, p.n0 + j, GRAD ? o1 : o2);
+      if (on && r < nrow) {
+        const float4 x = *reinterpret_cast<const float4 *>(zs + lr * ZS + j);
+        gemm_epi1<MODE>(x.x + bad, bias.x, dt.x, a[b].x, t[b].x, o1.x, o2.x);
+        gemm_epi1<MODE>(x.y + bad, bias.y, dt.y, a[b].y, t[b].y, o1.y, o2.y);
+        gemm_epi1<MODE>(x.z + bad, bias.z, dt.z, a[b].z, t[b].z, o1.z, o2.z);
+        gemm_epi1<MODE>(x.w + bad, bias.w, dt.w, a[b].w, t[b].w, o1.w, o2.w);
+        if (ep.out1) *reinterpret_cast<float4 *>(ep.out1 + at) = o1;
+        if (MODE != EPI_STORE && MODE != EPI_GRAD && ep.out2) *reinterpret_cast<float4 *>(ep.out2 + at) = o2;
+      }
+      float sc = ep.tscale;
+      if (GRAD) {  // 8 lanes hold a row's 32 columns
+        float m = fmaxf(fmaxf(fabsf(o1.x), fabsf(o1.y)), fmaxf(fabsf(o1.z), fabsf(o1.w)));
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const int k = gate_exp(m);
+        sc = pow2i(k);
+        if ((lane & 7) == 0 && r < nrow && (on || pad)) ep.texp[gemm_exp_at(nc, p.mt, lr, (p.n0 + j) / kGemmK)] = (int8_t)k;
+      }
+      if (MODE != EPI_STORE && ep.tile && r < nrow && (on || pad))
+        gemm_tile_store4(ep, p.mt, lr, p.n0 + j, GRAD ? o1 : o2, sc);
     }
   }
 }
 
-template <int NW, bool TILED>
+template <int NW, bool TILED, bool GATES>
 __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_split(const __grid_constant__ GemmArgs g) {
   using C = GemmCfg<NW, TILED>;
   constexpr int ST = kGemmStages;
@@ -451,10 +472,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_split(const __grid_con
       tc::f2 acc[NW / 4];
 #pragma unroll
       for (int k = 0; k < NW / 4; ++k) acc[k] = tc::pk1(0.f);
+      // scale exponents of eight chunks (a load per chunk, which the arrivals on accfree
+      // wait for, made the six GEMMs of 98,304 atoms 10 % slower)
+      const int2 *aexp = GATES ? reinterpret_cast<const int2 *>(g.Aexp + gemm_exp_at(nc, p.mt, row, 0)) : nullptr;
+      int2 ew = GATES ? *aexp : make_int2(0, 0);
       // the other group has added all of the previous tile's sums: no stage's
       // barrier is more than one phase ahead of this group's wait
       if (EG == 2 && i > 0) ok = __all_sync(0xffffffffu, gemm_wait(&drained, (i - 1) & 1, abort));
       for (int c = 0; c < nc && ok; ++c, next()) {
+        if (GATES && c > 0) {
+          if ((c & 7) == 0) ew = aexp[c >> 3];
+          else if ((c & 3) == 0) ew.x = ew.y;
+          else ew.x >>= 8;
+        }
+        const float u = GATES ? pow2i(-(int)(int8_t)ew.x) : 1.f;
         ok = __all_sync(0xffffffffu, gemm_wait(&done[s], ph, abort));
         if (!ok) break;
         tc::fence_after_sync();
@@ -464,9 +495,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_split(const __grid_con
           tc::tmem_ld16_issue(tl + s * NW + q, r);
           tc::tmem_wait();
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            acc[q / 2 + k] =
-                tc::add2(acc[q / 2 + k], tc::pk(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1])));
+          for (int k = 0; k < 8; ++k) {
+            const tc::f2 x = tc::pk(__uint_as_float(r[2 * k]), __uint_as_float(r[2 * k + 1]));
+            acc[q / 2 + k] = GATES ? tc::fma2(x, tc::pk1(u), acc[q / 2 + k]) : tc::add2(acc[q / 2 + k], x);
+          }
         }
         tc::fence_before_sync();
         tc::mbar_arrive(&accfree[s]);
@@ -499,12 +531,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_split(const __grid_con
         ok = all != 0;
       }
       const float bad = ok ? 0.f : __int_as_float(0x7fffffff);  // a wait gave up: NaN results
-      switch (gt.ep.mode) {
-        case EPI_STORE: gemm_epilogue<NW, EPI_STORE>(gt, p, zs, bad); break;
-        case EPI_TANH: gemm_epilogue<NW, EPI_TANH>(gt, p, zs, bad); break;
-        case EPI_TANH_RES: gemm_epilogue<NW, EPI_TANH_RES>(gt, p, zs, bad); break;
-        case EPI_GRAD_RES: gemm_epilogue<NW, EPI_GRAD_RES>(gt, p, zs, bad); break;
-        case EPI_GRAD: gemm_epilogue<NW, EPI_GRAD>(gt, p, zs, bad); break;
+      if constexpr (GATES) {
+        if (gt.ep.mode == EPI_STORE) gemm_epilogue<NW, EPI_STORE>(gt, p, zs, bad);
+        else if (gt.ep.mode == EPI_GRAD_RES) gemm_epilogue<NW, EPI_GRAD_RES>(gt, p, zs, bad);
+        else gemm_epilogue<NW, EPI_GRAD>(gt, p, zs, bad);
+      } else {
+        if (gt.ep.mode == EPI_TANH) gemm_epilogue<NW, EPI_TANH>(gt, p, zs, bad);
+        else gemm_epilogue<NW, EPI_TANH_RES>(gt, p, zs, bad);
       }
       // zs is free again; and every thread of the group has arrived on drained and
       // zfree before one of them waits there for a later phase
@@ -517,12 +550,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_split(const __grid_con
   if (warp == 0) tc::tmem_dealloc(tbase, C::TM);
 }
 
-template <int NW, bool TILED>
+template <int NW, bool TILED, bool GATES>
 static int launch_gemm_m(const GemmArgs &g, int nsm, cudaStream_t st) {
   const int smem = GemmCfg<NW, TILED>::SMEM;
-  DPB_CUDA_TRY(cudaFuncSetAttribute(k_gemm_split<NW, TILED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  DPB_CUDA_TRY(cudaFuncSetAttribute(k_gemm_split<NW, TILED, GATES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   const int ntile = (g.N + NW - 1) / NW * g.mt0[g.ntypes];
-  k_gemm_split<NW, TILED><<<ntile < nsm ? ntile : nsm, kGemmThreads, smem, st>>>(g);
+  k_gemm_split<NW, TILED, GATES><<<ntile < nsm ? ntile : nsm, kGemmThreads, smem, st>>>(g);
   count_launch();
   DPB_LAUNCH_CHECK();
   return DPB_OK;
@@ -530,9 +563,11 @@ static int launch_gemm_m(const GemmArgs &g, int nsm, cudaStream_t st) {
 
 template <int NW>
 static int launch_gemm_w(const GemmArgs &g, int nsm, cudaStream_t st) {
-  return g.At ? launch_gemm_m<NW, true>(g, nsm, st) : launch_gemm_m<NW, false>(g, nsm, st);
+  if (!g.At) return launch_gemm_m<NW, false, false>(g, nsm, st);
+  return g.Aexp ? launch_gemm_m<NW, true, true>(g, nsm, st) : launch_gemm_m<NW, true, false>(g, nsm, st);
 }
 
+size_t gemm_exp_bytes(size_t rows, int K) { return rows * (((K + kGemmK - 1) / kGemmK + 7) & ~7); }
 size_t gemm_operand_halves(int mt, int K) { return (size_t)mt * ((K + kGemmK - 1) / kGemmK) * (2 * kGemmPart); }
 
 // Every centre type in one launch (g.t, g.mt0 filled).  128 columns per CTA keep
