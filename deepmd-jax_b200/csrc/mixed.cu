@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kFwdThreads, 2) k_mix_embed_fwd(DevModel M, Sy
                                                                   int *__restrict__ err) {
   using MD = MixDims<E0, E1, E2>;
   using SP = HalfSplit<E0, E1, E2>;
-  extern __shared__ __align__(1024) char smem[];
+  extern __shared__ __align__(128) char smem[];
   char *netb = smem;
   float *small = reinterpret_cast<float *>(netb + round1k(MD::NETB));
   char *opa = reinterpret_cast<char *>(small) + round1k(MD::NSMALL * 4);
@@ -957,7 +957,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
   using MD = MixDims<E0, E1, E2>;
   using SP = HalfSplit<E0, E1, E2>;
   constexpr int DTB_BYTES = kDtbRows * MD::N2 * 2;
-  extern __shared__ __align__(1024) char smem[];
+  extern __shared__ __align__(128) char smem[];
   char *netb = smem;
   float *small = reinterpret_cast<float *>(netb + round1k(MD::NETB));
   char *dtb = reinterpret_cast<char *>(small) + round1k(MD::NSMALL * 4);
@@ -1333,9 +1333,20 @@ struct FitCfg {
   static constexpr int RA = HAB > 3 * STAGEA ? HAB : 3 * STAGEA;  // activations, and layer 0's A ring
   static constexpr int NA = RA / STAGEA < 8 ? RA / STAGEA : 8;
   static constexpr int ST = DEEP ? (FW > 240 ? 4 : 5) : (FW > 240 ? 2 : 3);
-  // biases and dt of every layer, output weights
-  static size_t smem(int L) { return (size_t)RA + (size_t)ST * STAGE + (size_t)(2 * L + 1) * FW * 4; }
-  static_assert(RA + ST * STAGE + (2 * kMaxFitLayers + 1) * FW * 4 <= 226 * 1024, "fitting ring");
+  // biases of the L layers, dt of layers 1 .. L - 1 (of layer 0 for L = 1), output
+  // weights, and the energies that one half of the epilogue hands to the other:
+  // these in the biases of layer 0, which are done with then, where they fit
+  static __host__ __device__ constexpr int dt_at(int L, int l) { return (L + (L > 1 ? l - 1 : l)) * FW; }
+  static __host__ __device__ constexpr int wout_at(int L) { return (L + (L > 1 ? L - 1 : 1)) * FW; }
+  static __host__ __device__ constexpr int esum_at(int L) { return L > 1 && FW >= 128 ? 0 : wout_at(L) + FW; }
+  static __host__ __device__ constexpr size_t smem(int L) {
+    return (size_t)RA + (size_t)ST * STAGE + (size_t)(wout_at(L) + FW + (esum_at(L) ? 128 : 0)) * 4;
+  }
+  static constexpr int STATIC = 256;  // barriers, TMEM address, flag
+  static_assert((2 * ST + 2 * NA + 6) * 8 + 8 <= STATIC, "static shared memory");
+  // 1 KB of every CTA is the system's
+  static_assert((DEEP ? 1 : 2) * (smem(kMaxFitLayers) + STATIC + 1024) <= 228 * 1024, "CTAs per SM at every depth");
+  static_assert(smem(kMaxFitLayers) + STATIC <= 227 * 1024, "fitting ring");
 };
 
 // Bounded mbarrier wait that also gives up once another role of the CTA gave
@@ -1412,16 +1423,18 @@ __global__ void __launch_bounds__(kFitThreads, DEEP ? 1 : 2) k_mix_fit(DevModel 
   using C = FitCfg<FW, DEEP>;
   constexpr int ST = C::ST, KC = C::KC, NA = C::NA;
   static_assert(FW % 16 == 0 && FW <= 256, "fit width");
-  extern __shared__ __align__(1024) char smem[];
+  // (an alignment of 1 KB here or in another kernel of this file would round every
+  // kernel's static part up to it)
+  extern __shared__ __align__(128) char smem[];
   char *HA = smem;              // 128 x FW fp16, K-major (kmajor_off); during layer 0 its A ring
   char *ring = smem + C::RA;    // ST stages
-  float *cst = reinterpret_cast<float *>(ring + ST * C::STAGE);  // bias[l], dt[l], w_out
+  float *cst = reinterpret_cast<float *>(ring + ST * C::STAGE);  // bias[l], dt[l], w_out, energies
   __shared__ __align__(8) uint64_t full[ST], empty[ST], fullA[NA], emptyA[NA], accf, accfD[2], epid, accfree[2];
   __shared__ uint32_t tbase_s;
   __shared__ int abort_s;
-  __shared__ float esum_s[128];  // the second half's energy partial per atom
   const int tid = threadIdx.x, warp = tc::warp_index();
   const int L = M.nfit, K0 = M.A * M.E2;
+  float *esum_s = cst + C::esum_at(L);  // the second half's energy partial per atom
   const int NG = 2 * L - 1 + (K0 + kFitDgN - 1) / kFitDgN;
   volatile int *abort = &abort_s;
   if (tid == 0) {
@@ -1461,9 +1474,9 @@ __global__ void __launch_bounds__(kFitThreads, DEEP ? 1 : 2) k_mix_fit(DevModel 
     for (int l = 0; l < kMaxFitLayers; ++l)
       if (l < L) {
         cst[l * FW + tid] = v[2 * l];
-        cst[(L + l) * FW + tid] = v[2 * l + 1];
+        if (l > 0 || L == 1) cst[C::dt_at(L, l) + tid] = v[2 * l + 1];
       }
-    cst[2 * L * FW + tid] = v[2 * kMaxFitLayers];
+    cst[C::wout_at(L) + tid] = v[2 * kMaxFitLayers];
   }
   if (warp == 0) tc::tmem_alloc(&tbase_s, 256);
   tc::fence_before_sync();
@@ -1650,7 +1663,8 @@ __global__ void __launch_bounds__(kFitThreads, DEEP ? 1 : 2) k_mix_fit(DevModel 
       // after next as soon as it is used
       const bool res = dt != nullptr;
       const int hs = res && !M.mfdt[ti][l - 1] ? l - 1 : L + l - 1;  // the layer below's output
-      const float *cb_ = cst + l * FW, *cd_ = cst + (L + l) * FW, *cw_ = cst + 2 * L * FW;
+      // (layer 0 of several has no dt: it reads there what it does not use)
+      const float *cb_ = cst + l * FW, *cd_ = cst + C::dt_at(L, l), *cw_ = cst + C::wout_at(L);
       float hp[2][8];
 #pragma unroll
       for (int q = 0; q < 2; ++q)
@@ -1734,7 +1748,7 @@ __global__ void __launch_bounds__(kFitThreads, DEEP ? 1 : 2) k_mix_fit(DevModel 
       const bool use_gh = res_l && l != L - 1;
       const float usc = 1.f / (M.fit_wsc[ti][l] * M.fit_gsc[ti][l]), gsc = M.fit_gsc[ti][l - 1];
       // dt of layer l - 1 (1 without residual), output weights
-      const float *cd_ = cst + (L + l - 1) * FW, *cw_ = cst + 2 * L * FW;
+      const float *cd_ = cst + C::dt_at(L, l - 1), *cw_ = cst + C::wout_at(L);
       float ghc[2][8], tcur[2][8];
 #pragma unroll
       for (int q = 0; q < 2; ++q)
