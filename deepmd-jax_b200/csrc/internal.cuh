@@ -5,6 +5,21 @@
 #include <cmath>
 #include <vector>
 
+namespace dpb {
+// The mixed fitting kernel's deep weight ring (1, one CTA per SM) or its shallow
+// one (0, two), as timed for launches of this many 128-row tiles; every other
+// launch, and all of them at -1, take the rule on sizes.
+struct FitShape {
+  int deep = -1, tiles = 0;
+};
+// The 128-row tiles of the fitting over all centre types.
+inline int fit_tiles(int ntypes, const int *type_count, int nframes) {
+  int n = 0;
+  for (int t = 0; t < ntypes; ++t) n += (type_count[t] * nframes + 127) / 128;
+  return n;
+}
+}  // namespace dpb
+
 struct dpb_model {
   dpb::DevModel dm;
   std::vector<void *> allocs;
@@ -14,10 +29,9 @@ struct dpb_model {
   int device;
   // launch shapes chosen by dpb_md_autotune (they never change results):
   // atoms (warps) per block of the mixed dE/dT kernel, and the mixed fitting
-  // kernel's deep weight ring (1 CTA per SM) instead of the shallow one (2
-  // CTAs per SM)
+  // kernel's shape
   mutable int dT_warps = 4;
-  mutable int fit_deep = 0;
+  mutable dpb::FitShape fit;
 };
 
 namespace dpb {

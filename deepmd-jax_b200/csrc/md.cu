@@ -1622,11 +1622,13 @@ extern "C" int dpb_md_autotune(dpb_md *m, int *nl_warps, int *dT_warps, int *fit
   }
   // mixed form: the fitting kernel's shallow (2 CTAs per SM) or deep (1 CTA
   // per SM) weight ring, timed over whole evaluations of the current state
+  FitShape &fit = m->model->fit;
   if (!rc && m->d.precision == DPB_PREC_MIXED) {
-    int bestd = m->model->fit_deep;
+    int bestd = -1;
+    fit.tiles = fit_tiles(m->ntypes, m->type_count, m->P);
     tbest = 1e30f;
     for (int deep = 0; deep < 2 && !rc; ++deep) {
-      m->model->fit_deep = deep;
+      fit.deep = deep;
       int r = md_forces(m, st);  // warm-up
       cudaEventRecord(a, st);
       for (int k = 0; k < 3 && !r; ++k) r = md_forces(m, st);
@@ -1637,7 +1639,7 @@ extern "C" int dpb_md_autotune(dpb_md *m, int *nl_warps, int *dT_warps, int *fit
       if (r) rc = r;
       else if (ms < tbest) { tbest = ms; bestd = deep; }
     }
-    m->model->fit_deep = bestd;
+    fit.deep = rc ? -1 : bestd;
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
@@ -1646,7 +1648,7 @@ extern "C" int dpb_md_autotune(dpb_md *m, int *nl_warps, int *dT_warps, int *fit
   if (!rc && cudaStreamSynchronize(st) != cudaSuccess) rc = DPB_ERR_CUDA;
   if (nl_warps) *nl_warps = m->nl_warps;
   if (dT_warps) *dT_warps = m->model->dT_warps;
-  if (fit_stages) *fit_stages = m->d.precision == DPB_PREC_MIXED ? (m->model->fit_deep ? 12 : 4) : 0;
+  if (fit_stages) *fit_stages = m->d.precision == DPB_PREC_MIXED ? (fit.deep > 0 ? 12 : 4) : 0;
   return rc;
 }
 

@@ -1333,6 +1333,10 @@ struct FitCfg {
   static constexpr int RA = HAB > 3 * STAGEA ? HAB : 3 * STAGEA;  // activations, and layer 0's A ring
   static constexpr int NA = RA / STAGEA < 8 ? RA / STAGEA : 8;
   static constexpr int ST = DEEP ? (FW > 240 ? 4 : 5) : (FW > 240 ? 2 : 3);
+  // time of two tiles that share an SM over that of one that has it to itself, in
+  // eighths: 1.53 to 1.78 measured for widths 64 and 128 (K0 400 to 1600, one to three
+  // layers), 1.72 to 1.93 for 208 to 256 (one to four)
+  static constexpr int PAIR8 = FW <= 128 ? 13 : 15;
   // biases of the L layers, dt of layers 1 .. L - 1 (of layer 0 for L = 1), output
   // weights, and the energies that one half of the epilogue hands to the other:
   // these in the biases of layer 0, which are done with then, where they fit
@@ -1886,27 +1890,28 @@ int launch_mix_fit(const DevModel &M, const SysDesc &D, const __half *Gb, DGT *d
 // The instantiation of the model's padded hidden width and ring depth.
 template <int FW, typename DGT>
 static int launch_mix_fit_d(const DevModel &M, const SysDesc &D, const __half *Gb, DGT *dG, float *scratch,
-                            float *Eatom, double *energy, int *err, bool deep, cudaStream_t st) {
-  // two tiles that share an SM take 5/3 of one that has it to itself (138 us and
-  // 83 us at width 240, K0 = 1600), so the shape with fewer such units in its
-  // whole waves is taken
-  int tiles = 0;
-  for (int ti = 0; ti < M.ntypes; ++ti) tiles += ((D.offs[ti + 1] - D.offs[ti]) * D.F + 127) / 128;
-  const int sms = num_sms();
-  deep = deep || 3 * ((tiles + sms - 1) / sms) < 5 * ((tiles + 2 * sms - 1) / (2 * sms));
+                            float *Eatom, double *energy, int *err, FitShape shape, cudaStream_t st) {
+  // unless timed for this many tiles, the shape whose whole waves take less
+  int cnt[kMaxTypes];
+  for (int ti = 0; ti < M.ntypes; ++ti) cnt[ti] = D.offs[ti + 1] - D.offs[ti];
+  const int tiles = fit_tiles(M.ntypes, cnt, D.F), sms = num_sms();
+  const bool deep = shape.deep >= 0 && shape.tiles == tiles
+                        ? shape.deep != 0
+                        : 8 * ((tiles + sms - 1) / sms) <
+                              FitCfg<FW, false>::PAIR8 * ((tiles + 2 * sms - 1) / (2 * sms));
   return deep ? launch_mix_fit<FW, DGT, true>(M, D, Gb, dG, scratch, Eatom, energy, err, st)
               : launch_mix_fit<FW, DGT, false>(M, D, Gb, dG, scratch, Eatom, energy, err, st);
 }
 
 template <typename DGT>
 int launch_mix_fit_any(const DevModel &M, const SysDesc &D, const __half *Gb, DGT *dG, float *scratch,
-                       float *Eatom, double *energy, int *err, bool deep, cudaStream_t st) {
+                       float *Eatom, double *energy, int *err, FitShape shape, cudaStream_t st) {
   switch (M.mfw) {
-    case 64: return launch_mix_fit_d<64, DGT>(M, D, Gb, dG, scratch, Eatom, energy, err, deep, st);
-    case 128: return launch_mix_fit_d<128, DGT>(M, D, Gb, dG, scratch, Eatom, energy, err, deep, st);
-    case 208: return launch_mix_fit_d<208, DGT>(M, D, Gb, dG, scratch, Eatom, energy, err, deep, st);
-    case 240: return launch_mix_fit_d<240, DGT>(M, D, Gb, dG, scratch, Eatom, energy, err, deep, st);
-    case 256: return launch_mix_fit_d<256, DGT>(M, D, Gb, dG, scratch, Eatom, energy, err, deep, st);
+    case 64: return launch_mix_fit_d<64, DGT>(M, D, Gb, dG, scratch, Eatom, energy, err, shape, st);
+    case 128: return launch_mix_fit_d<128, DGT>(M, D, Gb, dG, scratch, Eatom, energy, err, shape, st);
+    case 208: return launch_mix_fit_d<208, DGT>(M, D, Gb, dG, scratch, Eatom, energy, err, shape, st);
+    case 240: return launch_mix_fit_d<240, DGT>(M, D, Gb, dG, scratch, Eatom, energy, err, shape, st);
+    case 256: return launch_mix_fit_d<256, DGT>(M, D, Gb, dG, scratch, Eatom, energy, err, shape, st);
     default: return DPB_ERR_UNSUPPORTED;
   }
 }
@@ -2031,7 +2036,7 @@ int launch_embed_bwd_gen(const DevModel &, const SysDesc &, int, const float *, 
 static int mixed_eval_compressed(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm,
                                  const float *box, const int32_t *nbrs, double *energy, float *Eatom, float4 *F4,
                                  double *virial, float *T, __half *Gb, float *dG, float *scratch, int *err,
-                                 bool fit_deep, cudaStream_t st) {
+                                 FitShape fit, cudaStream_t st) {
   const size_t NF = (size_t)D.N * D.F;
   const size_t NG = NF * M.A * M.E2;  // a multiple of 16 (mixed_supported)
   int rc;
@@ -2048,7 +2053,7 @@ static int mixed_eval_compressed(const DevModel &M, const SysDesc &D, const floa
   DPB_LAUNCH_CHECK();
   prof_end(PROF_EMBED_FWD, st);
   prof_begin(PROF_MIXED_FIT, st);
-  rc = launch_mix_fit_any<float>(M, D, Gb, dG, scratch, Eatom, energy, err, fit_deep, st);
+  rc = launch_mix_fit_any<float>(M, D, Gb, dG, scratch, Eatom, energy, err, fit, st);
   prof_end(PROF_MIXED_FIT, st);
   if (rc) return rc;
   prof_begin(PROF_EMBED_BWD, st);
@@ -2142,7 +2147,7 @@ int *mixed_err(const DevModel &M, size_t NF, void *ws) { return mixed_ws(M, NF, 
 
 int mixed_eval(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm, const float *box,
                const int32_t *nbrs, double *energy, float *Eatom, float4 *F4, double *virial, void *ws,
-               cudaStream_t st, int dT_warps, bool fit_deep) {
+               cudaStream_t st, int dT_warps, FitShape fit) {
   const size_t NF = (size_t)D.N * D.F;
   const MixedWs mw = mixed_ws(M, NF, ws);
   int *err = mw.err;
@@ -2151,14 +2156,14 @@ int mixed_eval(const DevModel &M, const SysDesc &D, const float *pos, const int3
   float4 *posS = mw.posS;
   if (M.ngrids > 0 || !M.emb_tuned)
     return mixed_eval_compressed(M, D, pos, perm, box, nbrs, energy, Eatom, F4, virial, T, Gb, dG, scratch, err,
-                                 fit_deep, st);
+                                 fit, st);
   int rc = launch_pos_sorted(D, pos, perm, posS, st);
   if (rc) return rc;
   rc = mixed_descriptors(M, D, posS, box, nbrs, T, Gb, mw.rows, mw.rcnt, err, st);
   if (rc) return rc;
   prof_begin(PROF_MIXED_FIT, st);
   __half *dGb = reinterpret_cast<__half *>(dG);  // dE/dG in FP16 times fit_dgsc (the dE/dT input)
-  rc = launch_mix_fit_any<__half>(M, D, Gb, dGb, scratch, Eatom, energy, err, fit_deep, st);
+  rc = launch_mix_fit_any<__half>(M, D, Gb, dGb, scratch, Eatom, energy, err, fit, st);
   prof_end(PROF_MIXED_FIT, st);
   if (rc) return rc;
   prof_begin(PROF_MIXED_DT, st);

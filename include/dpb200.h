@@ -330,11 +330,11 @@ DPB_API int dpb_md_device_pointers(dpb_md *md, dpb_md_pointers_t *ptrs);
  * launch shapes to XLA): times the neighbour search at 4 / 8 / 16 centres
  * per block and, for the mixed form, dE/dT at 2 / 4 / 8 atoms per block and
  * the tensor-core fitting kernel with its shallow weight ring (reported as 4;
- * 2 CTAs per SM unless the tiles are too few for that) and its deep one
- * (reported as 12; 1 CTA per SM), timed over whole evaluations, on this
- * engine's current state, and keeps the fastest
+ * 2 CTAs per SM) and its deep one (reported as 12; 1 CTA per SM), timed over
+ * whole evaluations, on this engine's current state, and keeps the fastest
  * (*nl_warps, *dT_warps and *fit_stages report the choice; *fit_stages is 0
- * for the FP32 form; the dE/dT and ring choices are stored on the model).
+ * for the FP32 form; the dE/dT choice is stored on the model, the ring's with
+ * the number of 128-atom tiles that it was timed for).
  * Results do not depend on the shapes.  Call after dpb_md_init and before
  * capturing dpb_md_run into a graph; ends with the list and forces of the
  * current positions. */
