@@ -1953,12 +1953,17 @@ size_t mixed_workspace_per_atom(const DevModel &M) {
 template <int E2, int N2, int W>
 static void launch_mix_dT_s(const DevModel &M, size_t NF, const float *T, const __half *dGb, __half *dTh,
                             float *dTs, cudaStream_t st) {
-  // warp-strided atoms, 12 warps per SM (what its registers hold): a warp zeroes
-  // its tiles once and loads one atom ahead (more blocks than are resident, so two
-  // or three atoms per warp: 280 us for 98,304 atoms, 261 us now)
-  const size_t cap = (size_t)num_sms() * (W < 12 ? 12 / W : 1);
-  const unsigned grid = (unsigned)std::min((NF + W - 1) / W, cap);
-  const int smem = W * DtCfg<E2, N2>::WARP_BYTES;
+  // warp-strided atoms, as many blocks as the SMs hold: a warp zeroes its tiles once
+  // and loads one atom ahead (more blocks than are resident, so two or three atoms
+  // per warp: 280 us for 98,304 atoms at W = 4, 261 us now)
+  constexpr int smem = W * DtCfg<E2, N2>::WARP_BYTES;
+  static const int per_sm = [] {  // registers are given to warps in units of 256, on four schedulers of 16,384
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, k_mix_dT<E2, N2, W>) != cudaSuccess) return 1;
+    const int warps = 4 * (16384 / ((fa.numRegs + 7) / 8 * 256));
+    return std::max(1, std::min({warps / W, 64 / W, 228 * 1024 / (smem + 1024)}));
+  }();
+  const unsigned grid = (unsigned)std::min((NF + W - 1) / W, (size_t)num_sms() * per_sm);
   cudaFuncSetAttribute(k_mix_dT<E2, N2, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   k_mix_dT<E2, N2, W><<<grid, 32 * W, smem, st>>>(M, (int)NF, T, dGb, dTh, dTs);
   count_launch();

@@ -1,6 +1,6 @@
 """dpb_md_autotune times the shapes that it names: with fewer fitting tiles than SMs
 (12,288 atoms, 96 tiles) both weight rings run, and the one that it reports is the one
-that later steps launch."""
+that later steps launch; the dE/dT candidates fill the SMs."""
 import json
 
 import pytest
@@ -45,3 +45,19 @@ def test_both_rings_are_timed_and_the_choice_runs(tuned):
     assert sorted(ring.values()) == [False, True]
     ran = [("true>" in n) for n, _ in after if "k_mix_fit" in n]
     assert ran and all(deep == (shapes["fit_ring_stages"] == 12) for deep in ran)
+
+
+def test_dT_candidates_fill_the_sms(tuned):
+    """Every dE/dT candidate launches as many blocks as its registers and shared memory let an SM hold."""
+    shapes, during, _ = tuned
+    grids = {}
+    for name, a in during:
+        if "k_mix_dT<" in name:
+            warps = a["block"][0] // 32
+            by_regs = 4 * (16384 // (-(-a["registers per thread"] // 8) * 256)) // warps
+            grids[warps] = (a["grid"][0], min(by_regs, 64 // warps, 228 * 1024 // (a["shared memory"] + 1024)))
+    print(grids)
+    assert sorted(grids) == [2, 4, 8]
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for warps, (grid, per_sm) in grids.items():
+        assert grid == min(-(-12288 // warps), sms * per_sm)
