@@ -258,7 +258,8 @@ extern "C" int dpb_model_create(const dpb_model_desc *d, dpb_model **out) {
       rc = upload(m, d->embed_kernel[k * ne + l], (size_t)ew_in[l] * ew_out[l], &M.ew[k][l]);
       if (rc == DPB_OK) rc = upload(m, d->embed_bias[k * ne + l], (size_t)ew_out[l], &M.eb[k][l]);
     }
-  // shared-memory images of the embedding nets for the tensor-core kernels:
+  // shared-memory images of the embedding nets for the tensor-core kernels (which
+  // a tabulated model does not run, although it may come with its nets):
   // FP16 B tiles (K-major) of layers 1 and 2 with the layer's bias as one
   // more K row (the A operands carry a ones column there), and the FP32 first
   // layer (w0, b0 in FP32) (mixed.cu, MixDims)
@@ -268,7 +269,7 @@ extern "C" int dpb_model_create(const dpb_model_desc *d, dpb_model **out) {
     const int W1B = N1 * K1 * 2, W2B = N2 * K2 * 2;
     M.net_img_bytes = W1B + W2B;
     M.net_small_floats = (2 * M.E0 + 3) / 4 * 4;
-    for (int k = 0; k < nt * nt && rc == DPB_OK && have_mlp && M.emb_tuned; ++k) {
+    for (int k = 0; k < nt * nt && rc == DPB_OK && have_mlp && M.emb_tuned && M.ngrids == 0; ++k) {
       std::vector<uint8_t> img(M.net_img_bytes, 0);
       const float *W1 = d->embed_kernel[k * 3 + 1], *W2 = d->embed_kernel[k * 3 + 2];
       const float *b1 = d->embed_bias[k * 3 + 1], *b2 = d->embed_bias[k * 3 + 2];
