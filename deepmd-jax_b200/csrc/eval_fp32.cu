@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(256) k_embed_fwd(DevModel M, SysDesc D, int ti
                                                    const int32_t *__restrict__ perm, const float *__restrict__ box,
                                                    const int32_t *__restrict__ nbrs, float *__restrict__ Tout,
                                                    float *__restrict__ Gout, float *__restrict__ gmax) {
-  extern __shared__ float smem[];
+  extern __shared__ __align__(16) float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   float *rowbuf = smem + warp * embed_fwd_warp_floats<E2>();
   float *Ts = rowbuf + 64 * 12;
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(256, 2) k_embed_bwd(DevModel M, SysDesc D, int
                                                    const float *__restrict__ dG, float4 *__restrict__ F4,
                                                    double *__restrict__ virial) {
   constexpr int NQ = (E2 + 31) / 32;
-  extern __shared__ float smem[];
+  extern __shared__ __align__(16) float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const int A = M.A;
   constexpr int AS = E2 + 1, BS = E2 + 4;  // row strides: dot products along rows without bank conflicts
