@@ -1,6 +1,6 @@
 #!/usr/bin/env python
 """Benchmark: MD throughput (atom-steps/s) of 98,304-atom water NVE on one
-B200, BF16/FP32 mixed form beside the plain FP32 form.
+B200, FP16/FP32 mixed form beside the FP32 form.
 
   python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference]
 

@@ -186,9 +186,10 @@ __device__ __forceinline__ uint4 pack8h(const float *v, float s) {
 
 // ---------------------------------------------------------------- embedding rows in packed FP16
 // The per-row epilogues of both embedding kernels work on pairs of adjacent
-// columns packed in one register (__half2): tanh.approx.f16x2 (one MUFU
-// operation per two columns), HADD2 for the residual, HFMA2 for the tangent
-// (1 - t^2) dz + d_prev of the adjoint's forward-mode recompute.  A pair
+// columns packed in one register (__half2): tanh in FP32 (one MUFU operation
+// per column) rounded to FP16, HADD2 for the residual, HFMA2 for the tangent
+// (1 - t^2) dz + d_prev of the adjoint's forward-mode recompute, 1 - t^2 from the
+// FP32 tanh.  A pair
 // (c, c + 1) with c even; its residual source (utils.py:115-123, x_prev =
 // repeat(x, Z)) is the pair (c, c + 1) of the layer below when Z = 1 and
 // column c / 2, broadcast to both halves, when Z = 2.

@@ -48,8 +48,20 @@ extern "C" {
 #define DPB_ERR_SCRATCH_LIMIT 261
 
 /* Precision of the evaluation.
- * DPB_PREC_FP32:  all arithmetic in FP32 (the reference's float32 with
- *                 jax_default_matmul_precision='float32', deepmd_jax/__init__.py:10).
+ * DPB_PREC_FP32:  FP32 accuracy (the reference's float32 with
+ *                 jax_default_matmul_precision='float32', deepmd_jax/__init__.py:10):
+ *                 inputs, weights, activations, sums and results are FP32, and
+ *                 matrix products run on the tensor cores with each operand as
+ *                 the sum of two FP16 parts (22 significant bits; fitting weights
+ *                 three parts, 33 bits), products added in FP32.  The 22 bits hold
+ *                 for embedding activations above 1/8 in magnitude (below it
+ *                 their error is 3e-8 absolute), for fitting activations above
+ *                 2^-17 of their bound (at most one per layer where |dt| <= 1), and for
+ *                 descriptor entries and adjoint gates above 2^-17 of the largest
+ *                 of their atom (gates: of its 32 columns).  Displacements are the
+ *                 nearest image d - L rint(d / L) in boxes wider than 2 rcut.
+ *                 Tabulated nets and embedding shapes other than 25-50-100 and
+ *                 32-32-64 run in FP32 multiply-adds up to the descriptor.
  * DPB_PREC_MIXED: embedding/fitting contractions in FP16 on the tensor cores
  *                 with FP32 accumulation; s(r), env matrix, first embedding
  *                 layer, per-atom energies and forces in FP32. */
