@@ -102,7 +102,7 @@ int mixed_descriptors_f32(const DevModel &M, const SysDesc &D, const float *pos,
                           const float *box, const int32_t *nbrs, float *T, float *G, int *err, void *ws,
                           cudaStream_t st);
 int fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Eatom, double *energy, char *w,
-                   cudaStream_t st);
+                   int *err, cudaStream_t st);
 }  // namespace dpb
 
 using namespace dpb;
@@ -481,7 +481,7 @@ static int fill_sys(const dpb_model *m, int natoms, int nframes, const int *type
 // scale of layer 0's operand).  w: scratch for the per-layer activations and
 // adjoints.
 int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Eatom, double *energy, char *w,
-                        cudaStream_t st) {
+                        int *err, cudaStream_t st) {
   const size_t NF = (size_t)D.N * D.F;
   const int E2 = M.E2, A = M.A, K0 = A * E2, L = M.nfit, FWM = fit_width_max(M);
   float *tb[kMaxFitLayers], *hb[kMaxFitLayers];
@@ -498,6 +498,7 @@ int dpb::fit_fp32_chain(const DevModel &M, const SysDesc &D, float *G, float *Ea
   int8_t *ex[2] = {nullptr, nullptr};  // scale exponents of the gates in op[]
   GemmArgs g{};
   EnergyArgs en{};
+  g.err = err;
   int ty[kMaxTypes], n = 0;  // the types present
   for (int ti = 0; ti < M.ntypes; ++ti) {
     const int cnt = D.offs[ti + 1] - D.offs[ti];
@@ -660,7 +661,7 @@ static int eval_fp32(const DevModel &M, const SysDesc &D, const float *pos, cons
   if (rc) return rc;
   prof_end(PROF_EMBED_FWD, st);
   prof_begin(PROF_FIT, st);
-  rc = fit_fp32_chain(M, D, G, Eatom, energy, w, st);
+  rc = fit_fp32_chain(M, D, G, Eatom, energy, w, err, st);
   if (rc) return rc;
   prof_end(PROF_FIT, st);
   prof_begin(PROF_EMBED_BWD, st);

@@ -179,6 +179,7 @@ struct GemmArgs {
   const int8_t *Aexp;   // with At: the tiles' scale exponents (gemm_exp_at), or NULL: 0
   int lda, K, N, ntypes;
   int mt0[kMaxTypes + 1];  // first 128-row tile of each type
+  int *err;                // set when a wait gave up
   GemmType t[kMaxTypes];
 };
 

@@ -547,6 +547,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) k_gemm_split(const __grid_con
   }
   tc::fence_before_sync();
   __syncthreads();
+  if (tid == 0 && abort_s) atomicOr(g.err, 1);  // a wait gave up (k_finalize)
   if (warp == 0) tc::tmem_dealloc(tbase, C::TM);
 }
 
