@@ -65,14 +65,14 @@ int split_embed_fwd(const DevModel &M, const SysDesc &D, int ba, const float4 *p
                     const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, float *G, float *gmax, int *err,
                     cudaStream_t st);
 int split_embed_bwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
-                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, const float *dG, float4 *F4,
+                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, const float *dG, ForceSum *F4,
                     double *virial, int *err, cudaStream_t st);
 template <int E2>
 int launch_embed_fwd_cmp(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
                          const int32_t *, float *, float *, float *, cudaStream_t);
 template <int E2>
 int launch_embed_bwd_cmp(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
-                         const int32_t *, const float *, const float *, float4 *, double *, cudaStream_t);
+                         const int32_t *, const float *, const float *, ForceSum *, double *, cudaStream_t);
 // fitting GEMMs on the tensor cores (gemm_split.cu)
 size_t gemm_tiles_halves(int N, int K);
 size_t gemm_operand_halves(int mt, int K);
@@ -83,12 +83,12 @@ int launch_gemm_split(const GemmArgs &g, cudaStream_t st);
 int launch_embed_fwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
                          const int32_t *, float *, float *, float *, cudaStream_t);
 int launch_embed_bwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
-                         const int32_t *, const float *, const float *, float4 *, double *, cudaStream_t);
+                         const int32_t *, const float *, const float *, ForceSum *, double *, cudaStream_t);
 int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, __half *gZ, int8_t *gexp,
                       double *energy, const int32_t *seg, cudaStream_t st);
-int launch_eval_begin(size_t NF, float4 *F4, size_t nE, double *energy, double *virial, int *err, cudaStream_t st);
+int launch_eval_begin(size_t NF, ForceSum *F4, size_t nE, double *energy, double *virial, int *err, cudaStream_t st);
 int *mixed_err(const DevModel &M, size_t NF, void *ws);
-int launch_finalize(int, int, const float4 *, float *, const float *, const int32_t *, float *, double *, int,
+int launch_finalize(int, int, const ForceSum *, float *, const float *, const int32_t *, float *, double *, int,
                     const float *, const int32_t *, const int *, uint32_t *, cudaStream_t);
 // mixed path (mixed.cu)
 int mixed_supported(const DevModel &M);
@@ -96,7 +96,7 @@ int mixed_fit_width(const DevModel &M);
 size_t mixed_workspace_per_atom(const DevModel &M);
 size_t mixed_workspace_fixed(const DevModel &M);
 int mixed_eval(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm, const float *box,
-               const int32_t *nbrs, double *energy, float *Eatom, float4 *F4, double *virial, void *ws,
+               const int32_t *nbrs, double *energy, float *Eatom, ForceSum *F4, double *virial, void *ws,
                cudaStream_t st, int dT_warps, FitShape fit);
 int mixed_descriptors_f32(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm,
                           const float *box, const int32_t *nbrs, float *T, float *G, int *err, void *ws,
@@ -431,14 +431,14 @@ static size_t fp32_ws_bytes(const DevModel &M, size_t NF) {
   const size_t fw = fit_width_max(M), op = al((NF + (size_t)127 * M.ntypes) * ((fw + 31) / 32 * 32) * 4);
   const size_t gh = M.nfit > 2 ? 2 * fw : 0;
   const size_t ex = al(gemm_exp_bytes(NF + (size_t)127 * M.ntypes, (int)fw)) * (M.nfit == 1 ? 1 : 2);
-  return al(NF * ((10 * M.E2 + M.A * M.E2 + hid + gh + 1) * 4 + 16)) + ex + op +
+  return al(NF * ((10 * M.E2 + M.A * M.E2 + hid + gh + 1) * 4 + sizeof(ForceSum))) + ex + op +
          (M.nfit == 1 || op <= NF * (size_t)(M.A * M.E2) * 4 ? 0 : op);
 }
 
 // Workspace of NF atoms with nE energy / virial rows.
 static size_t eval_ws_bytes(const DevModel &M, size_t NF, size_t nE) {
   size_t a = fp32_ws_bytes(M, NF) + 16 * 256 + al(nE * 9 * 8);
-  size_t b = al(NF * mixed_workspace_per_atom(M)) + mixed_workspace_fixed(M) + al(NF * 16) + al(NF * 4) +
+  size_t b = al(NF * mixed_workspace_per_atom(M)) + mixed_workspace_fixed(M) + al(NF * sizeof(ForceSum)) + al(NF * 4) +
              al(nE * 9 * 8) + 16 * 256;
   return std::max(a, b);
 }
@@ -646,7 +646,7 @@ static int embed_fwd_fp32(const DevModel &M, const SysDesc &D, const float *pos,
 }
 
 static int eval_fp32(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm,
-                     const float *box, const int32_t *nbrs, double *energy, float4 *F4, float *Eatom,
+                     const float *box, const int32_t *nbrs, double *energy, ForceSum *F4, float *Eatom,
                      double *virial, char *base, char *w, size_t nE, int *err, cudaStream_t st) {
   const size_t NF = (size_t)D.N * D.F;
   const int E2 = M.E2, A = M.A, K0 = A * E2;
@@ -700,7 +700,7 @@ int dpb::eval_impl(const dpb_model *m, int precision, const float *pos, const in
   const DevModel &M = m->dm;
   const size_t NF = (size_t)natoms * nframes;
   char *w = (char *)workspace;
-  float4 *F4 = (float4 *)w; w += al(NF * 16);
+  ForceSum *F4 = (ForceSum *)w; w += al(NF * sizeof(ForceSum));
   float *Eatom = (float *)w; w += al(NF * 4);
   double *vir = virial;
   double *vscratch = (double *)w; w += al(nE * 9 * 8);
@@ -726,7 +726,7 @@ namespace dpb {
 int eval_tune_dT(const dpb_model *m, int natoms, int nframes, void *workspace, cudaStream_t st, int *best) {
   const size_t NF = (size_t)natoms * nframes;
   char *w = (char *)workspace;
-  w += al(NF * 16);
+  w += al(NF * sizeof(ForceSum));
   w += al(NF * 4);
   w += al((size_t)nframes * 9 * 8);
   return mixed_tune_dT(m->dm, NF, w, st, best);

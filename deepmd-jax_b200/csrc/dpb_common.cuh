@@ -151,6 +151,20 @@ __device__ __forceinline__ void row_adjoint(const RowGeom &g, float inv_std, con
   gx[2] = gh2 * inv_rp + g_r * d2;
 }
 
+// Force accumulator of an atom: FP64, so that the order of the atomics does not show
+// in the FP32 force.  (With FP32 sums, one 16-byte atomic per pair, two runs differed
+// in 21,000 of 36,864 components, and forces of the FP32 form lay 7.3e-7 instead of
+// 6.9e-7 from float64.  98,304 atoms: mixed adjoint 1.447 -> 1.426 ms, the centre's sum
+// without its stop in shared memory; FP32 adjoint 4.32 -> 4.34 ms.)
+struct __align__(16) ForceSum {
+  double x, y, z, pad;
+};
+__device__ __forceinline__ void force_add(ForceSum &f, float x, float y, float z) {
+  atomicAdd(&f.x, (double)x);
+  atomicAdd(&f.y, (double)y);
+  atomicAdd(&f.z, (double)z);
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -863,7 +863,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
                                                                const int32_t *__restrict__ nbrs,
                                                                const float4 *__restrict__ rows_g,
                                                                const int *__restrict__ rcnt,
-                                                               const float *__restrict__ dT, float4 *__restrict__ F4,
+                                                               const float *__restrict__ dT, ForceSum *__restrict__ F4,
                                                                double *__restrict__ virial, int *__restrict__ err) {
   using SD = SplitDims<E0, E1, E2>;
   using SM = SplitBwdSmem<E0, E1, E2>;
@@ -874,7 +874,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
   float4 *rowbuf = reinterpret_cast<float4 *>(smem + SM::rowbuf);
   __shared__ int wcnt[kSplitThreads / 32];
   __shared__ float3 ri_s[kBlkAtoms];
-  __shared__ float fi_s[4 * 3];
+  __shared__ int src_s[4];  // user index of each centre
   __shared__ double vir_s[9];
   __shared__ float wvir_s[4][9];
   __shared__ __align__(8) uint64_t mbar;
@@ -928,8 +928,8 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
     if (tid < nb) {
       const float4 q = posS[g0 + tid];
       ri_s[tid] = make_float3(q.x, q.y, q.z);
+      src_s[tid] = __float_as_int(q.w);
     }
-    if (tid < 12) fi_s[tid] = 0.f;
     for (int e = tid; e < nb * 10 * E2; e += kSplitThreads) {  // dT rows [slot][c][w] -> [slot][w][12]
       const int sc = e / E2, w = e - sc * E2, slot = sc / 10, c = sc - slot * 10;
       dTs[(slot * E2 + w) * 12 + c] = dT[g0 * 10 * E2 + e];
@@ -1077,7 +1077,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
             float gx[3];
             row_adjoint(gm, inv_std, uu, gst * sm[SD::O_SC + 2], gx);
             if (act) {
-              atomicAdd(&F4[frame_base + (packed >> 3)], make_float4(-gx[0], -gx[1], -gx[2], 0.f));
+              force_add(F4[frame_base + (packed >> 3)], -gx[0], -gx[1], -gx[2]);
 #pragma unroll
               for (int p3 = 0; p3 < 3; ++p3)
 #pragma unroll
@@ -1097,9 +1097,7 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
             }
             const int kp = __shfl_up_sync(0xffffffffu, key, 1);
             if (act && (lane == 0 || kp != key)) {
-              atomicAdd(&fi_s[slot * 3 + 0], s0);
-              atomicAdd(&fi_s[slot * 3 + 1], s1);
-              atomicAdd(&fi_s[slot * 3 + 2], s2);
+              force_add(F4[frame_base + src_s[slot]], s0, s1, s2);
             }
           }
           rowstart += nrows;
@@ -1118,11 +1116,6 @@ __global__ void __launch_bounds__(kSplitThreads, 2) k_split_bwd(DevModel M, SysD
     __syncthreads();
     if (tid < 9)
       vir_s[tid] += ((double)wvir_s[0][tid] + (double)wvir_s[1][tid]) + ((double)wvir_s[2][tid] + (double)wvir_s[3][tid]);
-    if (tid < nb * 3) {
-      const int a = tid / 3, k = tid - a * 3;
-      const int src = __float_as_int(posS[g0 + a].w);
-      atomicAdd(reinterpret_cast<float *>(&F4[frame_base + src]) + k, fi_s[tid]);
-    }
     __syncthreads();
   }
   if (!ok) {
@@ -1169,7 +1162,7 @@ static int launch_fwd(const DevModel &M, const SysDesc &D, int ba, const float4 
 
 template <int E0, int E1, int E2>
 static int launch_bwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
-                      const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, const float *dG, float4 *F4,
+                      const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, const float *dG, ForceSum *F4,
                       double *virial, int *err, cudaStream_t st) {
   const int nblk = blocks_total(D, ba), smem = SplitBwdSmem<E0, E1, E2>::total;
   if (!nblk) return DPB_OK;
@@ -1196,7 +1189,7 @@ int split_embed_fwd(const DevModel &M, const SysDesc &D, int ba, const float4 *p
 }
 
 int split_embed_bwd(const DevModel &M, const SysDesc &D, int ba, const float4 *posS, const float *box,
-                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, const float *dG, float4 *F4,
+                    const int32_t *nbrs, const float4 *rows, const int *rcnt, float *T, const float *dG, ForceSum *F4,
                     double *virial, int *err, cudaStream_t st) {
   return M.E2 == 100 ? launch_bwd<25, 50, 100>(M, D, ba, posS, box, nbrs, rows, rcnt, T, dG, F4, virial, err, st)
                      : launch_bwd<32, 32, 64>(M, D, ba, posS, box, nbrs, rows, rcnt, T, dG, F4, virial, err, st);

@@ -7,7 +7,7 @@
 //                 the descriptor G (A x W) and its largest entry.
 //   k_embed_bwd   warp per centre atom: dE/dT from dE/dG, then the rows' h and
 //                 dh/ds~ give dE/ds~ and dE/dR~; the row adjoint gives dE/dx,
-//                 scattered as forces (float4 atomics) and reduced into the
+//                 scattered as forces (FP64 atomics) and reduced into the
 //                 virial.
 //   k_fit_energy, k_finalize
 // The tuned uncompressed nets run in embed_split.cu, other shapes in
@@ -236,7 +236,7 @@ __device__ __forceinline__ void embed_rows_bwd_cmp(const float *__restrict__ coe
                                                    int ng, int n, const float *__restrict__ rowbuf,
                                                    float *__restrict__ hd, const float *__restrict__ dT,
                                                    float inv_std, float mean, int lane, float &fi0, float &fi1,
-                                                   float &fi2, float (&vir)[9], float4 *__restrict__ F4,
+                                                   float &fi2, float (&vir)[9], ForceSum *__restrict__ F4,
                                                    size_t frame_base) {
   static_assert(E2 % 4 == 0, "table width");
   const bool act = lane < n;
@@ -330,7 +330,7 @@ __device__ __forceinline__ void embed_rows_bwd_cmp(const float *__restrict__ coe
   float gx[3];
   row_adjoint(gm, inv_std, u, gst, gx);
   if (act) {
-    atomicAdd(&F4[frame_base + jj], make_float4(-gx[0], -gx[1], -gx[2], 0.f));
+    force_add(F4[frame_base + jj], -gx[0], -gx[1], -gx[2]);
     fi0 += gx[0]; fi1 += gx[1]; fi2 += gx[2];
 #pragma unroll
     for (int p = 0; p < 3; ++p)
@@ -350,7 +350,7 @@ template <int E2>
 __global__ void __launch_bounds__(256, 2) k_embed_bwd(DevModel M, SysDesc D, int ti, const float *__restrict__ pos,
                                                    const int32_t *__restrict__ perm, const float *__restrict__ box,
                                                    const int32_t *__restrict__ nbrs, const float *__restrict__ Tin,
-                                                   const float *__restrict__ dG, float4 *__restrict__ F4,
+                                                   const float *__restrict__ dG, ForceSum *__restrict__ F4,
                                                    double *__restrict__ virial) {
   constexpr int NQ = (E2 + 31) / 32;
   extern __shared__ __align__(16) float smem[];
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(256, 2) k_embed_bwd(DevModel M, SysDesc D, int
       __syncwarp();
     }
     fi0 = warp_sum(fi0); fi1 = warp_sum(fi1); fi2 = warp_sum(fi2);
-    if (lane == 0) atomicAdd(&F4[frame_base + (perm ? perm[i] : i)], make_float4(fi0, fi1, fi2, 0.f));
+    if (lane == 0) force_add(F4[frame_base + (perm ? perm[i] : i)], fi0, fi1, fi2);
   }
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
@@ -598,12 +598,12 @@ __global__ void __launch_bounds__(256) k_fit_energy(EnergyArgs g, const float *_
   }
 }
 
-// Forces (float4 accumulator) and per-atom energies to the caller's layout;
+// Forces (from their FP64 sums) and per-atom energies to the caller's layout;
 // non-finite positions or results raise status bit 16 and, as NaN inputs do
 // in the reference's float arithmetic, make the frame's energy NaN.  *err != 0:
 // a tensor-core wait gave up, and what its CTA did not write is left from an
 // earlier call, so every result is NaN.
-__global__ void k_finalize(int NF, int N, const float4 *__restrict__ F4, float *__restrict__ force,
+__global__ void k_finalize(int NF, int N, const ForceSum *__restrict__ F4, float *__restrict__ force,
                            const float *__restrict__ Eatom_sorted, const int32_t *__restrict__ perm,
                            float *__restrict__ atom_energy, double *__restrict__ energy, int nE,
                            const float *__restrict__ pos, const int32_t *__restrict__ seg,
@@ -612,7 +612,8 @@ __global__ void k_finalize(int NF, int N, const float4 *__restrict__ F4, float *
   const bool gave_up = err && *err != 0;
   const float nan = __int_as_float(0x7fffffff);
   if (g < NF) {
-    const float4 v = gave_up ? make_float4(nan, nan, nan, 0.f) : F4[g];
+    const ForceSum a = F4[g];
+    const float3 v = gave_up ? make_float3(nan, nan, nan) : make_float3((float)a.x, (float)a.y, (float)a.z);
     force[(size_t)g * 3 + 0] = v.x;
     force[(size_t)g * 3 + 1] = v.y;
     force[(size_t)g * 3 + 2] = v.z;
@@ -647,7 +648,7 @@ int launch_embed_fwd_cmp(const DevModel &M, const SysDesc &D, int ti, const floa
 
 template <int E2>
 int launch_embed_bwd_cmp(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
-                         const float *box, const int32_t *nbrs, const float *T, const float *dG, float4 *F4,
+                         const float *box, const int32_t *nbrs, const float *T, const float *dG, ForceSum *F4,
                          double *virial, cudaStream_t st) {
   const int cnt = D.offs[ti + 1] - D.offs[ti];
   if (cnt == 0) return DPB_OK;
@@ -665,10 +666,10 @@ template int launch_embed_fwd_cmp<100>(const DevModel &, const SysDesc &, int, c
 template int launch_embed_fwd_cmp<64>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
                                       const float *, const int32_t *, float *, float *, float *, cudaStream_t);
 template int launch_embed_bwd_cmp<100>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
-                                       const float *, const int32_t *, const float *, const float *, float4 *,
+                                       const float *, const int32_t *, const float *, const float *, ForceSum *,
                                        double *, cudaStream_t);
 template int launch_embed_bwd_cmp<64>(const DevModel &, const SysDesc &, int, const float *, const int32_t *,
-                                      const float *, const int32_t *, const float *, const float *, float4 *, double *,
+                                      const float *, const int32_t *, const float *, const float *, ForceSum *, double *,
                                       cudaStream_t);
 
 int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, float *Eatom, __half *gZ, int8_t *gexp,
@@ -681,7 +682,7 @@ int launch_fit_energy(const EnergyArgs &g, const float *H, const float *tl, floa
   return DPB_OK;
 }
 
-int launch_finalize(int NF, int N, const float4 *F4, float *force, const float *Eatom, const int32_t *perm,
+int launch_finalize(int NF, int N, const ForceSum *F4, float *force, const float *Eatom, const int32_t *perm,
                     float *atom_energy, double *energy, int nE, const float *pos, const int32_t *seg,
                     const int *err, uint32_t *status, cudaStream_t st) {
   int n = NF > nE ? NF : nE;
@@ -694,13 +695,13 @@ int launch_finalize(int NF, int N, const float4 *F4, float *force, const float *
 
 }  // namespace dpb
 
-extern "C" int dpb_selftest_finalize(int natoms, int nframes, const float *acc, const float *pos, const int *err,
+extern "C" int dpb_selftest_finalize(int natoms, int nframes, const double *acc, const float *pos, const int *err,
                                      double *energy, float *atom_energy, float *force, uint32_t *status,
                                      void *stream) {
   if (natoms <= 0 || nframes <= 0 || !acc || !pos || !energy || !atom_energy || !force || !status ||
       (reinterpret_cast<uintptr_t>(acc) & 15) != 0)
     return DPB_ERR_INVALID_ARG;
-  return dpb::launch_finalize(natoms * nframes, natoms, reinterpret_cast<const float4 *>(acc), force, atom_energy,
+  return dpb::launch_finalize(natoms * nframes, natoms, reinterpret_cast<const dpb::ForceSum *>(acc), force, atom_energy,
                               nullptr, atom_energy, energy, nframes, pos, nullptr, err, status,
                               (cudaStream_t)stream);
 }

@@ -338,7 +338,7 @@ struct RowOut {
 };
 
 __device__ __forceinline__ void gen_row_finish(const RowGeom &gm, bool act, int jj, float inv_std, const float u[10],
-                                               const float v[10], RowOut &ro, float4 *__restrict__ F4,
+                                               const float v[10], RowOut &ro, ForceSum *__restrict__ F4,
                                                size_t frame_base) {
   const float sn = gm.s * inv_std;
   const float inv_rp = 1.f / (gm.r + 1e-16f);
@@ -351,7 +351,7 @@ __device__ __forceinline__ void gen_row_finish(const RowGeom &gm, bool act, int 
   float gx[3];
   row_adjoint(gm, inv_std, u, gst, gx);
   if (act) {
-    atomicAdd(&F4[frame_base + jj], make_float4(-gx[0], -gx[1], -gx[2], 0.f));
+    force_add(F4[frame_base + jj], -gx[0], -gx[1], -gx[2]);
     ro.fi0 += gx[0];
     ro.fi1 += gx[1];
     ro.fi2 += gx[2];
@@ -378,7 +378,7 @@ __device__ __forceinline__ void gen_row_geom(const float *rowbuf, bool act, int 
 // u = dT.h, v = dT.dh at the output, then the row adjoint.
 __device__ void gen_rows_bwd(const GenNet &G, const float *__restrict__ W, int n, const float *__restrict__ rowbuf,
                              const float *__restrict__ dT, float *hA, float *dA, float *hB, float *dB, float inv_std,
-                             float mean, int lane, RowOut &ro, float4 *__restrict__ F4, size_t frame_base) {
+                             float mean, int lane, RowOut &ro, ForceSum *__restrict__ F4, size_t frame_base) {
   const bool act = lane < n;
   RowGeom gm;
   int jj;
@@ -474,7 +474,7 @@ __device__ void gen_rows_bwd(const GenNet &G, const float *__restrict__ W, int n
 
 __device__ void gen_rows_bwd_cmp(const float *__restrict__ coeff, float srmin, float delta, int ng, int E, int n,
                                  const float *__restrict__ rowbuf, const float *__restrict__ dT, float inv_std,
-                                 float mean, int lane, RowOut &ro, float4 *__restrict__ F4, size_t frame_base) {
+                                 float mean, int lane, RowOut &ro, ForceSum *__restrict__ F4, size_t frame_base) {
   const bool act = lane < n;
   RowGeom gm;
   int jj;
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(256) k_embed_bwd_gen(DevModel M, GenNet G, Sys
                                                        const float *__restrict__ pos, const int32_t *__restrict__ perm,
                                                        const float *__restrict__ box, const int32_t *__restrict__ nbrs,
                                                        const float *__restrict__ Tin, const float *__restrict__ dG,
-                                                       float4 *__restrict__ F4, double *__restrict__ virial) {
+                                                       ForceSum *__restrict__ F4, double *__restrict__ virial) {
   extern __shared__ float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
   const int A = M.A, E = G.E;
@@ -666,7 +666,7 @@ __global__ void __launch_bounds__(256) k_embed_bwd_gen(DevModel M, GenNet G, Sys
       __syncwarp();
     }
     const float f0 = warp_sum(ro.fi0), f1 = warp_sum(ro.fi1), f2 = warp_sum(ro.fi2);
-    if (lane == 0) atomicAdd(&F4[frame_base + (perm ? perm[i] : i)], make_float4(f0, f1, f2, 0.f));
+    if (lane == 0) force_add(F4[frame_base + (perm ? perm[i] : i)], f0, f1, f2);
   }
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
@@ -718,7 +718,7 @@ int launch_embed_fwd_gen(const DevModel &M, const SysDesc &D, int ti, const floa
 }
 
 int launch_embed_bwd_gen(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
-                         const float *box, const int32_t *nbrs, const float *T, const float *dG, float4 *F4,
+                         const float *box, const int32_t *nbrs, const float *T, const float *dG, ForceSum *F4,
                          double *virial, cudaStream_t st) {
   const int cnt = D.offs[ti + 1] - D.offs[ti];
   if (cnt == 0) return DPB_OK;

@@ -952,7 +952,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
                                                                   const float *__restrict__ dTs,
                                                                   const float4 *__restrict__ rows_g,
                                                                   const int *__restrict__ rcnt,
-                                                                  float4 *__restrict__ F4,
+                                                                  ForceSum *__restrict__ F4,
                                                                   double *__restrict__ virial,
                                                                   int *__restrict__ err) {
   using MD = MixDims<E0, E1, E2>;
@@ -966,7 +966,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
   float4 *rowbuf = reinterpret_cast<float4 *>(opb + round1k(2 * MD::OPA));
   __shared__ int wcnt[kBwdThreads / 32];
   __shared__ float3 ri_s[kBlkAtoms];
-  __shared__ float fi_s[kBlkAtoms * 3];
+  __shared__ int src_s[kBlkAtoms];  // user index of each centre
   __shared__ float sc_s[kBlkAtoms];
   __shared__ double vir_s[9];
   __shared__ __align__(8) uint64_t mbar;
@@ -1042,8 +1042,8 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
       const float4 q = posS[g0 + tid];
       ri_s[tid] = make_float3(q.x, q.y, q.z);
       sc_s[tid] = dTs[g0 + tid];
+      src_s[tid] = __float_as_int(q.w);
     }
-    if (tid < kBlkAtoms * 3) fi_s[tid] = 0.f;
     // ---- DTB: rows n = 16 slot + c of the 8 atoms (K-major, K = N2); zero for c >= 10 and missing atoms
     for (int e = tid; e < kDtbRows * (MD::N2 / 8); e += kBwdThreads) {
       const int n = e / (MD::N2 / 8), k8 = (e - n * (MD::N2 / 8)) * 8;
@@ -1197,7 +1197,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
           gx[2] *= scl;
           if (half == 0) {
             if (act) {
-              atomicAdd(&F4[frame_base + jsrc], make_float4(-gx[0], -gx[1], -gx[2], 0.f));
+              force_add(F4[frame_base + jsrc], -gx[0], -gx[1], -gx[2]);
 #pragma unroll
               for (int p3 = 0; p3 < 3; ++p3)
 #pragma unroll
@@ -1218,9 +1218,7 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
             }
             const int kp = __shfl_up_sync(0xffffffffu, key, 1);
             if (act && (lane == 0 || kp != key)) {
-              atomicAdd(&fi_s[slot * 3 + 0], s0);
-              atomicAdd(&fi_s[slot * 3 + 1], s1);
-              atomicAdd(&fi_s[slot * 3 + 2], s2);
+              force_add(F4[frame_base + src_s[slot]], s0, s1, s2);
             }
           }
           rowstart += nrows;
@@ -1228,12 +1226,6 @@ __global__ void __launch_bounds__(kBwdThreads, 2) k_mix_embed_bwd(DevModel M, Sy
       }
     }
     if (!ok) break;
-    __syncthreads();
-    if (tid < nb * 3) {
-      const int a = tid / 3, k = tid - a * 3;
-      const int src = __float_as_int(posS[g0 + a].w);
-      atomicAdd(reinterpret_cast<float *>(&F4[frame_base + src]) + k, fi_s[tid]);
-    }
     tc::cp_async_wait<0>();
     __syncthreads();
   }
@@ -1263,7 +1255,7 @@ size_t mix_bwd_smem() {
 template <int E0, int E1, int E2>
 int launch_mix_embed_bwd(const DevModel &M, const SysDesc &D, const float4 *posS,
                          const float *box, const int32_t *nbrs, const __half *dTh, const float *dTs,
-                         const float4 *rows_g, const int *rcnt, float4 *F4, double *virial, int *err,
+                         const float4 *rows_g, const int *rcnt, ForceSum *F4, double *virial, int *err,
                          cudaStream_t st) {
   // one launch over every centre type and frame: a CTA's blocks run through the
   // frames of a type in increasing order, and it flushes its virial sum to a
@@ -1947,7 +1939,7 @@ size_t mixed_workspace_fixed(const DevModel &M) {
 size_t mixed_workspace_per_atom(const DevModel &M) {
   const int FW = M.mfw, K0 = M.A * M.E2;
   return (size_t)10 * M.E2 * 4 + (size_t)K0 * 2 + (size_t)K0 * 4 + (size_t)10 * n2_of(M) * 2 + 4 + 16 +
-         (size_t)kRowStoreCap * 16 + (size_t)M.ntypes * 4 + (size_t)(2 * M.nfit + 1) * FW * 4 + 64;
+         (size_t)kRowStoreCap * 16 + (size_t)M.ntypes * 4 + (size_t)(2 * M.nfit + 1) * FW * 4 + 48;
 }
 
 // dE/dT with W atoms (warps) per block, W in {2, 4, 8} (launch shape only).
@@ -2028,19 +2020,19 @@ int launch_embed_fwd_cmp(const DevModel &M, const SysDesc &D, int ti, const floa
                          const float *box, const int32_t *nbrs, float *T, float *G, float *gmax, cudaStream_t st);
 template <int E2>
 int launch_embed_bwd_cmp(const DevModel &M, const SysDesc &D, int ti, const float *pos, const int32_t *perm,
-                         const float *box, const int32_t *nbrs, const float *T, const float *dG, float4 *F4,
+                         const float *box, const int32_t *nbrs, const float *T, const float *dG, ForceSum *F4,
                          double *virial, cudaStream_t st);
 int launch_embed_fwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
                          const int32_t *, float *, float *, float *, cudaStream_t);
 int launch_embed_bwd_gen(const DevModel &, const SysDesc &, int, const float *, const int32_t *, const float *,
-                         const int32_t *, const float *, const float *, float4 *, double *, cudaStream_t);
+                         const int32_t *, const float *, const float *, ForceSum *, double *, cudaStream_t);
 
 // Embedding nets without tensor-core kernels in the mixed form - compressed
 // tables (a lookup, no GEMM) and shapes other than the tuned ones: the FP32
 // kernels produce T and G (FP32) and take the adjoint; the fitting chain runs
 // on the tensor cores from an FP16 copy of G.
 static int mixed_eval_compressed(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm,
-                                 const float *box, const int32_t *nbrs, double *energy, float *Eatom, float4 *F4,
+                                 const float *box, const int32_t *nbrs, double *energy, float *Eatom, ForceSum *F4,
                                  double *virial, float *T, __half *Gb, float *dG, float *scratch, int *err,
                                  FitShape fit, cudaStream_t st) {
   const size_t NF = (size_t)D.N * D.F;
@@ -2152,7 +2144,7 @@ int mixed_tune_dT(const DevModel &M, size_t NF, void *ws, cudaStream_t st, int *
 int *mixed_err(const DevModel &M, size_t NF, void *ws) { return mixed_ws(M, NF, ws).err; }
 
 int mixed_eval(const DevModel &M, const SysDesc &D, const float *pos, const int32_t *perm, const float *box,
-               const int32_t *nbrs, double *energy, float *Eatom, float4 *F4, double *virial, void *ws,
+               const int32_t *nbrs, double *energy, float *Eatom, ForceSum *F4, double *virial, void *ws,
                cudaStream_t st, int dT_warps, FitShape fit) {
   const size_t NF = (size_t)D.N * D.F;
   const MixedWs mw = mixed_ws(M, NF, ws);

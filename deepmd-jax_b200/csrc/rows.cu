@@ -23,16 +23,16 @@ __global__ void k_pos_sorted(size_t NF, int N, const float *__restrict__ pos, co
 // word zeroed in one launch.  (A memset each took 1.4 us and left 2 to 6 us
 // between them, also inside a graph: 20 us before the first kernel of 196 us at
 // 192 atoms.)
-__global__ void k_eval_begin(size_t NF, float4 *__restrict__ F4, size_t nE, double *__restrict__ energy,
+__global__ void k_eval_begin(size_t NF, ForceSum *__restrict__ F4, size_t nE, double *__restrict__ energy,
                              double *__restrict__ virial, int *__restrict__ err) {
   const size_t g = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g < NF) F4[g] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (g < NF) F4[g] = ForceSum{0.0, 0.0, 0.0, 0.0};
   if (g < nE) energy[g] = 0.0;
   if (g < 9 * nE) virial[g] = 0.0;
   if (err && g == 0) *err = 0;
 }
 
-int launch_eval_begin(size_t NF, float4 *F4, size_t nE, double *energy, double *virial, int *err, cudaStream_t st) {
+int launch_eval_begin(size_t NF, ForceSum *F4, size_t nE, double *energy, double *virial, int *err, cudaStream_t st) {
   const size_t n = std::max(NF, 9 * nE);
   k_eval_begin<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(NF, F4, nE, energy, virial, err);
   count_launch();

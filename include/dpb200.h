@@ -158,7 +158,8 @@ DPB_API int dpb_eval_workspace_bytes(const dpb_model *model, int natoms, int nfr
  *   nbrs     (F,N,sum(sel)) int32 device, layout of dpb_nlist_build
  *   energy   (F) float64 device out (total energy per frame)
  *   atom_energy (F,N) float32 device out or NULL
- *   force    (F,N,3) float32 device out, -dE/dpos
+ *   force    (F,N,3) float32 device out, -dE/dpos (summed in FP64 over pairs: the
+ *            same bits from call to call)
  *   virial   (F,9) float64 device out or NULL: W_ab = -sum_pairs x_a dE/dx_b
  *            with x = r_j - r_i; trace(W) = -dU/deps of a uniform strain
  *            (deepmd_jax/md_utils.py:139-159)
@@ -383,10 +384,10 @@ DPB_API int dpb_profile_enable(int on);
  * out: 128*64 floats (device), err: device int set on a barrier timeout. */
 DPB_API int dpb_selftest_tcgen05(int variant, float *out, int *err, void *stream);
 /* Diagnostics: the last step of an evaluation alone, on sums given by the
- * caller (acc: (F,N,4) float32, 16-byte aligned; energy (F), atom_energy (F,N)
+ * caller (acc: (F,N,4) float64, 16-byte aligned; energy (F), atom_energy (F,N)
  * in place).  err: device int or NULL; where it is set, as by a tensor-core wait
  * that gave up, every result becomes NaN and DPB_ST_NONFINITE is raised. */
-DPB_API int dpb_selftest_finalize(int natoms, int nframes, const float *acc, const float *pos, const int *err,
+DPB_API int dpb_selftest_finalize(int natoms, int nframes, const double *acc, const float *pos, const int *err,
                                   double *energy, float *atom_energy, float *force, uint32_t *status, void *stream);
 DPB_API int dpb_profile_read(int stage, double *ms, uint64_t *count);
 

@@ -20,11 +20,12 @@ def test_give_up_reaches_every_result(gave_up, natoms, nframes):
     def dev(shape, dtype=torch.float32):
         return torch.tensor(rng.normal(size=shape), dtype=dtype, device="cuda")
 
-    acc, pos, atom_energy = dev((nframes, natoms, 4)), dev((nframes, natoms, 3)), dev((nframes, natoms))
+    acc = dev((nframes, natoms, 4), torch.float64)
+    pos, atom_energy = dev((nframes, natoms, 3)), dev((nframes, natoms))
     energy, force = dev((nframes,), torch.float64), torch.zeros((nframes, natoms, 3), device="cuda")
     err = torch.full((1,), int(gave_up), dtype=torch.int32, device="cuda")
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
-    before = [t.clone() for t in (acc[..., :3], energy, atom_energy)]
+    before = [t.clone() for t in (acc[..., :3].float(), energy, atom_energy)]
     p = [ctypes.c_void_p(t.data_ptr()) for t in (acc, pos, err, energy, atom_energy, force, status)]
     assert lib.dpb_selftest_finalize(natoms, nframes, *p, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
     torch.cuda.synchronize()
