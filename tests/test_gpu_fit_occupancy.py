@@ -24,7 +24,10 @@ def test_two_fitting_ctas_fit_an_sm(width, layers, tmp_path):
                 precision="mixed")
     prof.export_chrome_trace(str(tmp_path / "trace.json"))
     with open(tmp_path / "trace.json") as f:
-        fits = [e for e in json.load(f)["traceEvents"] if "k_mix_fit" in e.get("name", "") and "grid" in e.get("args", {})]
+        events = [e for e in json.load(f)["traceEvents"] if "grid" in e.get("args", {})]
+    if not events:
+        pytest.skip("kernels cannot be traced here (another CUPTI client)")
+    fits = [e for e in events if "k_mix_fit" in e["name"]]
     assert len(fits) == 1 and "false>" in fits[0]["name"]      # the shape for many tiles
     args = fits[0]["args"]
     print(fits[0]["name"][:40], args["shared memory"], args["registers per thread"])
